@@ -25,91 +25,65 @@
 #pragma once
 #include <cstdint>
 
-#include "advect_ops.cuh"
+#include "pairs.cuh"
 
 namespace fesom {
 FESOM_VARIANT_BEGIN
 
 constexpr int NTMAX = 4;
 constexpr int kThreads = 256;
-// resident 256-thread blocks per SM each step kernel's register budget is
-// cut for (4 = 64 registers, 5 = 48, 6 = 40).  Measured on the FP64 plain
-// step at 1000x1000x64: more resident warps hide more gather latency than
-// the extra spills cost, up to these values (k_col1's shared memory allows
-// no more than 5 blocks anyway).  Build-time tuning knobs.
+constexpr int kEdgeThreads = 128, kColThreads = 128;
+// Resident 128-thread blocks per SM that each step kernel's register budget is
+// cut for.  The kernels are bound by the latency of their gathers; a lane issues the
+// loads of its whole stencil before it uses the first, so what hides the latency
+// is the loads in flight per warp: 16 warps of 128 registers per SM beat 20-24
+// with fewer (FP64, 400x400x64, two tracers: k_edge 0.30 ms at 4 blocks, 0.33 at 3; k_col1
+// 0.225 at 4, 0.256 / 0.30 at 3 / 5; k_col3 0.236 at 4, 0.237 / 0.32; FP32 k_edge 0.184 at 5, 0.193
+// / 0.188 at 4 / 6; k_col2 0.138 at 6, 0.152 at 5).  Build-time knobs.
 #ifndef FESOM_MINB_EDGE
-#define FESOM_MINB_EDGE 5
+#define FESOM_MINB_EDGE 4
 #endif
 #ifndef FESOM_MINB_COL1
-#define FESOM_MINB_COL1 5
+#define FESOM_MINB_COL1 4
 #endif
 #ifndef FESOM_MINB_COL2
-#define FESOM_MINB_COL2 6
+#define FESOM_MINB_COL2 4
 #endif
 #ifndef FESOM_MINB_COL3
-#define FESOM_MINB_COL3 6
+#define FESOM_MINB_COL3 4
 #endif
-#ifndef FESOM_MINB_GRAD
-#define FESOM_MINB_GRAD 5
-#endif
-// The same for the FP32-arithmetic kernels (FP32 and 16-bit storage), which
-// need fewer registers: timed on the same workload in FP32, 4 / 5 / 6 / 7
-// blocks (col2, col3: up to 8): edge best at 6 (1.98 ms), col1 at 7 (2.07),
-// col2 and col3 at 7 (1.68, 1.65; 8 no better), against 1.99 / 2.38 / 1.86 /
-// 1.97 ms with the FP64 budgets.
 #ifndef FESOM_MINB32_EDGE
-#define FESOM_MINB32_EDGE 6
+#define FESOM_MINB32_EDGE 5
 #endif
 #ifndef FESOM_MINB32_COL1
-#define FESOM_MINB32_COL1 7
+#define FESOM_MINB32_COL1 5
 #endif
 #ifndef FESOM_MINB32_COL2
-#define FESOM_MINB32_COL2 7
+#define FESOM_MINB32_COL2 6
 #endif
 #ifndef FESOM_MINB32_COL3
-#define FESOM_MINB32_COL3 7
+#define FESOM_MINB32_COL3 5
 #endif
-#ifndef FESOM_MINB32_GRAD
-#define FESOM_MINB32_GRAD 5
-#endif
-template <typename R>
-struct MinBlocks {
-  static constexpr int grad = FESOM_MINB_GRAD, edge = FESOM_MINB_EDGE, col1 = FESOM_MINB_COL1, col2 = FESOM_MINB_COL2,
-                       col3 = FESOM_MINB_COL3;
+template <typename R, int NT>
+struct StepBlocks {
+  static constexpr int edge = FESOM_MINB_EDGE, col1 = FESOM_MINB_COL1, col2 = FESOM_MINB_COL2, col3 = FESOM_MINB_COL3;
 };
-template <>
-struct MinBlocks<float> {
-  static constexpr int grad = FESOM_MINB32_GRAD, edge = FESOM_MINB32_EDGE, col1 = FESOM_MINB32_COL1,
-                       col2 = FESOM_MINB32_COL2, col3 = FESOM_MINB32_COL3;
+template <int NT>
+struct StepBlocks<float, NT> {  // four tracers a lane: 128 registers
+  static constexpr int edge = NT == 4 ? 4 : FESOM_MINB32_EDGE, col1 = NT == 4 ? 4 : FESOM_MINB32_COL1,
+                       col2 = NT == 4 ? 4 : FESOM_MINB32_COL2, col3 = NT == 4 ? 4 : FESOM_MINB32_COL3;
 };
-// Incidence records of each node kernel's block staged in shared memory or
-// read through L1, per arithmetic type.  Measured on the 1000x1000x64 step:
-// FP64 staged k_col1 3.28 ms (unstaged 3.34), k_col2 2.39 (2.50), k_col3 2.75
-// (2.75); FP32 unstaged k_col1 1.81 (staged 1.84), k_col2 1.61 (1.68), k_col3
-// 1.57 (1.60) -- the FP32 kernels keep more blocks resident, whose shared
-// memory would otherwise crowd out the L1.
-template <typename R>
-struct StageIncidence {
-  static constexpr bool col1 = true, col2 = true, col3 = true;
+// Tracers of a batch of NT that a lane advances together; it takes the groups one
+// after the other.  Two FP64 tracers share a column's records and geometry
+// (k_col1 0.225 ms against 2 x 0.156 for one at a time, k_col3 0.236 against 2 x 0.137),
+// except in k_col2, whose sums and bounds of two do not fit the registers (0.267
+// against 0.363).
+template <typename R, int NT>
+struct LaneTracers {
+  static constexpr int cap(int g) { return g < NT ? g : NT; }
+  static constexpr int col1 = cap(sizeof(R) == 8 ? 2 : 4), col2 = cap(sizeof(R) == 8 ? 1 : 4), col3 = col1;
 };
-template <>
-struct StageIncidence<float> {
-  static constexpr bool col1 = false, col2 = false, col3 = false;
-};
-// The LO gather of k_col1 issues the loads of this many incident edges
-// together before using any of them.  Every (edge, level) and (node, level)
-// address of a cell's level lies inside its padded column, so the loads of
-// dry edge levels, and of the clamped records past the node's last edge, are
-// in bounds; their values are discarded.  The fluxes are still accumulated
-// one edge at a time in ascending incidence order.  (Measured per kernel on
-// the 512-cell capped schedules at 1000x1000x64: k_col1 FP64 with 1 / 2 / 3
-// / 4 / 6 edges 3.24 / 2.89 / 2.76 / 3.14 / 2.98 ms, FP32 with 2 / 3 / 4 / 6
-// 1.71 / 1.59 / 1.71 / 1.76 ms; the same form is slower in k_col2 and
-// k_col3, whose loops stay one edge at a time.)
-#ifndef FESOM_GCHUNK_COL1
-#define FESOM_GCHUNK_COL1 3
-#endif
-constexpr int kGChunkCol1 = FESOM_GCHUNK_COL1;
+constexpr int kGradBlocks = 5;  // k_grad: 256-thread blocks
 constexpr int kCellsPerBlock = 512;      // schedule cap: wet cells per block (two per thread)
 constexpr int kMaxCellsPerBlock = 576;   // upper bound (target + deepest column)
 constexpr int kMaxItemsPerBlock = 512;
@@ -154,9 +128,9 @@ struct FusedArgs {
   const TS *T[NTMAX];     // values
   const TS *TAB[NTMAX];   // valuesAB (high-order fluxes)
   TS *T_out[NTMAX];
-  R *adf_h[NTMAX];        // (NT, S, edge) tracer-interleaved: adf_h[t] = adf_h[0] + t, stride NT
-  R *adf_v[NTMAX];        // (NT, S, node) interfaces, tracer-interleaved like adf_h
-  R *lo[NTMAX];           // (NT, S, node) tracer-interleaved like adf_h
+  R *adf_h;               // (S, edge) pairs of every tracer side by side (pairs.cuh, il_at)
+  R *adf_v;               // (S, node) interfaces, likewise
+  R *lo;                  // (S, node), likewise
   R *rpm[NTMAX];          // (2, S, node): limiter ratios R+ and R- of each cell side by side
   R *vflux;               // (S, edge), shared by the tracers
   R *gradn[NTMAX];        // (2, S, node): ring-mean gradient (gx, gy) of valuesAB
@@ -171,9 +145,8 @@ struct FusedArgs {
   R off[NTMAX];           // storage offsets (16-bit storage)
   uint32_t seed[NTMAX];   // per-step random stream of each tracer (stochastic rounding)
   int sround;             // 1: stochastic rounding of 16-bit stores
-  // edge volume fluxes: 0 computed from the velocity (stored in vflux when the
-  // limiter needs them), 1 computed and stored, 2 loaded from vflux (stored
-  // by an earlier launch with the same velocity)
+  // edge volume fluxes: 0, 1 computed from the velocity and stored, 2 loaded
+  // from vflux (stored by an earlier launch with the same velocity)
   int vflux_mode;
   // failure detection: count of non-finite new values (nullptr: not counted)
   unsigned long long *nonfinite;
@@ -203,44 +176,6 @@ __device__ __forceinline__ CellMap map_cells(const DSched &sc, int blk, int *s_o
   return cm;
 }
 
-// A node block's incidence records (the CSR slice of its nodes) staged in
-// shared memory by one cooperative load, so that every lane's walk over its
-// node's edges starts from shared memory instead of a dependent global load.
-// Blocks with more than kNeStage records read them from global memory.
-constexpr int kNeStage = 512;
-__host__ __device__ constexpr size_t smem_stage() {
-  return 16 + (size_t)kNeStage * sizeof(int4) + sizeof(int) * (kMaxItemsPerBlock + 1);
-}
-
-struct Incidence {
-  const int4 *ne;   // records of the block, from its first node's first record
-  const int *nep;   // per local node: first record (minus sub)
-  int sub;
-};
-
-// STAGE = false reads the records from global memory (through L1) and needs
-// no shared memory for them.
-template <bool STAGE = true, typename R>
-__device__ __forceinline__ Incidence stage_incidence(const DMeshT<R> &m, const CellMap &cm, void *region) {
-  int4 *s_ne = reinterpret_cast<int4 *>(((uintptr_t)region + 15) & ~(uintptr_t)15);
-  int *s_nep = reinterpret_cast<int *>(s_ne + kNeStage);
-  const int p0 = m.ne_ptr[cm.i0], p1 = m.ne_ptr[cm.i0 + cm.ni];
-  Incidence r;
-  if (STAGE && p1 - p0 <= kNeStage) {
-    for (int i = threadIdx.x; i < p1 - p0; i += blockDim.x) s_ne[i] = m.ne4[p0 + i];
-    for (int j = threadIdx.x; j <= cm.ni; j += blockDim.x) s_nep[j] = m.ne_ptr[cm.i0 + j] - p0;
-    r.ne = s_ne;
-    r.nep = s_nep;
-    r.sub = 0;
-  } else {
-    r.ne = m.ne4 + p0;
-    r.nep = m.ne_ptr + cm.i0;
-    r.sub = p0;
-  }
-  __syncthreads();
-  return r;
-}
-
 // ---------------------------------------------------------------------------
 // k_grad: ring-mean gradients of valuesAB (lib/oce_muscl_adv.F90:400-450:
 // the mean of tr_xy over the node's ring, weighted by element area), for the
@@ -263,42 +198,6 @@ __device__ __forceinline__ void st_pair(float *p, float x, float y) {
   *reinterpret_cast<float2 *>(p) = make_float2(x, y);
 }
 
-// Tracer-interleaved work arrays (adf_h, lo): tracer t's value of cell o is
-// at X[t][o * NT] with X[t] = X[0] + t, so one vector load brings a cell's
-// values of every tracer of the batch (NT = 1, 2 or 4).
-template <int NT, typename R>
-__device__ __forceinline__ R &il(R *const *x, int t, cix o) {
-  return x[t][(size_t)o * NT];
-}
-template <int NT>
-__device__ __forceinline__ void il_load(const double *x0, cix o, double *v) {
-  const double *p = x0 + (size_t)o * NT;
-  if constexpr (NT == 1) {
-    v[0] = p[0];
-  } else if constexpr (NT == 2) {
-    const double2 a = *reinterpret_cast<const double2 *>(p);
-    v[0] = a.x; v[1] = a.y;
-  } else {
-    static_assert(NT == 4, "batches hold 1, 2 or 4 tracers");
-    const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  }
-}
-template <int NT>
-__device__ __forceinline__ void il_load(const float *x0, cix o, float *v) {
-  const float *p = x0 + (size_t)o * NT;
-  if constexpr (NT == 1) {
-    v[0] = p[0];
-  } else if constexpr (NT == 2) {
-    const float2 a = *reinterpret_cast<const float2 *>(p);
-    v[0] = a.x; v[1] = a.y;
-  } else {
-    static_assert(NT == 4, "batches hold 1, 2 or 4 tracers");
-    const float4 a = *reinterpret_cast<const float4 *>(p);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-  }
-}
-
 template <typename R, typename TS, int NT>
 __device__ __forceinline__ void grad_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk, int *smem) {
   int *s_off = smem, *s_item = smem + kMaxItemsPerBlock + 1;
@@ -313,7 +212,7 @@ __device__ __forceinline__ void grad_block(const DMeshT<R> &m, const FusedArgs<R
 }
 
 template <typename R, typename TS, int NT>
-__global__ void __launch_bounds__(kThreads, MinBlocks<R>::grad) k_grad(DMeshT<R> m, FusedArgs<R, TS> a) {
+__global__ void __launch_bounds__(kThreads, kGradBlocks) k_grad(DMeshT<R> m, FusedArgs<R, TS> a) {
   extern __shared__ int smem[];
   grad_block<R, TS, NT>(m, a, blockIdx.x, smem);
 }
@@ -359,120 +258,402 @@ __device__ __forceinline__ void ring_mean_n(const DMeshT<R> &m, const TS *const 
   }
 }
 
+// x / 6 and x / 3, correctly rounded.  The reciprocals of 3 and 6 round with a
+// relative error of 2^-54 (FP32: 2^-25), so q = RN(x y) is already a faithful
+// quotient and one Markstein correction rounds it (div_rcp needs two).  The
+// sign of a zero is not kept.  Straight-line: extreme magnitudes (nonzero below
+// 2^-900, or not finite), for which the remainder may be inexact, set `bad`, and the
+// caller computes that lane again with plain divisions.
+template <int B>  // B = 3 or 6
+__device__ __forceinline__ double div_3k(double x, bool &bad) {
+  const double y = 1.0 / B;
+  const double q = x * y;
+  const unsigned u = 2u * (unsigned)__double2hiint(x);
+  bad |= (u - 0x0f600000u >= 0xffe00000u - 0x0f600000u) && u != 0u;
+  return __fma_rn(__fma_rn(-(double)B, q, x), y, q);
+}
+template <int B>
+__device__ __forceinline__ float div_3k(float x, bool &bad) {
+  const float y = 1.0f / B;
+  const float q = x * y;
+  const unsigned u = 2u * __float_as_uint(x);
+  bad |= (u - 0x1b000000u >= 0xff000000u - 0x1b000000u) && u != 0u;  // 2^-100
+  return __fmaf_rn(__fmaf_rn(-(float)B, q, x), y, q);
+}
+template <typename R>
+__device__ __forceinline__ R div6(R x, bool &bad) { return div_3k<6>(x, bad); }
+template <typename R>
+__device__ __forceinline__ R div3(R x, bool &bad) { return div_3k<3>(x, bad); }
+
+// learned flux: 16 features of one MUSCL edge level in the flow's frame, in
+// units of the local variation sig, and the scale of the network's output
+template <typename TS>
+__device__ __forceinline__ void edge_features(const DMeshT<float> &m, const FusedArgs<float, TS> &a, int t, int cell,
+                                              int k, float vflux, float t1, float t2, float x1, float x2, float Tmean1,
+                                              float Tmean2, float gux, float guy, float gdx, float gdy, float exa,
+                                              float eyr, float c_lo1, float c_lo2, cix o1, cix o2, bool shared) {
+  const float sixth = 1.0f / 6.0f;
+  const bool fwd = vflux >= 0.0f;
+  const float tu = fwd ? t1 : t2, td = fwd ? t2 : t1;
+  const float xu = fwd ? x1 : -x2, xd = fwd ? x2 : -x1;
+  const float face = 0.5f * (Tmean1 + Tmean2);
+  const float sig = fabsf(td - tu) + (fabsf(xu) + fabsf(xd)) * sixth + 1e-6f * (fabsf(tu) + fabsf(td)) + 1e-20f;
+  const float inv = 1.0f / sig;
+  const cix ou = fwd ? o1 : o2;
+  const float cour = fminf(fabsf(vflux) * a.dt / (m.areasvol[ou] * m.hnode_new[ou]), 4.0f);
+  const float gx = fwd ? gux : gdx, gy = fwd ? guy : gdy;
+  const float trans = (-eyr * gx + exa * gy) * inv;
+  float f[16];
+  f[0] = (td - tu) * inv;
+  f[1] = xu * sixth * inv;
+  f[2] = xd * sixth * inv;
+  f[3] = (face - tu) * inv;
+  f[4] = cour;
+  f[5] = cour * cour;
+  f[6] = fwd ? c_lo1 : c_lo2;
+  f[7] = fwd ? c_lo2 : c_lo1;
+  f[8] = (float)k / (float)max(1, m.nl - 2);
+  f[9] = shared ? 1.0f : 0.0f;
+  f[10] = fabsf(f[0]);
+  f[11] = f[1] - f[2];
+  f[12] = (xu * xd > 0.0f) ? 1.0f : -1.0f;
+  f[13] = fminf(fabsf(f[1]), fabsf(f[2]));
+  f[14] = fmaxf(-8.0f, fminf(8.0f, trans));
+  f[15] = 1.0f;
+  __align__(16) __nv_bfloat16 h[16];
+  for (int q = 0; q < 16; q++) h[q] = __float2bfloat16_rn(f[q]);
+  uint4 *dst = reinterpret_cast<uint4 *>(a.feat[t] + (size_t)cell * 16);
+  dst[0] = reinterpret_cast<const uint4 *>(h)[0];
+  dst[1] = reinterpret_cast<const uint4 *>(h)[1];
+  a.fscale[t][cell] = -vflux * sig;
+}
+
+// Record of an edge: the column bases of its nodes and its triangles' nodes,
+// and its level limits (DMeshT::edge_idx).
+struct EdgeIdx {
+  int4 a, b, c;
+  __device__ __forceinline__ int tri_levels() const { return c.x; }
+  __device__ __forceinline__ int c1_levels() const { return c.y; }
+  __device__ __forceinline__ int c2_levels() const { return c.z; }
+  __device__ __forceinline__ int levels() const { return c.w; }
+};
+template <typename R>
+__device__ __forceinline__ EdgeIdx edge_idx(const DMeshT<R> &m, int e) {
+  const int4 *p = m.edge_idx + 3 * (size_t)e;
+  return EdgeIdx{p[0], p[1], p[2]};
+}
+
+// Both levels of an edge pair once more, with plain divisions: the lanes whose
+// operands lie outside div6's range.
 template <typename R, typename TS, int NT, int HOR, int LIM>
-__device__ __forceinline__ void edge_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk, int *smem) {
-  int *s_off = smem, *s_item = smem + kMaxItemsPerBlock + 1;
-  const CellMap cm = map_cells(m.edge_sched, blk, s_off, s_item);
-  const R re = R(kREarthD), sixth = R(1.0 / 6.0);
-  for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
-    const int j = s_item[lc], e = cm.i0 + j, k = lc - (s_off[j] - cm.c0);
-    const cix o = (cix)e * m.S + k;
-    const int2 nn = m.edge_nodes[e];
-    R vflux;
-    if (a.vflux_mode == 2) {
-      vflux = a.vflux[o];
-    } else {
-      vflux = edge_vflux(m, edge_ctx(m, e), a.vel, k);
-      if (LIM == LIM_FCT || a.vflux_mode == 1) a.vflux[o] = vflux;
-    }
-    const cix o1 = (cix)nn.x * m.S + k, o2 = (cix)nn.y * m.S + k;
-    if (HOR == HOR_UPW1) {
-      for (int t = 0; t < NT; t++) {
-        const R flo = (LIM == LIM_FCT) ? upw1_flux(vflux, ldT(a.T[t], o1, a.off[t]), ldT(a.T[t], o2, a.off[t])) : R(0);
-        il<NT>(a.adf_h, t, o) = upw1_flux(vflux, ldT(a.TAB[t], o1, a.off[t]), ldT(a.TAB[t], o2, a.off[t])) - flo;
-      }
-      continue;
-    }
-    // edge_up_dn_grad (lib/oce_muscl_adv.F90:383-527)
-    R gux[NTMAX], guy[NTMAX], gdx[NTMAX], gdy[NTMAX];
-    const int2 ud = m.up_dn[e];
-    bool shared = false;
-    if (ud.x >= 0 && ud.y >= 0) shared = (k + 1) <= min(m.nlev_node_min[nn.x], m.nlev_node_min[nn.y]) - 1;
-    if (shared) {
-      trxy_n(m, a.TAB, a.off, NT, ud.x, k, gux, guy);
-      trxy_n(m, a.TAB, a.off, NT, ud.y, k, gdx, gdy);
-    } else {
-      // node ring means, computed once per node-level by k_grad
-      for (int t = 0; t < NT; t++) {
-        ld_pair(a.gradn[t] + 2 * o1, gux[t], guy[t]);
-        ld_pair(a.gradn[t] + 2 * o2, gdx[t], gdy[t]);
-      }
-    }
-    const R ex = m.edge_dxdy[2 * e], ey = m.edge_dxdy[2 * e + 1], aa = m.edge_a[e];
-    R c_lo1 = R(1), c_lo2 = R(1);
-    if (HOR == HOR_MUSCL) {
-      c_lo1 = (m.nbl[nn.x] - (k + 1) >= 0) ? R(1) : R(0);
-      c_lo2 = (m.nbl[nn.y] - (k + 1) >= 0) ? R(1) : R(0);
-    }
+__device__ __noinline__ void edge_pair_slow(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int e, int k0) {
+  const EdgeIdx x = edge_idx(m, e);
+  const R *g = m.edge_geo + 16 * (size_t)e;
+#pragma unroll 1
+  for (int k = k0; k < min(k0 + 2, x.levels()); k++) {
+    const cix o = (cix)e * m.S + k, o1 = (cix)x.a.x + k, o2 = (cix)x.a.y + k;
+    const R vf = a.vflux[o];
+    const R c1 = HOR == HOR_MFCT || k < x.c1_levels() ? R(1) : R(0), c2 = HOR == HOR_MFCT || k < x.c2_levels() ? R(1) : R(0);
+#pragma unroll 1
     for (int t = 0; t < NT; t++) {
-      const R t1 = ldT(a.TAB[t], o1, a.off[t]), t2 = ldT(a.TAB[t], o2, a.off[t]);
-      R Tmean2, Tmean1;
-      // lib/oce_adv_tra_hor.F90:454-469 (MUSCL), :743-753 (MFCT, no c_lo)
-      const R x2 = R(2) * (t2 - t1) + ex * aa * gdx[t] + ey * re * gdy[t];
-      const R x1 = R(2) * (t2 - t1) + ex * aa * gux[t] + ey * re * guy[t];
-      if (HOR == HOR_MUSCL) {
-        Tmean2 = t2 - div_rcp(x2, R(6), sixth) * c_lo2;
-        Tmean1 = t1 + div_rcp(x1, R(6), sixth) * c_lo1;
+      auto B = [&](int base) { return ldT<R>(a.TAB[t], (cix)base + k, a.off[t]); };
+      R gux, guy, gdx, gdy;
+      if (k < x.tri_levels()) {
+        const R u0 = B(x.a.z), u1 = B(x.a.w), u2 = B(x.b.x), d0 = B(x.b.y), d1 = B(x.b.z), d2 = B(x.b.w);
+        gux = (g[0] * u0 + g[1] * u1) + g[2] * u2;
+        guy = (g[3] * u0 + g[4] * u1) + g[5] * u2;
+        gdx = (g[6] * d0 + g[7] * d1) + g[8] * d2;
+        gdy = (g[9] * d0 + g[10] * d1) + g[11] * d2;
       } else {
-        Tmean2 = t2 - div_rcp(x2, R(6), sixth);
-        Tmean1 = t1 + div_rcp(x1, R(6), sixth);
+        ld_pair(a.gradn[t] + 2 * (size_t)o1, gux, guy);
+        ld_pair(a.gradn[t] + 2 * (size_t)o2, gdx, gdy);
       }
-      const R cHO = (vflux + fabs(vflux)) * Tmean1 + (vflux - fabs(vflux)) * Tmean2;
-      const R ho = -(R(0.5) * (R(1) - a.ph) * cHO) - vflux * a.ph * R(0.5) * (Tmean1 + Tmean2);
-      const R flo = (LIM == LIM_FCT) ? upw1_flux(vflux, ldT(a.T[t], o1, a.off[t]), ldT(a.T[t], o2, a.off[t])) : R(0);
+      const R b1 = B(x.a.x), b2 = B(x.a.y);
+      const R x2 = R(2) * (b2 - b1) + g[12] * gdx + g[13] * gdy;
+      const R x1 = R(2) * (b2 - b1) + g[12] * gux + g[13] * guy;
+      const R Tmean2 = b2 - x2 / R(6) * c2, Tmean1 = b1 + x1 / R(6) * c1;
+      const R cHO = (vf + fabs(vf)) * Tmean1 + (vf - fabs(vf)) * Tmean2;
+      const R ho = -(R(0.5) * (R(1) - a.ph) * cHO) - vf * a.ph * R(0.5) * (Tmean1 + Tmean2);
+      const R flo = (LIM == LIM_FCT) ? upw1_flux(vf, ldT<R>(a.T[t], o1, a.off[t]), ldT<R>(a.T[t], o2, a.off[t])) : R(0);
       il<NT>(a.adf_h, t, o) = ho - flo;
-      if constexpr (sizeof(R) == 4 && HOR == HOR_MUSCL) {
-        if (a.feat[t]) {
-          // features in the flow's frame, in units of the local variation sig
-          const bool fwd = vflux >= R(0);
-          const R tu = fwd ? t1 : t2, td = fwd ? t2 : t1;
-          const R xu = fwd ? x1 : -x2, xd = fwd ? x2 : -x1;
-          const R face = R(0.5) * (Tmean1 + Tmean2);
-          const R sig = fabs(td - tu) + (fabs(xu) + fabs(xd)) * sixth + R(1e-6) * (fabs(tu) + fabs(td)) + R(1e-20);
-          const R inv = R(1) / sig;
-          const cix ou = fwd ? o1 : o2;
-          const R cour = fmin(fabs(vflux) * a.dt / (m.areasvol[ou] * m.hnode_new[ou]), R(4));
-          const R gx = fwd ? gux[t] : gdx[t], gy = fwd ? guy[t] : gdy[t];
-          const R trans = (-ey * re * gx + ex * aa * gy) * inv;
-          float f[16];
-          f[0] = (float)((td - tu) * inv);
-          f[1] = (float)(xu * sixth * inv);
-          f[2] = (float)(xd * sixth * inv);
-          f[3] = (float)((face - tu) * inv);
-          f[4] = (float)cour;
-          f[5] = (float)(cour * cour);
-          f[6] = (float)(fwd ? c_lo1 : c_lo2);
-          f[7] = (float)(fwd ? c_lo2 : c_lo1);
-          f[8] = (float)k / (float)max(1, m.nl - 2);
-          f[9] = shared ? 1.0f : 0.0f;
-          f[10] = fabsf(f[0]);
-          f[11] = f[1] - f[2];
-          f[12] = (xu * xd > R(0)) ? 1.0f : -1.0f;
-          f[13] = fminf(fabsf(f[1]), fabsf(f[2]));
-          f[14] = fmaxf(-8.0f, fminf(8.0f, (float)trans));
-          f[15] = 1.0f;
-          const int cell = cm.c0 + lc;
-          __align__(16) __nv_bfloat16 h[16];
-          for (int q = 0; q < 16; q++) h[q] = __float2bfloat16_rn(f[q]);
-          uint4 *dst = reinterpret_cast<uint4 *>(a.feat[t] + (size_t)cell * 16);
-          dst[0] = reinterpret_cast<const uint4 *>(h)[0];
-          dst[1] = reinterpret_cast<const uint4 *>(h)[1];
-          a.fscale[t][cell] = (float)(-vflux * sig);
-        }
-      }
+      if constexpr (HOR == HOR_MUSCL_FEAT)
+        edge_features(m, a, t, m.edge_sched.cell_off[e] + k, k, vf, b1, b2, x1, x2, Tmean1, Tmean2, gux, guy, gdx, gdy,
+                      g[12], g[13], c1, c2, o1, o2, k < x.tri_levels());
     }
   }
 }
 
-template <typename R, typename TS, int NT, int HOR, int LIM>
-__global__ void __launch_bounds__(kThreads, MinBlocks<R>::edge) k_edge(DMeshT<R> m, FusedArgs<R, TS> a) {
-  extern __shared__ int smem[];
-  edge_block<R, TS, NT, HOR, LIM>(m, a, blockIdx.x, smem);
+// One edge pair.  RING: some lane of the warp has a level without both
+// triangles (the schedule groups such pairs into warps of their own), which
+// takes the node ring means of k_grad instead.  LOADV: the edge volume fluxes
+// are stored (vflux_mode 2); otherwise they are computed here and stored.
+template <typename R, typename TS, int NT, int HOR, int LIM, bool LOADV, bool RING>
+__device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int e, int k, const EdgeIdx &x) {
+  const cix o = (cix)e * m.S + k;
+  R vf[2];
+  if constexpr (LOADV) {
+    ldv2(a.vflux + o, vf);
+  } else {
+    const EdgeCtx<R> c = edge_ctx(m, e);
+    vf[0] = edge_vflux(m, c, a.vel, k);
+    vf[1] = k + 1 < c.levels ? edge_vflux(m, c, a.vel, k + 1) : R(0);
+    stv2(a.vflux + o, vf);
+  }
+  const cix o1 = (cix)x.a.x + k, o2 = (cix)x.a.y + k;
+  if constexpr (HOR == HOR_UPW1) {
+    const R vp[2] = {vf[0] + fabs(vf[0]), vf[1] + fabs(vf[1])}, vm[2] = {vf[0] - fabs(vf[0]), vf[1] - fabs(vf[1])};
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      R b1[2], b2[2];
+      ld_pair_T(a.TAB[t], o1, a.off[t], b1);
+      ld_pair_T(a.TAB[t], o2, a.off[t], b2);
+      R t1[2] = {b1[0], b1[1]}, t2[2] = {b2[0], b2[1]};
+      if (LIM == LIM_FCT && a.T[t] != a.TAB[t]) {
+        ld_pair_T(a.T[t], o1, a.off[t], t1);
+        ld_pair_T(a.T[t], o2, a.off[t], t2);
+      }
+      R out[2];
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const R flo = (LIM == LIM_FCT) ? R(-0.5) * (t1[q] * vp[q] + t2[q] * vm[q]) : R(0);
+        out[q] = R(-0.5) * (b1[q] * vp[q] + b2[q] * vm[q]) - flo;
+      }
+      if (k + 1 >= x.levels()) out[1] = R(0);
+      st_pair_il<NT, 1>(a.adf_h, t, o, out);
+    }
+  } else {
+    bool bad = false;
+    // the loads of G tracers are all issued before the first is used
+    constexpr int G = NT > 2 ? 2 : NT;
+#pragma unroll
+    for (int t0 = 0; t0 < NT; t0 += G) {
+      R b1[G][2], b2[G][2], u[G][3][2], d[G][3][2], p1[G][4], p2[G][4];
+#pragma unroll
+      for (int i = 0; i < G; i++) {
+        const TS *B = a.TAB[t0 + i];
+        const R off = a.off[t0 + i];
+        ld_pair_T(B, o1, off, b1[i]);
+        ld_pair_T(B, o2, off, b2[i]);
+        ld_pair_T(B, (cix)x.a.z + k, off, u[i][0]);
+        ld_pair_T(B, (cix)x.a.w + k, off, u[i][1]);
+        ld_pair_T(B, (cix)x.b.x + k, off, u[i][2]);
+        ld_pair_T(B, (cix)x.b.y + k, off, d[i][0]);
+        ld_pair_T(B, (cix)x.b.z + k, off, d[i][1]);
+        ld_pair_T(B, (cix)x.b.w + k, off, d[i][2]);
+        if constexpr (RING) {
+          ldv4(a.gradn[t0 + i] + 2 * (size_t)o1, p1[i]);
+          ldv4(a.gradn[t0 + i] + 2 * (size_t)o2, p2[i]);
+        }
+      }
+      R g[16];
+      {
+        const R *ge = m.edge_geo + 16 * (size_t)e;
+        ldv4(ge, g);
+        ldv4(ge + 4, g + 4);
+        ldv4(ge + 8, g + 8);
+        ldv2(ge + 12, g + 12);
+      }
+      const R exa = g[12], eyr = g[13];
+      const R hph = R(0.5) * (R(1) - a.ph);
+      R out[2 * G];
+#pragma unroll
+      for (int i = 0; i < G; i++) {
+        const int t = t0 + i;
+        R t1[2] = {b1[i][0], b1[i][1]}, t2[2] = {b2[i][0], b2[i][1]};
+        if (LIM == LIM_FCT && a.T[t] != a.TAB[t]) {
+          ld_pair_T(a.T[t], o1, a.off[t], t1);
+          ld_pair_T(a.T[t], o2, a.off[t], t2);
+        }
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          const bool sh = !RING || k + q < x.tri_levels();
+          const R c1 = k + q < x.c1_levels() ? R(1) : R(0), c2 = k + q < x.c2_levels() ? R(1) : R(0);
+          // edge_up_dn_grad (lib/oce_muscl_adv.F90:383-527)
+          R gux = (g[0] * u[i][0][q] + g[1] * u[i][1][q]) + g[2] * u[i][2][q];
+          R guy = (g[3] * u[i][0][q] + g[4] * u[i][1][q]) + g[5] * u[i][2][q];
+          R gdx = (g[6] * d[i][0][q] + g[7] * d[i][1][q]) + g[8] * d[i][2][q];
+          R gdy = (g[9] * d[i][0][q] + g[10] * d[i][1][q]) + g[11] * d[i][2][q];
+          if (RING && !sh) {
+            gux = p1[i][2 * q]; guy = p1[i][2 * q + 1];
+            gdx = p2[i][2 * q]; gdy = p2[i][2 * q + 1];
+          }
+          // lib/oce_adv_tra_hor.F90:454-469 (MUSCL), :743-753 (MFCT, no c_lo)
+          const R x2 = R(2) * (b2[i][q] - b1[i][q]) + exa * gdx + eyr * gdy;
+          const R x1 = R(2) * (b2[i][q] - b1[i][q]) + exa * gux + eyr * guy;
+          R Tmean2, Tmean1;
+          if (HOR != HOR_MFCT) {
+            Tmean2 = b2[i][q] - div6(x2, bad) * c2;
+            Tmean1 = b1[i][q] + div6(x1, bad) * c1;
+          } else {
+            Tmean2 = b2[i][q] - div6(x2, bad);
+            Tmean1 = b1[i][q] + div6(x1, bad);
+          }
+          const R vp = vf[q] + fabs(vf[q]), vm = vf[q] - fabs(vf[q]);
+          const R cHO = vp * Tmean1 + vm * Tmean2;
+          const R ho = -(hph * cHO) - vf[q] * a.ph * R(0.5) * (Tmean1 + Tmean2);
+          const R flo = (LIM == LIM_FCT) ? R(-0.5) * (t1[q] * vp + t2[q] * vm) : R(0);
+          out[2 * i + q] = ho - flo;
+          if constexpr (HOR == HOR_MUSCL_FEAT) {
+            if (k + q < x.levels())
+              edge_features(m, a, t, m.edge_sched.cell_off[e] + k + q, k + q, vf[q], b1[i][q], b2[i][q], x1, x2, Tmean1,
+                            Tmean2, gux, guy, gdx, gdy, exa, eyr, c1, c2, o1 + q, o2 + q, sh);
+          }
+        }
+      }
+      // a dry second level holds zero: the node kernels add it without a test
+      if (k + 1 >= x.levels())
+#pragma unroll
+        for (int i = 0; i < G; i++) out[2 * i + 1] = R(0);
+      st_pair_il<NT, G>(a.adf_h, t0, o, out);
+    }
+    if (bad) edge_pair_slow<R, TS, NT, HOR, LIM>(m, a, e, k);
+  }
+}
+
+// The edge pairs of `per` consecutive warps of the schedule; the records of
+// the next pair and the map entry of the one after it are loaded ahead of the
+// current pair's arithmetic, so that a pair costs one memory latency instead of
+// three dependent ones.
+template <typename R, typename TS, int NT, int HOR, int LIM, bool LOADV>
+__device__ __forceinline__ void edge_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk, int per) {
+  const DPairs &s = m.edge_pairs;
+  int warp = (blk * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5)) * per;
+  const int end = min(warp + per, s.nwarps);
+  if (warp >= end) return;
+  PairLane nxt = pair_lane(s, warp);
+  EdgeIdx idx = edge_idx(m, nxt.item);
+  PairLane nn = warp + 1 < end ? pair_lane(s, warp + 1) : nxt;
+  do {
+    const PairLane c = nxt;
+    const EdgeIdx x = idx;
+    if (++warp < end) {
+      nxt = nn;
+      idx = edge_idx(m, nxt.item);
+      if (warp + 1 < end) nn = pair_lane(s, warp + 1);
+    }
+    if (c.on) {
+      if (HOR != HOR_UPW1 && c.ring) edge_pair<R, TS, NT, HOR, LIM, LOADV, true>(m, a, c.item, c.k, x);
+      else edge_pair<R, TS, NT, HOR, LIM, LOADV, false>(m, a, c.item, c.k, x);
+    }
+  } while (warp < end);
+}
+
+template <typename R, typename TS, int NT, int HOR, int LIM, bool LOADV>
+__global__ void __launch_bounds__(kEdgeThreads, StepBlocks<R, NT>::edge)
+    k_edge(const __grid_constant__ DMeshT<R> m, const __grid_constant__ FusedArgs<R, TS> a, int per) {
+  edge_block<R, TS, NT, HOR, LIM, LOADV>(m, a, blockIdx.x, per);
 }
 
 // ---------------------------------------------------------------------------
-// k_col1: LO solution and vertical fluxes
+// Node columns: lanes hold level pairs, columns are packed whole into warps
+// (DMeshT::node_pairs), so the vertical stencils exchange values by shuffles and
+// the kernels need neither shared memory nor block barriers.
 // ---------------------------------------------------------------------------
+constexpr unsigned kFull = 0xffffffffu;
+
+// Node record (DMeshT::nrec, ne6): levels, the first six incident edges in
+// ascending edge id, and how many there are.
+struct NodeRec {
+  int4 h;
+  int4 e[3];
+  __device__ __forceinline__ int nlev() const { return h.x & 0xffff; }
+  __device__ __forceinline__ int degree() const { return (int)((unsigned)h.x >> 16); }
+  __device__ __forceinline__ int nlev_min() const { return h.y & 0x7fffffff; }
+  __device__ __forceinline__ bool ring_full() const { return h.y < 0; }
+  __device__ __forceinline__ int levels(int i) const { return ((i < 3 ? h.z : h.w) >> (10 * (i % 3))) & 1023; }
+  __device__ __forceinline__ unsigned edge(int i) const { return (unsigned)(i % 2 ? e[i / 2].z : e[i / 2].x); }
+  __device__ __forceinline__ unsigned other(int i) const { return (unsigned)(i % 2 ? e[i / 2].w : e[i / 2].y); }
+};
+template <typename R>
+__device__ __forceinline__ NodeRec node_rec(const DMeshT<R> &m, int n) {
+  NodeRec r;
+  r.h = m.nrec[n];
+  const int4 *p = m.ne6 + 3 * (size_t)n;
+  r.e[0] = p[0];
+  r.e[1] = p[1];
+  r.e[2] = p[2];
+  return r;
+}
+// f(cell of the edge, cell of the other node, node is the edge's second, edge
+// levels) for every incident edge in ascending edge id: the six of the record
+// unrolled (fewer: the rest have no levels), those beyond from the lists.
+template <typename R, typename F>
+__device__ __forceinline__ void for_edges(const DMeshT<R> &m, int n, int k, const NodeRec &rec, F f) {
+#pragma unroll
+  for (int i = 0; i < 6; i++)
+    f((cix)rec.edge(i) + k, (cix)(rec.other(i) & 0x7fffffffu) + k, (rec.other(i) >> 31) != 0, rec.levels(i));
+  if (rec.degree() > 6) {
+    const int p0 = m.ne_ptr[n];
+    for (int p = p0 + 6; p < p0 + rec.degree(); p++) {
+      const int4 q = m.ne4[p];
+      f((cix)(q.x >> 1) * m.S + k, (cix)q.w + k, (q.x & 1) != 0, q.z);
+    }
+  }
+}
+
+// a / b given y = RN(1 / b), correctly rounded (see div_rcp), straight-line:
+// numerators outside [2^-900, 2^900] other than zero set `bad` and the caller
+// divides again.  The sign of a zero result is not kept (no output of the step
+// depends on the sign of a zero quotient).
+__device__ __forceinline__ double div_fast(double a, double b, double y, bool &bad) {
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  const unsigned u = 2u * (unsigned)__double2hiint(a);
+  bad |= (u - 0x0f600000u > 0xf0800000u - 0x0f600000u) && u != 0u;
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+__device__ __forceinline__ float div_fast(float a, float b, float y, bool &bad) {
+  float q = a * y;
+  q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+  const unsigned u = 2u * __float_as_uint(a);
+  bad |= (u - 0x1b000000u > 0xe3000000u - 0x1b000000u) && u != 0u;
+  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
+// PPM weights of one column level (lib/oce_adv_tra_ver.F90:525-553): c1, c2, c3
+// of layer k's slope, and A .. E of the value at interface k (between layers
+// k - 1 and k) from the thicknesses h[-2 .. 1] around it.
+template <typename R>
+__device__ __forceinline__ void ppm_slope_weights(R hm, R h, R hp, R *c) {
+  c[0] = h / (hm + h + hp);
+  c[1] = (R(2) * hm + h) / (hp + h);
+  c[2] = (h + R(2) * hp) / (hm + h);
+}
+template <typename R>
+__device__ __forceinline__ void ppm_face_weights(R dzjm1, R dzj, R dzjp1, R dzjp2, R *c) {
+  c[0] = dzj / (dzj + dzjp1);
+  c[1] = R(1) / (dzjm1 + dzj + dzjp1 + dzjp2);
+  c[2] = (R(2) * dzjp1 * dzj) / (dzj + dzjp1) *
+         ((dzjm1 + dzj) / (R(2) * dzj + dzjp1) - (dzjp2 + dzjp1) / (R(2) * dzjp1 + dzj));
+  c[3] = dzj * (dzjm1 + dzj) / (R(2) * dzj + dzjp1);
+  c[4] = dzjp1 * (dzjp1 + dzjp2) / (dzj + R(2) * dzjp1);
+}
+
+// Level tables (DMeshT::ltab), S entries each, where every column has the same
+// thicknesses (uniform z levels): the PPM weights, 1/hnode, and for any mesh
+// QR4C's level distances, their reciprocal and its two offsets.
+enum { LT_C1 = 0, LT_C2, LT_C3, LT_A, LT_B, LT_C, LT_D, LT_E, LT_YH, LT_ZD, LT_YZD, LT_ZA, LT_ZB, LT_COUNT };
+template <typename R>
+__global__ void k_level_tables(DMeshT<R> m, int n, R *t) {
+  const int S = m.S;
+  const R *HN = m.hnode_new + (size_t)n * S, *H = m.hnode + (size_t)n * S;
+  const int nln = m.nlev_node[n] - 1;
+  for (int k = threadIdx.x; k < S; k += blockDim.x) {
+    R c[3] = {0, 0, 0}, f[5] = {0, 0, 0, 0, 0};
+    if (m.uniform_h && k >= 1 && k <= nln - 2) ppm_slope_weights(HN[k - 1], HN[k], HN[k + 1], c);
+    if (m.uniform_h && k >= 2 && k <= nln - 2) ppm_face_weights(HN[k - 2], HN[k - 1], HN[k], HN[k + 1], f);
+    for (int i = 0; i < 3; i++) t[(LT_C1 + i) * S + k] = c[i];
+    for (int i = 0; i < 5; i++) t[(LT_A + i) * S + k] = f[i];
+    t[LT_YH * S + k] = m.uniform_h && k < nln ? R(1) / H[k] : R(0);
+    const bool in = k >= 1 && k < m.nl - 1;
+    const R zd = in ? m.Z[k - 1] - m.Z[k] : R(1);
+    t[LT_ZD * S + k] = zd;
+    t[LT_YZD * S + k] = R(1) / zd;
+    t[LT_ZA * S + k] = in ? m.zbar[k] - m.Z[k] : R(0);
+    t[LT_ZB * S + k] = in ? m.zbar[k] - m.Z[k - 1] : R(0);
+  }
+}
+
 // PPM slope of layer j (1-based) with the limiter of lib/oce_adv_tra_ver.F90:
 // 525-540; c1, c2, c3 are the geometric factors of that layer.
 template <typename R>
@@ -484,373 +665,551 @@ __device__ __forceinline__ R ppm_slope(R Tm1, R T0, R Tp1, R c1, R c2, R c3) {
     d = R(0);
   return d;
 }
-
-template <typename R, typename TS, int NT, int VER, int LIM>
-__device__ __forceinline__ void col1_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk, int *smem) {
-  int *s_off = smem, *s_item = smem + kMaxItemsPerBlock + 1;
-  R *s_slope = (R *)(smem + kMaxItemsPerBlock + 1 + kMaxCellsPerBlock + 1);  // 16-byte aligned below
-  s_slope = (R *)(((uintptr_t)s_slope + 15) & ~(uintptr_t)15);
-  R *s_tv = s_slope + NT * kMaxCellsPerBlock;
-  // the vertical LO fluxes of stage C reuse the slopes' storage, dead after
-  // stage B: two arrays of shared memory instead of three leave more of the
-  // SM's unified L1 to the column and neighbour re-reads
-  R *s_fv = s_slope;
-  const CellMap cm = map_cells(m.node_sched, blk, s_off, s_item);
-  const Incidence inc = stage_incidence<StageIncidence<R>::col1>(m, cm, s_tv + NT * kMaxCellsPerBlock);
-  const int S = m.S;
-
-  // stage A: PPM slopes
-  for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
-    const int j = s_item[lc], n = cm.i0 + j, k = lc - (s_off[j] - cm.c0), nz = k + 1;
-    if (VER == VER_PPM) {
-      const int nlev = m.nlev_node[n];
-      if (nz >= 2 && nz <= nlev - 2) {
-        const R *HN = m.hnode_new + (cix)n * S;
-        const R dzjm1 = HN[k - 1], dzj = HN[k], dzjp1 = HN[k + 1];
-        const R c1 = dzj / (dzjm1 + dzj + dzjp1);
-        const R c2 = (R(2) * dzjm1 + dzj) / (dzjp1 + dzj);
-        const R c3 = (dzj + R(2) * dzjp1) / (dzjm1 + dzj);
-        for (int t = 0; t < NT; t++) {
-          const TS *Tc = a.TAB[t] + (cix)n * S;
-          s_slope[t * kMaxCellsPerBlock + lc] = ppm_slope(ldT(Tc, k - 1, a.off[t]), ldT(Tc, k, a.off[t]), ldT(Tc, k + 1, a.off[t]), c1, c2, c3);
-        }
-      }
-    }
-  }
-  __syncthreads();
-
-  // stage B: PPM interface values tv(i), interface i = nz (top of layer nz)
-  if (VER == VER_PPM) {
-    for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
-      const int j = s_item[lc], n = cm.i0 + j, k = lc - (s_off[j] - cm.c0), i = k + 1;
-      const int nlev = m.nlev_node[n];
-      const R *HN = m.hnode_new + (cix)n * S;
-      const R *Wc = a.W + (cix)n * S;
-      if (i == 1) {
-        for (int t = 0; t < NT; t++) s_tv[t * kMaxCellsPerBlock + lc] = ldT(a.TAB[t], (cix)n * S, a.off[t]);
-      } else if (i == nlev - 1) {
-        const R s = sgn1(Wc[nlev - 2]);
-        for (int t = 0; t < NT; t++) {
-          const TS *Tc = a.TAB[t] + (cix)n * S;
-          s_tv[t * kMaxCellsPerBlock + lc] = -ldT(Tc, nlev - 3, a.off[t]) * fmin2(s, R(0)) + ldT(Tc, nlev - 2, a.off[t]) * fmax2(s, R(0));
-        }
-      } else if (i == 2) {
-        for (int t = 0; t < NT; t++) {
-          const TS *Tc = a.TAB[t] + (cix)n * S;
-          s_tv[t * kMaxCellsPerBlock + lc] = R(0.5) * (ldT(Tc, 0, a.off[t]) + ldT(Tc, 1, a.off[t]));
-        }
-      } else {
-        // lib/oce_adv_tra_ver.F90:545-553 with nz = i - 1
-        const int nzz = i - 1;  // 1-based layer above the interface
-        const R dzjm1 = HN[nzz - 2], dzj = HN[nzz - 1], dzjp1 = HN[nzz], dzjp2 = HN[nzz + 1];
-        const R A = dzj / (dzj + dzjp1);
-        const R B = R(1) / (dzjm1 + dzj + dzjp1 + dzjp2);
-        const R C = (R(2) * dzjp1 * dzj) / (dzj + dzjp1) *
-                    ((dzjm1 + dzj) / (R(2) * dzj + dzjp1) - (dzjp2 + dzjp1) / (R(2) * dzjp1 + dzj));
-        const R D = dzj * (dzjm1 + dzj) / (R(2) * dzj + dzjp1);
-        const R E = dzjp1 * (dzjp1 + dzjp2) / (dzj + R(2) * dzjp1);
-        for (int t = 0; t < NT; t++) {
-          const TS *Tc = a.TAB[t] + (cix)n * S;
-          const R T0 = ldT(Tc, nzz - 1, a.off[t]), T1 = ldT(Tc, nzz, a.off[t]);
-          const R dj = s_slope[t * kMaxCellsPerBlock + lc - 1];   // layer nzz
-          const R djp1 = s_slope[t * kMaxCellsPerBlock + lc];     // layer nzz + 1
-          s_tv[t * kMaxCellsPerBlock + lc] = T0 + A * (T1 - T0) + B * (C * (T1 - T0) - D * djp1 + E * dj);
-        }
-      }
-    }
-    __syncthreads();
-  }
-
-  // stage C: fluxes at interface i = nz (and the bottom one for the deepest layer)
-  for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
-    const int j = s_item[lc], n = cm.i0 + j, k = lc - (s_off[j] - cm.c0);
-    const cix col = (cix)n * S;
-    const int nlev = m.nlev_node[n];
-    const R *Wc = a.W + col, *Ac = m.area + col;
-    const int i_last = (k + 2 == nlev) ? k + 2 : k + 1;
-    for (int i = k + 1; i <= i_last; i++) {
-      R lov[NTMAX], hov[NTMAX];
-      for (int t = 0; t < NT; t++) lov[t] = R(0);
-      if (LIM == LIM_FCT) {
-        for (int t = 0; t < NT; t++) {
-          Col<R, TS> cT;
-          cT.T = a.T[t] + col; cT.W = Wc; cT.A = Ac; cT.nlev = nlev; cT.off = a.off[t];
-          lov[t] = ver_upw1(cT, i);
-        }
-      }
-      if (VER == VER_PPM) {
-        // lib/oce_adv_tra_ver.F90:597-639
-        if (i == nlev) {
-          for (int t = 0; t < NT; t++) hov[t] = R(0) - lov[t];
-        } else if (i == 1) {
-          for (int t = 0; t < NT; t++) hov[t] = -(s_tv[t * kMaxCellsPerBlock + lc] * Wc[0] * Ac[0]) - lov[t];
-        } else {
-          const R w = Wc[i - 1];
-          if (!(w > R(0)) && !(w < R(0))) {
-            for (int t = 0; t < NT; t++) hov[t] = R(0) - lov[t];
-          } else {
-            const int jl = (w > R(0)) ? i : i - 1;              // supplying layer (1-based)
-            const int sl = lc + (jl - i);                        // its cell slot
-            const R dzj = m.hnode[col + jl - 1];
-            const R x = (w > R(0)) ? fmin2(w * a.dt / dzj, R(1)) : fmin2(-(w * a.dt / dzj), R(1));
-            const R two3 = R(2.0 / 3.0), sixth = R(1.0 / 6.0);
-            for (int t = 0; t < NT; t++) {
-              const R Tc = ldT(a.TAB[t], col + jl - 1, a.off[t]);
-              R aL = s_tv[t * kMaxCellsPerBlock + sl];
-              R aR = (jl + 1 == nlev) ? ldT(a.TAB[t], col + nlev - 2, a.off[t]) : s_tv[t * kMaxCellsPerBlock + sl + 1];
-              if ((aR - Tc) * (Tc - aL) <= R(0)) { aL = Tc; aR = Tc; }
-              // x / 6 by the corrected reciprocal (correctly rounded, as in the MUSCL fluxes)
-              if ((aR - aL) * (Tc - R(0.5) * (aL + aR)) > div_rcp((aR - aL) * (aR - aL), R(6), sixth)) aL = R(3) * Tc - R(2) * aR;
-              if ((aR - aL) * (Tc - R(0.5) * (aR + aL)) < -div_rcp((aR - aL) * (aR - aL), R(6), sixth)) aR = R(3) * Tc - R(2) * aL;
-              const R aj = R(6) * (Tc - R(0.5) * (aL + aR));
-              R tt;
-              if (w > R(0)) tt = (-aL - R(0.5) * x * (aR - aL + (R(1) - two3 * x) * aj));
-              else tt = (-aR + R(0.5) * x * (aR - aL - (R(1) - two3 * x) * aj));
-              hov[t] = tt * Ac[i - 1] * w - lov[t];
-            }
-          }
-        }
-      } else {
-        for (int t = 0; t < NT; t++) {
-          Col<R, TS> cA;
-          cA.T = a.TAB[t] + col; cA.W = Wc; cA.A = Ac; cA.nlev = nlev; cA.off = a.off[t];
-          if (VER == VER_QR4C) hov[t] = ver_qr4c(cA, m.zbar, m.Z, i, a.pv, lov[t]);
-          else if (VER == VER_CDIFF) hov[t] = ver_cdiff(cA, i, lov[t]);
-          else hov[t] = ver_upw1(cA, i) - lov[t];
-        }
-      }
-      for (int t = 0; t < NT; t++) {
-        il<NT>(a.adf_v, t, col + i - 1) = hov[t];
-        if (LIM == LIM_FCT && i == k + 1) s_fv[t * kMaxCellsPerBlock + lc] = lov[t];
-      }
-    }
-  }
-  if (LIM != LIM_FCT) return;
-  __syncthreads();
-
-  // stage D: horizontal LO gather and the LO solution
-  // (lib/oce_adv_tra_driver.F90:122-181, :202-211)
-  for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
-    const int j = s_item[lc], n = cm.i0 + j, k = lc - (s_off[j] - cm.c0), nz = k + 1;
-    const cix o = (cix)n * S + k;
-    const int nlev = m.nlev_node[n];
-    R acc[NTMAX], tself[NTMAX];
-    for (int t = 0; t < NT; t++) {
-      acc[t] = R(0);
-      tself[t] = ldT(a.T[t], o, a.off[t]);
-    }
-    for (int p = inc.nep[j] - inc.sub, pe = inc.nep[j + 1] - inc.sub; p < pe; p += kGChunkCol1) {
-      int4 qs[kGChunkCol1];
-      R vfs[kGChunkCol1], tos[kGChunkCol1][NT];
-#pragma unroll
-      for (int u = 0; u < kGChunkCol1; u++) {
-        qs[u] = inc.ne[min(p + u, pe - 1)];
-        vfs[u] = a.vflux[(cix)(qs[u].x >> 1) * S + k];
-        const cix oo = (cix)qs[u].w + k;  // the edge's other node (column base in .w)
-        for (int t = 0; t < NT; t++) tos[u][t] = ldT(a.T[t], oo, a.off[t]);
-      }
-#pragma unroll
-      for (int u = 0; u < kGChunkCol1; u++) {
-        if (p + u >= pe || nz > qs[u].z) continue;
-        const bool second = qs[u].x & 1;
-        for (int t = 0; t < NT; t++) {
-          // upw1_flux(vf, T(first node), T(second node))
-          const R F = second ? upw1_flux(vfs[u], tos[u][t], tself[t]) : upw1_flux(vfs[u], tself[t], tos[u][t]);
-          acc[t] = second ? acc[t] - F : acc[t] + F;
-        }
-      }
-    }
-    const R asv = m.areasvol[o], hn = m.hnode_new[o], h = m.hnode[o];
-    const R yasv = m.rcp[o], yhn = m.rcp[m.rcp_plane + o];  // reciprocal planes (k_rcp_planes)
-    for (int t = 0; t < NT; t++) {
-      const R fk = s_fv[t * kMaxCellsPerBlock + lc];
-      const R fk1 = (k + 2 == nlev) ? R(0) : s_fv[t * kMaxCellsPerBlock + lc + 1];
-      const R num = tself[t] * h + div_rcp((acc[t] + (fk - fk1)) * a.dt, asv, yasv);
-      il<NT>(a.lo, t, o) = div_rcp(num, hn, yhn);
-    }
-  }
+// PPM flux through an interface with velocity w (not zero) out of the layer of
+// value Tc with face values aL, aR and Courant number x (lib/oce_adv_tra_ver.F90:
+// 597-639); D divides by 6.
+template <typename R, typename D>
+__device__ __forceinline__ R ppm_face(R w, R Tc, R aL, R aR, R x, D div) {
+  const R two3 = R(2.0 / 3.0);
+  if ((aR - Tc) * (Tc - aL) <= R(0)) { aL = Tc; aR = Tc; }
+  if ((aR - aL) * (Tc - R(0.5) * (aL + aR)) > div((aR - aL) * (aR - aL))) aL = R(3) * Tc - R(2) * aR;
+  if ((aR - aL) * (Tc - R(0.5) * (aR + aL)) < -div((aR - aL) * (aR - aL))) aR = R(3) * Tc - R(2) * aL;
+  const R aj = R(6) * (Tc - R(0.5) * (aL + aR));
+  const R dn = (-aL - R(0.5) * x * (aR - aL + (R(1) - two3 * x) * aj));
+  const R up = (-aR + R(0.5) * x * (aR - aL - (R(1) - two3 * x) * aj));
+  return w > R(0) ? dn : up;
 }
 
-template <typename R, typename TS, int NT, int VER, int LIM>
-__global__ void __launch_bounds__(kThreads, MinBlocks<R>::col1) k_col1(DMeshT<R> m, FusedArgs<R, TS> a) {
-  extern __shared__ int smem[];
-  col1_block<R, TS, NT, VER, LIM>(m, a, blockIdx.x, smem);
+// vertical LO flux at interface k (0-based: top of layer k) of values Tk (layer
+// k) and Tm (layer k - 1); adv_tra_ver_upw1 (lib/oce_adv_tra_ver.F90:300-327)
+template <typename R>
+__device__ __forceinline__ R upw_v(R Tk, R Tm, R w, R A, int k, int nln) {
+  const R top = -(w * Tk * A);
+  const R in = -(R(0.5) * (Tk * (w + fabs(w)) + Tm * (w - fabs(w))) * A);
+  return k == 0 ? top : (k >= nln ? R(0) : in);
+}
+
+// The antidiffusive vertical fluxes of a pair's interfaces once more, level by
+// level from memory with plain divisions (operands outside the fast divisions'
+// range).
+template <typename R, typename TS, int NT, int G, int VER, int LIM>
+__device__ __noinline__ void col1_vert_slow(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, int n, int k0) {
+  const cix col = (cix)n * m.S;
+  const int nlev = m.nlev_node[n], nln = nlev - 1;
+  const R *W = a.W + col, *A = m.area + col, *H = m.hnode + col, *HN = m.hnode_new + col;
+#pragma unroll 1
+  for (int k = k0; k < min(k0 + 2, nln); k++)
+#pragma unroll 1
+    for (int t = t0; t < t0 + G; t++) {
+      auto T = [&](int j) { return ldT<R>(a.T[t], col + j, a.off[t]); };
+      auto B = [&](int j) { return ldT<R>(a.TAB[t], col + j, a.off[t]); };
+      const R lov = LIM == LIM_FCT ? upw_v(T(k), T(max(k - 1, 0)), W[k], A[k], k, nln) : R(0);
+      R hov;
+      if (VER == VER_PPM) {
+        auto slope = [&](int j) {
+          R c[3];
+          ppm_slope_weights(HN[j - 1], HN[j], HN[j + 1], c);
+          return ppm_slope(B(j - 1), B(j), B(j + 1), c[0], c[1], c[2]);
+        };
+        auto tv = [&](int j) {
+          if (j == 0) return B(0);
+          if (j == nln) return B(nln - 1);
+          if (j == nln - 1) {
+            const R s = sgn1(W[j]);
+            return -B(j - 1) * fmin2(s, R(0)) + B(j) * fmax2(s, R(0));
+          }
+          if (j == 1) return R(0.5) * (B(0) + B(1));
+          R c[5];
+          ppm_face_weights(HN[j - 2], HN[j - 1], HN[j], HN[j + 1], c);
+          const R T0 = B(j - 1), T1 = B(j);
+          return T0 + c[0] * (T1 - T0) + c[1] * (c[2] * (T1 - T0) - c[3] * slope(j) + c[4] * slope(j - 1));
+        };
+        const R w = W[k];
+        if (k == 0) {
+          hov = -(tv(0) * w * A[0]) - lov;
+        } else if (!(w > R(0)) && !(w < R(0))) {
+          hov = R(0) - lov;
+        } else {
+          const int j = w > R(0) ? k : k - 1;
+          const R d = w * a.dt / H[j];
+          const R x = w > R(0) ? fmin2(d, R(1)) : fmin2(-d, R(1));
+          hov = ppm_face(w, B(j), tv(j), tv(j + 1), x, [](R z) { return z / R(6); }) * A[k] * w - lov;
+        }
+      } else {
+        Col<R, TS> c;
+        c.T = a.TAB[t] + col; c.W = W; c.A = A; c.nlev = nlev; c.off = a.off[t];
+        hov = VER == VER_QR4C ? ver_qr4c(c, m.zbar, m.Z, k + 1, a.pv, lov)
+                              : (VER == VER_CDIFF ? ver_cdiff(c, k + 1, lov) : ver_upw1(c, k + 1) - lov);
+      }
+      il<NT>(a.adf_v, t, col + k) = hov;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// k_col1: LO solution and vertical fluxes
+// ---------------------------------------------------------------------------
+// UNI: the mesh has uniform z levels and the level tables hold the PPM weights
+// and reciprocal thicknesses; otherwise they are formed here.
+template <typename R, typename TS, int NT, int G, int VER, int LIM, bool UNI>
+__device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, const PairLane &l) {
+  const int n = l.item, k = l.k, S = m.S;
+  const cix col = (cix)n * S, o = col + k;
+  const NodeRec rec = node_rec(m, n);
+  const int nln = rec.nlev() - 1;
+  const int km = max(k - 1, 0), kp = min(k + 2, S - 1);
+  R W[2], A[2];
+  ldv2(a.W + o, W);
+  ldv2(m.area + o, A);
+  // values k - 1 .. k + 2 of valuesAB, and k - 1 .. k + 1 of the values
+  R x[G][4], ts[G][3] = {};
+#pragma unroll
+  for (int t = 0; t < G; t++) {
+    x[t][0] = ldT<R>(a.TAB[t0 + t], col + km, a.off[t0 + t]);
+    ld_pair_T(a.TAB[t0 + t], o, a.off[t0 + t], x[t] + 1);
+    x[t][3] = ldT<R>(a.TAB[t0 + t], col + kp, a.off[t0 + t]);
+    if (LIM == LIM_FCT) {
+      ts[t][0] = x[t][0];
+      ts[t][1] = x[t][1];
+      ts[t][2] = x[t][2];
+      if (a.T[t0 + t] != a.TAB[t0 + t]) {
+        ts[t][0] = ldT<R>(a.T[t0 + t], col + km, a.off[t0 + t]);
+        ld_pair_T(a.T[t0 + t], o, a.off[t0 + t], ts[t] + 1);
+      }
+    }
+  }
+  if (k + 1 >= nln)  // the second level is dry, whatever its cell holds
+#pragma unroll
+    for (int t = 0; t < G; t++) x[t][2] = ts[t][2] = R(0);
+  // horizontal LO gather (lib/oce_adv_tra_driver.F90:122-181): with the edge
+  // flux's sign turned to point out of this node, both ends' contributions are
+  // the same expression
+  R acc[G][2];
+  if (LIM == LIM_FCT) {
+#pragma unroll
+    for (int t = 0; t < G; t++) acc[t][0] = acc[t][1] = R(0);
+    for_edges(m, n, k, rec, [&](cix oe, cix oo, bool second, int lev) {
+      const bool w0 = k < lev, w1 = k + 1 < lev;
+      R v[2], to[G][2];
+      ldv2_if(a.vflux + oe, w0, v);
+#pragma unroll
+      for (int t = 0; t < G; t++) ld_pair_T_if(a.T[t0 + t], oo, a.off[t0 + t], w0, to[t]);
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const R vo = second ? -v[q] : v[q];
+        const R vp = vo + fabs(vo), vm = vo - fabs(vo);
+#pragma unroll
+        for (int t = 0; t < G; t++) {
+          const R F = R(-0.5) * (ts[t][1 + q] * vp + to[t][q] * vm);
+          acc[t][q] = acc[t][q] + (q == 0 ? F : (w1 ? F : R(0)));
+        }
+      }
+    });
+  }
+
+  bool bad = false;
+  R hov[2 * G], lov[G][2];
+#pragma unroll
+  for (int t = 0; t < G; t++)
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+      lov[t][q] = LIM == LIM_FCT ? upw_v(ts[t][1 + q], ts[t][q], W[q], A[q], k + q, nln) : R(0);
+  if constexpr (VER == VER_PPM) {
+    R c1[2], c2[2], c3[2], fA[2], fB[2], fC[2], fD[2], fE[2], h[3], yh[3];
+    if constexpr (UNI) {
+      const R *lt = m.ltab + k;
+      ldv2(lt + LT_C1 * S, c1); ldv2(lt + LT_C2 * S, c2); ldv2(lt + LT_C3 * S, c3);
+      ldv2(lt + LT_A * S, fA); ldv2(lt + LT_B * S, fB); ldv2(lt + LT_C * S, fC);
+      ldv2(lt + LT_D * S, fD); ldv2(lt + LT_E * S, fE);
+      h[0] = m.hT[km]; ldv2(m.hT + k, h + 1);
+      yh[0] = m.ltab[LT_YH * S + km]; ldv2(lt + LT_YH * S, yh + 1);
+    } else {
+      const R *HN = m.hnode_new + col, *H = m.hnode + col;
+      const R z[5] = {HN[max(k - 2, 0)], HN[km], HN[k], HN[k + 1], HN[kp]};
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        R c[3], f[5];
+        ppm_slope_weights(z[1 + q], z[2 + q], z[3 + q], c);
+        ppm_face_weights(z[q], z[1 + q], z[2 + q], z[3 + q], f);
+        c1[q] = c[0]; c2[q] = c[1]; c3[q] = c[2];
+        fA[q] = f[0]; fB[q] = f[1]; fC[q] = f[2]; fD[q] = f[3]; fE[q] = f[4];
+      }
+      h[0] = H[km]; h[1] = H[k]; h[2] = H[k + 1];
+    }
+#pragma unroll
+    for (int t = 0; t < G; t++) {
+      R s[2], tv[4];
+#pragma unroll
+      for (int q = 0; q < 2; q++) s[q] = ppm_slope(x[t][q], x[t][q + 1], x[t][q + 2], c1[q], c2[q], c3[q]);
+      const R sm = __shfl_up_sync(kFull, s[1], 1);
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        // interface values (lib/oce_adv_tra_ver.F90:545-553 with nz = k + q)
+        const int kk = k + q;
+        const R T0 = x[t][q], T1 = x[t][q + 1];
+        R v = T0 + fA[q] * (T1 - T0) + fB[q] * (fC[q] * (T1 - T0) - fD[q] * s[q] + fE[q] * (q == 0 ? sm : s[0]));
+        if (kk == 1) v = R(0.5) * (T0 + T1);
+        const R sg = sgn1(W[q]);
+        if (kk == nln - 1) v = -T0 * fmin2(sg, R(0)) + T1 * fmax2(sg, R(0));
+        if (kk == 0) v = T1;
+        tv[1 + q] = v;
+      }
+      tv[0] = __shfl_up_sync(kFull, tv[2], 1);
+      tv[3] = __shfl_down_sync(kFull, tv[1], 1);
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int kk = k + q;
+        const R w = W[q];
+        const bool pos = w > R(0);
+        const R Tc = pos ? x[t][q + 1] : x[t][q];
+        const R aL = pos ? tv[q + 1] : tv[q];
+        const R aR = pos ? (kk == nln - 1 ? x[t][q + 1] : tv[q + 2]) : tv[q + 1];
+        R d;
+        if constexpr (UNI) d = div_fast(w * a.dt, pos ? h[q + 1] : h[q], pos ? yh[q + 1] : yh[q], bad);
+        else d = w * a.dt / (pos ? h[q + 1] : h[q]);
+        const R cx = pos ? fmin2(d, R(1)) : fmin2(-d, R(1));
+        const R f = ppm_face(w, Tc, aL, aR, cx, [&](R z) { return div6(z, bad); });
+        R v = f * A[q] * w - lov[t][q];
+        if (!pos && !(w < R(0))) v = R(0) - lov[t][q];
+        if (kk == 0) v = -(tv[1 + q] * w * A[q]) - lov[t][q];
+        hov[2 * t + q] = kk >= nln ? R(0) : v;
+      }
+    }
+  } else if constexpr (VER == VER_QR4C) {
+    // lib/oce_adv_tra_ver.F90:397-436, the reference's assignments in order
+    R zd[2], yz[2], za[2], zb[2];
+    const R *lt = m.ltab + k;
+    ldv2(lt + LT_ZD * S, zd); ldv2(lt + LT_YZD * S, yz); ldv2(lt + LT_ZA * S, za); ldv2(lt + LT_ZB * S, zb);
+#pragma unroll
+    for (int t = 0; t < G; t++) {
+      R g[4];
+#pragma unroll
+      for (int q = 0; q < 2; q++) g[1 + q] = div_fast(x[t][q] - x[t][q + 1], zd[q], yz[q], bad);
+      g[0] = __shfl_up_sync(kFull, g[2], 1);
+      g[3] = __shfl_down_sync(kFull, g[1], 1);
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int kk = k + q;
+        const R w = W[q], T0 = x[t][q], T1 = x[t][q + 1];
+        R v = lov[t][q];
+        const R mid = -(R(0.5) * (T0 + T1) * w * A[q]);
+        if (kk == 0) v = -(T1 * w * A[q]) - v;
+        if (kk == 1) v = mid - v;
+        if (kk == nln - 1) v = mid - v;
+        const R m1 = T1 + div3((R(2) * g[1 + q] + g[2 + q]) * za[q], bad);
+        const R m2 = T0 + div3((R(2) * g[1 + q] + g[q]) * zb[q], bad);
+        const R tm = (w + fabs(w)) * m1 + (w - fabs(w)) * m2;
+        const R f = (-(R(0.5) * (R(1) - a.pv) * tm) - a.pv * (R(0.5) * (m1 + m2)) * w) * A[q] - v;
+        if (kk >= 2 && kk <= nln - 2) v = f;
+        hov[2 * t + q] = kk >= nln ? R(0) : v;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int t = 0; t < G; t++)
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int kk = k + q;
+        const R T0 = x[t][q], T1 = x[t][q + 1];
+        R v;
+        if constexpr (VER == VER_CDIFF) {
+          const R c = R(0.5) * (T0 + T1);
+          v = (kk == 0 ? -(W[q] * T1 * A[q]) : -(c * W[q] * A[q])) - lov[t][q];
+        } else {
+          v = upw_v(T1, T0, W[q], A[q], kk, nln) - lov[t][q];
+        }
+        hov[2 * t + q] = kk >= nln ? R(0) : v;
+      }
+  }
+  const bool st = l.on && !l.halo;
+  if (st) {
+    st_pair_il<NT, G>(a.adf_v, t0, o, hov);
+    if (k + 2 == nln)  // the bottom interface of a column of whole pairs
+      for (int t = 0; t < G; t++) il<NT>(a.adf_v, t0 + t, o + 2) = R(0);
+  }
+  if constexpr (LIM == LIM_FCT) {
+    // LO solution (lib/oce_adv_tra_driver.F90:202-211)
+    R asv[2], yas[2], hn[2], yhn[2], h[2], out[2 * G];
+    const cix oh = (cix)n * m.hS + k;
+    ldv2(m.areasvol + o, asv);
+    ldv2(m.rcp + o, yas);
+    ldv2(m.hnT + oh, hn);
+    ldv2(m.yhnT + oh, yhn);
+    ldv2(m.hT + oh, h);
+    bool badl = false;
+#pragma unroll
+    for (int t = 0; t < G; t++) {
+      const R dn = __shfl_down_sync(kFull, lov[t][0], 1);
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const R f1 = q == 0 ? lov[t][1] : (k + 2 >= nln ? R(0) : dn);
+        acc[t][q] = (acc[t][q] + (lov[t][q] - f1)) * a.dt;
+        const R num = ts[t][1 + q] * h[q] + div_fast(acc[t][q], asv[q], yas[q], badl);
+        out[2 * t + q] = div_fast(num, hn[q], yhn[q], badl);
+      }
+    }
+    if (badl) {
+      for (int t = 0; t < G; t++)
+        for (int q = 0; q < 2; q++) out[2 * t + q] = (ts[t][1 + q] * h[q] + acc[t][q] / asv[q]) / hn[q];
+    }
+    if (st) st_pair_il<NT, G>(a.lo, t0, o, out);
+  }
+  if (bad && st) col1_vert_slow<R, TS, NT, G, VER, LIM>(m, a, t0, n, k);
+}
+
+// The column pairs of `per` consecutive warps of the schedule, one after the
+// other; the next pair's map entry is loaded ahead.
+template <typename R, typename F>
+__device__ __forceinline__ void col_warps(const DMeshT<R> &m, int blk, int per, F f) {
+  const DPairs &s = m.node_pairs;
+  int warp = (blk * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5)) * per;
+  const int end = min(warp + per, s.nwarps);
+  if (warp >= end) return;
+  PairLane nxt = pair_lane(s, warp);
+  do {
+    const PairLane c = nxt;
+    if (++warp < end) nxt = pair_lane(s, warp);
+    f(c);
+  } while (warp < end);
+}
+
+template <typename R, typename TS, int NT, int VER, int LIM, bool UNI>
+__device__ __forceinline__ void col1_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk, int per) {
+  constexpr int G = LaneTracers<R, NT>::col1;
+  col_warps(m, blk, per, [&](const PairLane &l) {
+#pragma unroll
+    for (int t0 = 0; t0 < NT; t0 += G) col1_pair<R, TS, NT, G, VER, LIM, UNI>(m, a, t0, l);
+  });
+}
+template <typename R, typename TS, int NT, int VER, int LIM, bool UNI>
+__global__ void __launch_bounds__(kColThreads, StepBlocks<R, NT>::col1)
+    k_col1(const __grid_constant__ DMeshT<R> m, const __grid_constant__ FusedArgs<R, TS> a, int per) {
+  col1_block<R, TS, NT, VER, LIM, UNI>(m, a, blockIdx.x, per);
 }
 
 // ---------------------------------------------------------------------------
 // k_col2: bounds, in/out sums, ratios (lib/oce_adv_tra_fct.F90:105-374)
 // ---------------------------------------------------------------------------
+// Quotients of the limiter ratios, straight-line.  FP64: the hardware's
+// approximate reciprocal (about 2^-20) refined by Newton steps y += y (1 - b y), the
+// last of which rounds 1 / b correctly unless b's significand is all ones, then
+// the quotient by Markstein's correction (see div_rcp).  Operands outside [2^-500,
+// 2^500] (other than a zero numerator) and that significand set `bad`, and the
+// caller divides again.
+__device__ __forceinline__ double rcp_newton(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+  return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+}
+__device__ __forceinline__ double div_any(double a, double b, bool &bad) {
+  double y = rcp_newton(b);
+  y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  const unsigned ua = 2u * (unsigned)__double2hiint(a), ub = 2u * (unsigned)__double2hiint(b);
+  bad |= ub - 0x41600000u > 0xbe600000u - 0x41600000u || (ua - 0x41600000u > 0xbe600000u - 0x41600000u && ua != 0u) ||
+         ((unsigned)__double2hiint(b) | 0xfff00000u) == 0xffffffffu;
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+// Reciprocal for FP64 quotients that are rounded to FP32 afterwards: one Newton
+// step (error about 2^-40).
+__device__ __forceinline__ double rcp_newton1(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+}
+
+// FCT bounds of one cell from the ring elements, for nodes whose ring list is
+// incomplete (lib/oce_adv_tra_fct.F90:105-181).
+template <typename R>
+struct Bounds {
+  R mx, mn;
+};
 template <typename R, typename TS, int NT>
-__device__ __forceinline__ void col2_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk, int *smem) {
-  int *s_off = smem, *s_item = smem + kMaxItemsPerBlock + 1;
-  R *s_mx = (R *)(smem + kMaxItemsPerBlock + 1 + kMaxCellsPerBlock + 1);
-  s_mx = (R *)(((uintptr_t)s_mx + 15) & ~(uintptr_t)15);
-  R *s_mn = s_mx + NT * kMaxCellsPerBlock;
-  const CellMap cm = map_cells(m.node_sched, blk, s_off, s_item);
-  const Incidence inc = stage_incidence<StageIncidence<R>::col2>(m, cm, s_mn + NT * kMaxCellsPerBlock);
-  const int S = m.S;
+__device__ __noinline__ Bounds<R> ring_bounds(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t, int n, int k) {
   const R big = R(1e3);
+  Bounds<R> b{R(0), R(0)};
+  const int p0 = m.ring_ptr[n], p1 = m.ring_ptr[n + 1];
+#pragma unroll 1
+  for (int p = p0; p < p1; p++) {
+    const int el = m.ring_elem[p];
+    R hi = -big, lw = big;
+    if (k < m.nlev_elem[el] - 1) {
+      const int *en = m.elem_nodes + 3 * (size_t)el;
+      R h[3], l[3];
+      for (int q = 0; q < 3; q++) {
+        const cix o = (cix)en[q] * m.S + k;
+        const R lv = il<NT>(a.lo, t, o), tv = ldT<R>(a.T[t], o, a.off[t]);
+        h[q] = fmax2(lv, tv);
+        l[q] = fmin2(lv, tv);
+      }
+      hi = fmax3(h[0], h[1], h[2]);
+      lw = fmin3(l[0], l[1], l[2]);
+    }
+    b.mx = p == p0 ? hi : fmax2(b.mx, hi);
+    b.mn = p == p0 ? lw : fmin2(b.mn, lw);
+  }
+  return b;
+}
 
-  for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
-    const int j = s_item[lc], n = cm.i0 + j, k = lc - (s_off[j] - cm.c0), nz = k + 1;
-    R tmx[NTMAX], tmn[NTMAX];
-    if (m.ring_full[n]) {
-      // With a complete ring, the nodes of the ring elements wet at this level
-      // are the node itself and the far ends of its edges wet at this level
-      // (each such edge has a wet triangle holding both ends); max and min
-      // are exact, so the bounds equal the per-element ones below.
-      const cix on = (cix)n * S + k;
-      R lv[NTMAX];
-      il_load<NT>(a.lo[0], on, lv);
-      for (int t = 0; t < NT; t++) {
-        const R l = lv[t], tt = ldT(a.T[t], on, a.off[t]);
-        tmx[t] = fmax2(l, tt);
-        tmn[t] = fmin2(l, tt);
-      }
-#pragma unroll 4
-    for (int p = inc.nep[j] - inc.sub, pe = inc.nep[j + 1] - inc.sub; p < pe; p++) {
-        const int4 q = inc.ne[p];
-        if (nz > q.z) continue;
-        const cix o = (cix)q.w + k;
-        il_load<NT>(a.lo[0], o, lv);
-        for (int t = 0; t < NT; t++) {
-          const R l = lv[t], tt = ldT(a.T[t], o, a.off[t]);
-          tmx[t] = fmax2(tmx[t], fmax2(l, tt));
-          tmn[t] = fmin2(tmn[t], fmin2(l, tt));
-        }
-      }
-      if (nz > m.nlev_node_min[n] - 1) {  // a ring element is dry here: +-big enter the bounds
-        for (int t = 0; t < NT; t++) {
-          tmx[t] = fmax2(tmx[t], -big);
-          tmn[t] = fmin2(tmn[t], big);
-        }
-      }
-      for (int t = 0; t < NT; t++) {
-        s_mx[t * kMaxCellsPerBlock + lc] = tmx[t];
-        s_mn[t * kMaxCellsPerBlock + lc] = tmn[t];
-      }
-      continue;
-    }
-    for (int p = m.ring_ptr[n]; p < m.ring_ptr[n + 1]; p++) {
-      const int el = m.ring_elem[p];
-      const bool wet = nz <= m.nlev_elem[el] - 1;
-      int e0 = 0, e1 = 0, e2 = 0;
-      if (wet) {
-        const int *en = m.elem_nodes + 3 * el;
-        e0 = en[0]; e1 = en[1]; e2 = en[2];
-      }
-      for (int t = 0; t < NT; t++) {
-        R amx, amn;
-        if (wet) {
-          const cix o0 = (cix)e0 * S + k, o1 = (cix)e1 * S + k, o2 = (cix)e2 * S + k;
-          const R l0 = il<NT>(a.lo, t, o0), l1 = il<NT>(a.lo, t, o1), l2 = il<NT>(a.lo, t, o2);
-          const R t0 = ldT(a.T[t], o0, a.off[t]), t1 = ldT(a.T[t], o1, a.off[t]), t2 = ldT(a.T[t], o2, a.off[t]);
-          amx = fmax3(fmax2(l0, t0), fmax2(l1, t1), fmax2(l2, t2));
-          amn = fmin3(fmin2(l0, t0), fmin2(l1, t1), fmin2(l2, t2));
-        } else {
-          amx = -big;
-          amn = big;
-        }
-        if (p == m.ring_ptr[n]) { tmx[t] = amx; tmn[t] = amn; }
-        else { tmx[t] = fmax2(tmx[t], amx); tmn[t] = fmin2(tmn[t], amn); }
-      }
-    }
-    for (int t = 0; t < NT; t++) {
-      s_mx[t * kMaxCellsPerBlock + lc] = tmx[t];
-      s_mn[t * kMaxCellsPerBlock + lc] = tmn[t];
+template <typename R, typename TS, int NT, int G>
+__device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, const PairLane &l) {
+  const int n = l.item, k = l.k, S = m.S;
+  const cix o = (cix)n * S + k;
+  const NodeRec rec = node_rec(m, n);
+  const int nln = rec.nlev() - 1;
+  const R big = R(1e3);
+  R lo[2 * G], av[2 * G], mx[2 * G], mn[2 * G], fp[2 * G], fm[2 * G];
+  ld_pair_il<NT, G>(a.lo, t0, o, lo);
+  ld_pair_il<NT, G>(a.adf_v, t0, o, av);
+#pragma unroll
+  for (int t = 0; t < G; t++) {
+    R tt[2];
+    ld_pair_T(a.T[t0 + t], o, a.off[t0 + t], tt);
+    // interface k + 2 (zero at the column's bottom)
+    const R a2 = k + 2 < nln ? il<NT>(a.adf_v, t0 + t, o + 2) : R(0);
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int i = 2 * t + q;
+      mx[i] = fmax2(lo[i], tt[q]);
+      mn[i] = fmin2(lo[i], tt[q]);
+      const R v0 = av[i], v1 = q == 0 ? av[i + 1] : a2;
+      fp[i] = R(0) + (fmax2(R(0), v0) + fmax2(R(0), -v1));
+      fm[i] = R(0) + (fmin2(R(0), v0) + fmin2(R(0), -v1));
     }
   }
-  __syncthreads();
-
-  const R eps = R((double)1e-16f);  // real(MP) :: flux_eps = 1e-16 (default-real literal)
-  for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
-    const int j = s_item[lc], n = cm.i0 + j, k = lc - (s_off[j] - cm.c0), nz = k + 1;
-    const cix col = (cix)n * S, o = col + k;
-    const int nl1 = m.nlev_node[n];
-    const bool edge_lev = (nz == 1 || nz == nl1 - 1);
-    R fp[NTMAX], fm[NTMAX];
-    {
-      R v0[NTMAX], v1[NTMAX];  // interfaces k and k + 1 of every tracer
-      il_load<NT>(a.adf_v[0], o, v0);
-      il_load<NT>(a.adf_v[0], o + 1, v1);
-      for (int t = 0; t < NT; t++) {
-        fp[t] = R(0) + (fmax2(R(0), v0[t]) + fmax2(R(0), -v1[t]));
-        fm[t] = R(0) + (fmin2(R(0), v0[t]) + fmin2(R(0), -v1[t]));
-      }
+  // in/out sums over the incident edges and, with a complete ring, the bounds:
+  // the nodes of the ring elements wet at a level are the node itself and the
+  // far ends of its edges wet there (each such edge has a wet triangle holding
+  // both ends); max and min are exact, so these equal the per-element ones
+  for_edges(m, n, k, rec, [&](cix oe, cix oo, bool second, int lev) {
+    const bool w0 = k < lev, w1 = k + 1 < lev;
+    R f[2 * G], l1[2 * G], t1[2 * G];
+    ld_pair_il_if<NT, G>(a.adf_h, t0, oe, w0, f);
+    ld_pair_il_if<NT, G>(a.lo, t0, oo, w0, l1);
+#pragma unroll
+    for (int t = 0; t < G; t++) ld_pair_T_if(a.T[t0 + t], oo, a.off[t0 + t], w0, t1 + 2 * t);
+#pragma unroll
+    for (int i = 0; i < 2 * G; i++) {
+      const bool w = i % 2 == 0 ? w0 : w1;
+      const R hi = fmax2(l1[i], t1[i]), lw = fmin2(l1[i], t1[i]);
+      mx[i] = (w && hi > mx[i]) ? hi : mx[i];
+      mn[i] = (w && lw < mn[i]) ? lw : mn[i];
+      const R g = second ? -f[i] : f[i];  // zero where the edge is dry
+      fp[i] = fp[i] + fmax2(R(0), g);
+      fm[i] = fm[i] + fmin2(R(0), g);
     }
-#pragma unroll 4
-    for (int p = inc.nep[j] - inc.sub, pe = inc.nep[j + 1] - inc.sub; p < pe; p++) {
-      const int4 q = inc.ne[p];
-      if (nz > q.z) continue;
-      R fv[NTMAX];
-      il_load<NT>(a.adf_h[0], (cix)(q.x >> 1) * S + k, fv);
-      for (int t = 0; t < NT; t++) {
-        const R f = fv[t];
-        if (q.x & 1) {
-          fp[t] = fp[t] + fmax2(R(0), -f);
-          fm[t] = fm[t] + fmin2(R(0), -f);
-        } else {
-          fp[t] = fp[t] + fmax2(R(0), f);
-          fm[t] = fm[t] + fmin2(R(0), f);
-        }
-      }
+  });
+  if (!rec.ring_full()) {
+#pragma unroll
+    for (int i = 0; i < 2 * G; i++) {
+      const Bounds<R> b = ring_bounds<R, TS, NT>(m, a, t0 + i / 2, n, k + i % 2);
+      mx[i] = b.mx;
+      mn[i] = b.mn;
     }
-    const R asv = m.areasvol[o];
-    const R yasv = m.rcp[o];  // 1/areasvol plane (k_rcp_planes)
-    for (int t = 0; t < NT; t++) {
-      const int b = t * kMaxCellsPerBlock + lc;
-      const R LO = il<NT>(a.lo, t, o);
-      R bmax, bmin;
-      if (edge_lev) {
-        bmax = s_mx[b] - LO;
-        bmin = s_mn[b] - LO;
-      } else {
-        bmax = fmax3(s_mx[b - 1], s_mx[b], s_mx[b + 1]) - LO;
-        bmin = fmin3(s_mn[b - 1], s_mn[b], s_mn[b + 1]) - LO;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 2 * G; i++)
+      if (k + i % 2 + 1 > rec.nlev_min() - 1) {  // a ring element is dry here: +-big enter the bounds
+        mx[i] = fmax2(mx[i], -big);
+        mn[i] = fmin2(mn[i], big);
       }
+  }
+  R asv[2], yas[2];
+  ldv2(m.areasvol + o, asv);
+  ldv2(m.rcp + o, yas);  // 1/areasvol plane (k_rcp_planes)
+  if (k + 1 >= nln) asv[1] = yas[1] = R(1);  // dry
+  double dtv[2];
+  if constexpr (sizeof(R) == 4) {
+    dtv[0] = (double)a.dt * rcp_newton1((double)asv[0]);
+    dtv[1] = (double)a.dt * rcp_newton1((double)asv[1]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < G; t++) {
+    // the layers above and below (lib/oce_adv_tra_fct.F90:183-229)
+    const R mxu = __shfl_up_sync(kFull, mx[2 * t + 1], 1), mxd = __shfl_down_sync(kFull, mx[2 * t], 1);
+    const R mnu = __shfl_up_sync(kFull, mn[2 * t + 1], 1), mnd = __shfl_down_sync(kFull, mn[2 * t], 1);
+    R bx[2], bn[2], out[4];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int i = 2 * t + q, kk = k + q;
+      const bool edge_lev = kk == 0 || kk == nln - 1;
+      const R ux = q == 0 ? fmax3(mxu, mx[2 * t], mx[2 * t + 1]) : fmax3(mx[2 * t], mx[2 * t + 1], mxd);
+      const R un = q == 0 ? fmin3(mnu, mn[2 * t], mn[2 * t + 1]) : fmin3(mn[2 * t], mn[2 * t + 1], mnd);
+      bx[q] = (edge_lev ? mx[i] : ux) - lo[i];
+      bn[q] = (edge_lev ? mn[i] : un) - lo[i];
+    }
+    // R+ = min(1, bmax / (P+ dt / V + eps)), R- likewise; flux_eps is a
+    // default-real literal.  In FP32 the denominators, where cancellation with it
+    // matters, and the quotients are formed in FP64.  A quotient of a positive
+    // denominator not above bmax is at least 1: where that holds for the warp (limiting
+    // is local) the FP32 kernels do not divide (FP64: the test costs more than it
+    // saves, 0.277 against 0.258 ms at 400x400x64).
+    const double eps = (double)1e-16f;
+    bool bad = false, need = false;
+    double up[2], um[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int i = 2 * t + q;
       if constexpr (sizeof(R) == 8) {
-        // two scalar stores into the pair: R+ leaves the registers before R- is formed
-        R flux = div_rcp(fp[t] * a.dt, asv, yasv) + eps;
-        a.rpm[t][2 * o] = fmin2(R(1), bmax / flux);
-        flux = div_rcp(fm[t] * a.dt, asv, yasv) - eps;
-        a.rpm[t][2 * o + 1] = fmin2(R(1), bmin / flux);
+        up[q] = div_fast(fp[i] * a.dt, asv[q], yas[q], bad) + eps;
+        um[q] = div_fast(fm[i] * a.dt, asv[q], yas[q], bad) - eps;
       } else {
-        // FP32 arithmetic: the ratio denominators, where cancellation with
-        // flux_eps matters, are formed and divided in FP64
-        const double e64 = (double)1e-16f, dt64 = (double)a.dt, asv64 = (double)asv;
-        double flux = (double)fp[t] * dt64 / asv64 + e64;
-        a.rpm[t][2 * o] = (R)fmin2(1.0, (double)bmax / flux);
-        flux = (double)fm[t] * dt64 / asv64 - e64;
-        a.rpm[t][2 * o + 1] = (R)fmin2(1.0, (double)bmin / flux);
+        up[q] = (double)fp[i] * dtv[q] + eps;
+        um[q] = (double)fm[i] * dtv[q] - eps;
+        bad |= !(fabs(up[q]) < 1e200) || !(fabs(um[q]) < 1e200);
+      }
+      out[2 * q] = out[2 * q + 1] = R(1);
+      need |= k + q < nln && (!(up[q] > 0.0 && (double)bx[q] >= up[q]) || !(um[q] < 0.0 && (double)bn[q] <= um[q]));
+    }
+    if (sizeof(R) == 8 || need) {
+      auto div = [&](double x, double y) {
+        if constexpr (sizeof(R) == 8) return div_any(x, y, bad);
+        else return x * rcp_newton1(y);
+      };
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        out[2 * q] = (R)fmin2(1.0, div((double)bx[q], up[q]));
+        out[2 * q + 1] = (R)fmin2(1.0, div((double)bn[q], um[q]));
+      }
+    }
+    if (k + 1 >= nln) out[2] = out[3] = R(0);  // dry: read by k_col3 against a zero flux
+    if (l.on && !l.halo) {
+      stv4(a.rpm[t0 + t] + 2 * (size_t)o, out);
+      if (bad) {
+        for (int q = 0; q < 2; q++) {
+          const int i = 2 * t + q;
+          double u, v;
+          if constexpr (sizeof(R) == 8) {
+            u = fp[i] * a.dt / asv[q];
+            v = fm[i] * a.dt / asv[q];
+          } else {
+            u = (double)fp[i] * (double)a.dt / (double)asv[q];
+            v = (double)fm[i] * (double)a.dt / (double)asv[q];
+          }
+          out[2 * q] = (R)fmin2(1.0, (double)bx[q] / (u + eps));
+          out[2 * q + 1] = (R)fmin2(1.0, (double)bn[q] / (v - eps));
+        }
+        if (k + 1 >= nln) out[2] = out[3] = R(0);
+        stv4(a.rpm[t0 + t] + 2 * (size_t)o, out);
       }
     }
   }
 }
 
 template <typename R, typename TS, int NT>
-__global__ void __launch_bounds__(kThreads, MinBlocks<R>::col2) k_col2(DMeshT<R> m, FusedArgs<R, TS> a) {
-  extern __shared__ int smem[];
-  col2_block<R, TS, NT>(m, a, blockIdx.x, smem);
+__device__ __forceinline__ void col2_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk, int per) {
+  constexpr int G = LaneTracers<R, NT>::col2;
+  col_warps(m, blk, per, [&](const PairLane &l) {
+#pragma unroll
+    for (int t0 = 0; t0 < NT; t0 += G) col2_pair<R, TS, NT, G>(m, a, t0, l);
+  });
 }
-
-// limited vertical flux at interface i (lib/oce_adv_tra_fct.F90:396-427);
-// av: the tracer's slot of the column's interleaved interface fluxes (stride
-// NT); rpm: the column's (R+, R-) pairs
-template <int NT, typename R>
-__device__ __forceinline__ R limit_v(const R *av, const R *rpm, int i, int nlev) {
-  const R f = av[(i - 1) * NT];
-  if (i == nlev) return f;
-  R ae = R(1);
-  if (i == 1) {
-    ae = (f >= R(0)) ? fmin2(ae, rpm[0]) : fmin2(ae, rpm[1]);
-  } else if (f >= R(0)) {
-    ae = fmin2(ae, rpm[2 * (i - 2) + 1]);
-    ae = fmin2(ae, rpm[2 * (i - 1)]);
-  } else {
-    ae = fmin2(ae, rpm[2 * (i - 2)]);
-    ae = fmin2(ae, rpm[2 * (i - 1) + 1]);
-  }
-  return ae * f;
+template <typename R, typename TS, int NT>
+__global__ void __launch_bounds__(kColThreads, StepBlocks<R, NT>::col2)
+    k_col2(const __grid_constant__ DMeshT<R> m, const __grid_constant__ FusedArgs<R, TS> a, int per) {
+  col2_block<R, TS, NT>(m, a, blockIdx.x, per);
 }
 
 // ---------------------------------------------------------------------------
@@ -858,9 +1217,7 @@ __device__ __forceinline__ R limit_v(const R *av, const R *rpm, int i, int nlev)
 // ---------------------------------------------------------------------------
 // Reciprocals of the static cell geometry, 1/areasvol and 1/hnode_new, for
 // the Markstein divisions of k_col1's LO solution, k_col2's ratio
-// denominators and k_col3's update (computed per step they cost an IEEE
-// division each; measured in k_col3: loading them is 2-3 % faster, while
-// the same for k_col1's ten PPM weights was slower).
+// denominators and k_col3's update.
 template <typename R>
 __global__ void k_rcp_planes(DMeshT<R> m, R *rcp) {
   const size_t plane = (size_t)m.S * m.N;
@@ -872,93 +1229,148 @@ __global__ void k_rcp_planes(DMeshT<R> m, R *rcp) {
   }
 }
 
-template <typename R, typename TS, int NT, int LIM>
-__device__ __forceinline__ void col3_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk, int *smem) {
-  int *s_off = smem, *s_item = smem + kMaxItemsPerBlock + 1;
-  const CellMap cm = map_cells(m.node_sched, blk, s_off, s_item);
-  const Incidence inc = stage_incidence<StageIncidence<R>::col3>(m, cm, smem + kMaxItemsPerBlock + 1 + kMaxCellsPerBlock + 1);
+// limited vertical flux (lib/oce_adv_tra_fct.F90:396-427): ra = (R+, R-) of
+// the layer above the interface, rh of the layer below it
+template <typename R>
+__device__ __forceinline__ R limit_v(R f, const R *ra, const R *rh, bool top) {
+  const R p = top ? rh[0] : fmin2(ra[1], rh[0]);
+  const R q = top ? rh[1] : fmin2(ra[0], rh[1]);
+  return (f >= R(0) ? p : q) * f;
+}
+
+template <typename R, typename TS, int NT>
+__device__ __forceinline__ void col3_store(const FusedArgs<R, TS> &a, int t, cix o, int wet, const R *v) {
+  TS s[2];
+#pragma unroll
+  for (int q = 0; q < 2; q++)
+    s[q] = stT<R, TS>(v[q], a.off[t], a.sround != 0, a.sround ? mix32(a.seed[t] ^ mix32((uint32_t)(o + q))) : 0u);
+  if constexpr (std::is_same<R, TS>::value) {
+    if (wet == 2) stv2(a.T_out[t] + o, v);
+    else a.T_out[t][o] = s[0];
+  } else {
+    a.T_out[t][o] = s[0];
+    if (wet == 2) a.T_out[t][o + 1] = s[1];
+  }
+  if (a.nonfinite) {
+    const int c = !isfinite(v[0]) + (wet == 2 && !isfinite(v[1]));
+    if (c) atomicAdd(a.nonfinite, (unsigned long long)c);
+  }
+}
+
+// A pair's update with the divisions `div` (the fast ones, or plain ones again
+// for the lanes whose operands lie outside their range).
+template <typename R, typename TS, int NT, int G, int LIM, typename D>
+__device__ __forceinline__ void col3_update(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, int n, int k, const NodeRec &rec,
+                                            D div, R (*out)[2]) {
   const int S = m.S;
-  for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
-    const int j = s_item[lc], n = cm.i0 + j, k = lc - (s_off[j] - cm.c0), nz = k + 1;
-    const cix col = (cix)n * S, o = col + k;
-    const int nlev = m.nlev_node[n];
-    const R asv = m.areasvol[o], hn = m.hnode_new[o];
-    const R yasv = m.rcp[o], yhn = m.rcp[m.rcp_plane + o];
-    R dv[NTMAX], dh[NTMAX];
-    for (int t = 0; t < NT; t++) {
-      const R *av = a.adf_v[t] + (size_t)col * NT;
-      dv[t] = R(0);
-      if (LIM == LIM_FCT) {
-        dv[t] = dv[t] - ldT(a.T[t], o, a.off[t]) * m.hnode[o] + il<NT>(a.lo, t, o) * hn;
-        const R fk = limit_v<NT>(av, a.rpm[t] + 2 * col, nz, nlev);
-        const R fk1 = limit_v<NT>(av, a.rpm[t] + 2 * col, nz + 1, nlev);
-        dv[t] = dv[t] + div_rcp((fk - fk1) * a.dt, asv, yasv);
-      } else {
-        dv[t] = dv[t] + div_rcp((av[k * NT] - av[(k + 1) * NT]) * a.dt, asv, yasv);
-      }
-      dh[t] = R(0);
-    }
-    R rps[NTMAX], rms[NTMAX];
+  const cix o = (cix)n * S + k, oh = (cix)n * m.hS + k;
+  const int nln = rec.nlev() - 1;
+  R asv[2], yas[2], hn[2], yhn[2], h[2], av[2 * G], lo[2 * G], dh[G][2], rs[G][4];
+  ldv2(m.areasvol + o, asv);
+  ldv2(m.rcp + o, yas);
+  ldv2(m.hnT + oh, hn);
+  ldv2(m.yhnT + oh, yhn);
+  ld_pair_il<NT, G>(a.adf_v, t0, o, av);
+  if (LIM == LIM_FCT) {
+    ldv2(m.hT + oh, h);
+    ld_pair_il<NT, G>(a.lo, t0, o, lo);
+#pragma unroll
+    for (int t = 0; t < G; t++) ldv4(a.rpm[t0 + t] + 2 * (size_t)o, rs[t]);
+  }
+#pragma unroll
+  for (int t = 0; t < G; t++) dh[t][0] = dh[t][1] = R(0);
+  for_edges(m, n, k, rec, [&](cix oe, cix oo, bool second, int lev) {
+    const bool w0 = k < lev;
+    R f[2 * G], ro[G][4];
+    ld_pair_il_if<NT, G>(a.adf_h, t0, oe, w0, f);
     if (LIM == LIM_FCT)
-      for (int t = 0; t < NT; t++) {
-        ld_pair(a.rpm[t] + 2 * o, rps[t], rms[t]);
-      }
-#pragma unroll 4
-    for (int p = inc.nep[j] - inc.sub, pe = inc.nep[j + 1] - inc.sub; p < pe; p++) {
-      const int4 q = inc.ne[p];
-      if (nz > q.z) continue;
-      const bool second = q.x & 1;
-      const cix oo = (cix)q.w + k;  // the edge's other node (column base in .w)
-      R fv[NTMAX];
-      il_load<NT>(a.adf_h[0], (cix)(q.x >> 1) * S + k, fv);
-      for (int t = 0; t < NT; t++) {
-        R f = fv[t];
+#pragma unroll
+      for (int t = 0; t < G; t++) ldv4_if(a.rpm[t0 + t] + 2 * (size_t)oo, w0, ro[t]);
+#pragma unroll
+    for (int t = 0; t < G; t++)
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        // flux into this node (zero where the edge is dry): positive ones are
+        // limited by its R+ and the other node's R-, negative ones by the converse
+        R g = second ? -f[2 * t + q] : f[2 * t + q];
         if (LIM == LIM_FCT) {
-          // r+/- at the edge's first (o1) and second (o2) node
-          R rpo, rmo;
-          ld_pair(a.rpm[t] + 2 * oo, rpo, rmo);
-          const R rp1 = second ? rpo : rps[t], rm1 = second ? rmo : rms[t];
-          const R rp2 = second ? rps[t] : rpo, rm2 = second ? rms[t] : rmo;
-          R ae = R(1);
-          if (f >= R(0)) {
-            ae = fmin2(ae, rp1);
-            ae = fmin2(ae, rm2);
-          } else {
-            ae = fmin2(ae, rm1);
-            ae = fmin2(ae, rp2);
-          }
-          f = ae * f;
+          const R p = fmin2(rs[t][2 * q], ro[t][2 * q + 1]), r = fmin2(rs[t][2 * q + 1], ro[t][2 * q]);
+          g = (g >= R(0) ? p : r) * g;
         }
-        const R term = div_rcp(f * a.dt, asv, yasv);
-        dh[t] = second ? dh[t] - term : dh[t] + term;
+        dh[t][q] = dh[t][q] + div(g * a.dt, asv[q], yas[q]);
       }
+  });
+#pragma unroll
+  for (int t = 0; t < G; t++) {
+    R tt[2];
+    ld_pair_T(a.T[t0 + t], o, a.off[t0 + t], tt);
+    if (k + 1 >= nln) tt[1] = R(0);  // dry, whatever the cell holds
+    R fv[3];
+    const R a2 = k + 2 < nln ? il<NT>(a.adf_v, t0 + t, o + 2) : R(0);
+    if (LIM == LIM_FCT) {
+      R ru[2] = {R(1), R(1)}, rd[2] = {R(1), R(1)};
+      if (k > 0) ld_pair(a.rpm[t0 + t] + 2 * (size_t)(o - 1), ru[0], ru[1]);
+      if (k + 2 < nln) ld_pair(a.rpm[t0 + t] + 2 * (size_t)(o + 2), rd[0], rd[1]);
+      fv[0] = limit_v(av[2 * t], ru, rs[t], k == 0);
+      fv[1] = limit_v(av[2 * t + 1], rs[t], rs[t] + 2, false);
+      fv[2] = limit_v(a2, rs[t] + 2, rd, false);
+    } else {
+      fv[0] = av[2 * t];
+      fv[1] = av[2 * t + 1];
+      fv[2] = a2;
     }
-    for (int t = 0; t < NT; t++) {
-      const R del = R(0) + dh[t] + dv[t];
-      const R tnew = ldT(a.T[t], o, a.off[t]) + div_rcp(del, hn, yhn);
-      a.T_out[t][o] = stT<R, TS>(tnew, a.off[t], a.sround != 0, a.sround ? mix32(a.seed[t] ^ mix32((uint32_t)o)) : 0u);
-      if (a.nonfinite && !isfinite(tnew)) atomicAdd(a.nonfinite, 1ull);
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      R dv = R(0);
+      if (LIM == LIM_FCT) dv = dv - tt[q] * h[q] + lo[2 * t + q] * hn[q];
+      dv = dv + div((fv[q] - fv[q + 1]) * a.dt, asv[q], yas[q]);
+      const R del = R(0) + dh[t][q] + dv;
+      out[t][q] = tt[q] + div(del, hn[q], yhn[q]);
     }
   }
 }
 
-template <typename R, typename TS, int NT, int LIM>
-__global__ void __launch_bounds__(kThreads, MinBlocks<R>::col3) k_col3(DMeshT<R> m, FusedArgs<R, TS> a) {
-  extern __shared__ int smem[];
-  col3_block<R, TS, NT, LIM>(m, a, blockIdx.x, smem);
+template <typename R, typename TS, int NT, int G, int LIM>
+__device__ __noinline__ void col3_pair_slow(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, int n, int k) {
+  const NodeRec rec = node_rec(m, n);
+  R out[G][2];
+  col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [](R x, R y, R) { return x / y; }, out);
+  for (int t = 0; t < G; t++) col3_store<R, TS, NT>(a, t0 + t, (cix)n * m.S + k, min(rec.nlev() - 1 - k, 2), out[t]);
 }
 
-// dynamic shared memory of each kernel
+template <typename R, typename TS, int NT, int G, int LIM>
+__device__ __forceinline__ void col3_pair(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, const PairLane &l) {
+  if (!l.on || l.halo) return;
+  const int n = l.item, k = l.k;
+  const NodeRec rec = node_rec(m, n);
+  const int wet = min(rec.nlev() - 1 - k, 2);
+  bool bad = false;
+  R out[G][2];
+  col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [&](R x, R y, R z) { return div_fast(x, y, z, bad); }, out);
+  if (bad) {
+    col3_pair_slow<R, TS, NT, G, LIM>(m, a, t0, n, k);
+    return;
+  }
+#pragma unroll
+  for (int t = 0; t < G; t++) col3_store<R, TS, NT>(a, t0 + t, (cix)n * m.S + k, wet, out[t]);
+}
+
+template <typename R, typename TS, int NT, int LIM>
+__device__ __forceinline__ void col3_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk, int per) {
+  constexpr int G = LaneTracers<R, NT>::col3;
+  col_warps(m, blk, per, [&](const PairLane &l) {
+#pragma unroll
+    for (int t0 = 0; t0 < NT; t0 += G) col3_pair<R, TS, NT, G, LIM>(m, a, t0, l);
+  });
+}
+template <typename R, typename TS, int NT, int LIM>
+__global__ void __launch_bounds__(kColThreads, StepBlocks<R, NT>::col3)
+    k_col3(const __grid_constant__ DMeshT<R> m, const __grid_constant__ FusedArgs<R, TS> a, int per) {
+  col3_block<R, TS, NT, LIM>(m, a, blockIdx.x, per);
+}
+
+// dynamic shared memory of the cell-map kernels (k_grad, the learned flux)
 constexpr size_t smem_edge() { return sizeof(int) * (kMaxItemsPerBlock + 1 + kMaxCellsPerBlock + 1); }
-template <typename R>
-constexpr size_t smem_col(int nt, int arrays) {
-  return sizeof(int) * (kMaxItemsPerBlock + 1 + kMaxCellsPerBlock + 1) + 16 + sizeof(R) * (size_t)arrays * nt * kMaxCellsPerBlock;
-}
-// k_col2 / k_col3: their arrays plus the staged incidence records
-template <typename R>
-constexpr size_t smem_col_staged(int nt, int arrays) {
-  return smem_col<R>(nt, arrays) + smem_stage();
-}
 
 FESOM_VARIANT_END
 }  // namespace fesom

@@ -53,11 +53,19 @@ using cix = unsigned;
 // constant near the field's mean, so that the storage ulp follows the
 // anomaly's magnitude.  Arithmetic is always in R.
 // ---------------------------------------------------------------------------
+// f64u: FP64 storage in caller-owned buffers that are only 8-byte aligned (no
+// vector accesses).
+struct f64u {
+  double v;
+};
 template <typename R, typename TS, typename I>
 __device__ __forceinline__ R ldT(const TS *p, I i, R off) {
   if constexpr (std::is_same<R, TS>::value) {
     (void)off;
     return p[i];
+  } else if constexpr (std::is_same<TS, f64u>::value) {
+    (void)off;
+    return p[i].v;
   } else {
     return R(p[i]) + off;
   }
@@ -105,6 +113,9 @@ __device__ __forceinline__ TS stT(R v, R off, bool sround, uint32_t r) {
   if constexpr (std::is_same<R, TS>::value) {
     (void)off; (void)sround; (void)r;
     return v;
+  } else if constexpr (std::is_same<TS, f64u>::value) {
+    (void)off; (void)sround; (void)r;
+    return TS{v};
   } else if constexpr (std::is_same<TS, __nv_bfloat16>::value) {
     const float x = float(v - off);
     return sround ? bf16_sround(x, r) : __float2bfloat16_rn(x);
@@ -114,7 +125,8 @@ __device__ __forceinline__ TS stT(R v, R off, bool sround, uint32_t r) {
   }
 }
 
-enum HorScheme { HOR_UPW1 = 0, HOR_MUSCL = 1, HOR_MFCT = 2 };
+// HOR_MUSCL_FEAT: MUSCL edge kernels that also write the learned flux's features
+enum HorScheme { HOR_UPW1 = 0, HOR_MUSCL = 1, HOR_MFCT = 2, HOR_MUSCL_FEAT = 3 };
 enum VerScheme { VER_UPW1 = 0, VER_PPM = 1, VER_QR4C = 2, VER_CDIFF = 3 };
 enum Limiter { LIM_NONE = 0, LIM_FCT = 1 };
 

@@ -63,7 +63,7 @@ enum { PH_GRAD = 0, PH_EDGE, PH_COL1, PH_COL2, PH_COL3, PH_COUNT };
 
 constexpr size_t kTaskSmem = (sizeof(BatchTask) + 15) / 16 * 16;
 size_t batch_smem() {
-  return kTaskSmem + std::max(smem_col_staged<float>(kNT, 2), smem_col_staged<float>(kNT, 0));
+  return kTaskSmem + smem_edge();
 }
 
 // prefix: PH_COUNT rows of (ntasks + 1) running totals of each task's blocks;
@@ -98,10 +98,10 @@ __global__ void __launch_bounds__(256, MINB)
         const int vblk = g - pre[task];
         switch (ph) {
           case PH_GRAD: grad_block<float, float, kNT>(st.m, st.a, vblk, work); break;
-          case PH_EDGE: edge_block<float, float, kNT, HOR, LIM>(st.m, st.a, vblk, work); break;
-          case PH_COL1: col1_block<float, float, kNT, VER, LIM>(st.m, st.a, vblk, work); break;
-          case PH_COL2: col2_block<float, float, kNT>(st.m, st.a, vblk, work); break;
-          default: col3_block<float, float, kNT, LIM>(st.m, st.a, vblk, work); break;
+          case PH_EDGE: edge_block<float, float, kNT, HOR, LIM, true>(st.m, st.a, vblk, kEdgeRun); break;
+          case PH_COL1: col1_block<float, float, kNT, VER, LIM, true>(st.m, st.a, vblk, kColRun); break;
+          case PH_COL2: col2_block<float, float, kNT>(st.m, st.a, vblk, kColRun); break;
+          default: col3_block<float, float, kNT, LIM>(st.m, st.a, vblk, kColRun); break;
         }
       }
       if (!grid_sync(bar, nb, spin_limit)) return;
@@ -163,19 +163,19 @@ static_assert(sizeof(PhasePack) <= 32000, "phase pack must fit the kernel parame
 // (Copying the descriptor into shared memory instead was slower still:
 // 491-525 ms, the pointers then occupy registers.)
 #ifndef FESOM_PHASE_MINB_GRAD
-#define FESOM_PHASE_MINB_GRAD FESOM_MINB32_GRAD
+#define FESOM_PHASE_MINB_GRAD 5
 #endif
 #ifndef FESOM_PHASE_MINB_EDGE
-#define FESOM_PHASE_MINB_EDGE 5
+#define FESOM_PHASE_MINB_EDGE 2
 #endif
 #ifndef FESOM_PHASE_MINB_COL1
-#define FESOM_PHASE_MINB_COL1 6
+#define FESOM_PHASE_MINB_COL1 2
 #endif
 #ifndef FESOM_PHASE_MINB_COL2
-#define FESOM_PHASE_MINB_COL2 6
+#define FESOM_PHASE_MINB_COL2 2
 #endif
 #ifndef FESOM_PHASE_MINB_COL3
-#define FESOM_PHASE_MINB_COL3 6
+#define FESOM_PHASE_MINB_COL3 2
 #endif
 template <int PH>
 struct PhaseBudget {
@@ -197,23 +197,15 @@ __global__ void __launch_bounds__(kThreads, PhaseBudget<PH>::v) k_batch_phase(co
     const int vblk = g - p.prefix[task];
     const BatchTask &st = p.t[task];
     if (PH == PH_GRAD) grad_block<float, float, kNT>(st.m, st.a, vblk, smem);
-    else if (PH == PH_EDGE) edge_block<float, float, kNT, HOR, LIM>(st.m, st.a, vblk, smem);
-    else if (PH == PH_COL1) col1_block<float, float, kNT, VER, LIM>(st.m, st.a, vblk, smem);
-    else if (PH == PH_COL2) col2_block<float, float, kNT>(st.m, st.a, vblk, smem);
-    else col3_block<float, float, kNT, LIM>(st.m, st.a, vblk, smem);
+    else if (PH == PH_EDGE) edge_block<float, float, kNT, HOR, LIM, true>(st.m, st.a, vblk, kEdgeRun);
+    else if (PH == PH_COL1) col1_block<float, float, kNT, VER, LIM, true>(st.m, st.a, vblk, kColRun);
+    else if (PH == PH_COL2) col2_block<float, float, kNT>(st.m, st.a, vblk, kColRun);
+    else col3_block<float, float, kNT, LIM>(st.m, st.a, vblk, kColRun);
   }
 }
 
-// dynamic shared memory of each phase: that of its standalone kernel
-size_t phase_smem(int ph) {
-  switch (ph) {
-    case PH_GRAD:
-    case PH_EDGE: return smem_edge();
-    case PH_COL1: return StageIncidence<float>::col1 ? smem_col_staged<float>(kNT, 2) : smem_col<float>(kNT, 2);
-    case PH_COL2: return StageIncidence<float>::col2 ? smem_col_staged<float>(kNT, 2) : smem_col<float>(kNT, 2);
-    default: return StageIncidence<float>::col3 ? smem_col_staged<float>(kNT, 0) : smem_col<float>(kNT, 0);
-  }
-}
+// dynamic shared memory of each phase
+size_t phase_smem(int ph) { return ph == PH_GRAD ? smem_edge() : 0; }
 
 struct PhaseKernel {
   const void *fn = nullptr;
@@ -302,13 +294,14 @@ struct BatchImpl {
   bool learned = false;
   // work-array slots, host task table (wave-major) and blocks per phase
   struct Slot {
-    void *adfh[kNT], *adfv[kNT], *lo[kNT], *rpm[kNT], *gradn[kNT];
+    void *adfh, *adfv, *lo, *rpm[kNT], *gradn[kNT];
   };
   std::vector<std::vector<Slot>> slots;
   std::vector<BatchTask> tasks;
   std::vector<int> task_slot;  // work-array slot of each task
   std::vector<int> wave_first;
-  std::vector<std::vector<int>> nblk;
+  std::vector<std::vector<int>> nblk;     // of tile.threads threads (path 0)
+  std::vector<std::vector<int>> nblk_ph;  // of kThreads threads (path 1)
   PhaseKernel phk[PH_COUNT];
   int phgrid[PH_COUNT] = {0, 0, 0, 0, 0};
   // phase launches of two steps captured as a graph; valid while the first
@@ -397,12 +390,22 @@ void refresh_vflux(BatchImpl &B) {
 
 // The task table (wave-major) from the members' current tracer buffers and
 // the batch's work-array slots.
+int phase_blocks(const BatchImpl &B, const DMeshT<float> &m, int ph, int threads) {
+  switch (ph) {
+    case PH_GRAD: return B.sch.hor == HOR_UPW1 ? 0 : m.grad_sched.nblk;
+    case PH_EDGE: return pair_blocks(m.edge_pairs, threads, kEdgeRun);
+    case PH_COL2: return B.sch.lim == LIM_FCT ? pair_blocks(m.node_pairs, threads, kColRun) : 0;
+    default: return pair_blocks(m.node_pairs, threads, kColRun);
+  }
+}
+
 void make_tasks(BatchImpl &B) {
   const int M = (int)B.members.size(), W = B.tile.wave;
   B.tasks.clear();
   B.task_slot.clear();
   B.wave_first.clear();
   B.nblk.assign(PH_COUNT, std::vector<int>());
+  B.nblk_ph.assign(PH_COUNT, std::vector<int>());
   for (int w = 0; w < B.nwaves; w++) {
     B.wave_first.push_back((int)B.tasks.size());
     for (int m = 0; m < M; m++) {
@@ -417,12 +420,12 @@ void make_tasks(BatchImpl &B) {
           a.T[t] = (const float *)tr.T;
           a.TAB[t] = (const float *)(B.refresh_ab ? tr.T : tr.TAB);
           a.T_out[t] = (float *)tr.Tout;
-          a.adf_h[t] = (float *)sl.adfh[t];
-          a.adf_v[t] = (float *)sl.adfv[t];
-          a.lo[t] = (float *)sl.lo[t];
           a.rpm[t] = (float *)sl.rpm[t];
           a.gradn[t] = (float *)sl.gradn[t];
         }
+        a.adf_h = (float *)sl.adfh;
+        a.adf_v = (float *)sl.adfv;
+        a.lo = (float *)sl.lo;
         a.vflux = (float *)P.vflux;
         a.vflux_mode = 2;
         a.vel = (const float *)P.vel;
@@ -432,11 +435,10 @@ void make_tasks(BatchImpl &B) {
         a.pv = (float)B.sch.pv;
         B.tasks.push_back(T);
         B.task_slot.push_back(b % W);
-        B.nblk[PH_GRAD].push_back(B.sch.hor == HOR_UPW1 ? 0 : P.dm32.grad_sched.nblk);
-        B.nblk[PH_EDGE].push_back(P.dm32.edge_sched.nblk);
-        B.nblk[PH_COL1].push_back(P.dm32.node_sched.nblk);
-        B.nblk[PH_COL2].push_back(B.sch.lim == LIM_FCT ? P.dm32.node_sched.nblk : 0);
-        B.nblk[PH_COL3].push_back(P.dm32.node_sched.nblk);
+        for (int ph = 0; ph < PH_COUNT; ph++) {
+          B.nblk[ph].push_back(phase_blocks(B, P.dm32, ph, B.tile.threads));
+          B.nblk_ph[ph].push_back(phase_blocks(B, P.dm32, ph, kThreads));
+        }
       }
     }
   }
@@ -548,12 +550,10 @@ void Batch::set_tile(const BatchTile &tile) {
     const int used = std::min(W, B.ntr[m] / kNT);
     for (int j = 0; j < used; j++) {
       BatchImpl::Slot &sl = B.slots[m][j];
-      // adf_h, lo and adf_v interleaved by tracer (stride kNT)
-      char *ah = (char *)B.walloc(kNT * es), *lo = (char *)B.walloc(kNT * ns), *av = (char *)B.walloc(kNT * ns);
+      sl.adfh = B.walloc(kNT * es);
+      sl.lo = B.walloc(kNT * ns);
+      sl.adfv = B.walloc(kNT * ns);
       for (int t = 0; t < kNT; t++) {
-        sl.adfh[t] = ah + t * sizeof(float);
-        sl.adfv[t] = av + t * sizeof(float);
-        sl.lo[t] = lo + t * sizeof(float);
         sl.rpm[t] = B.walloc(2 * ns);
         sl.gradn[t] = B.walloc(2 * ns);
       }
@@ -676,7 +676,7 @@ void phase_step(BatchImpl &B) {
           p.prefix[0] = 0;
           for (size_t i = c0; i < std::min(sel.size(), c0 + kPackTasks); i++) {
             p.t[p.ntasks] = B.tasks[sel[i]];
-            p.prefix[p.ntasks + 1] = p.prefix[p.ntasks] + B.nblk[ph][sel[i]];
+            p.prefix[p.ntasks + 1] = p.prefix[p.ntasks] + B.nblk_ph[ph][sel[i]];
             p.ntasks++;
           }
           const int total = p.prefix[p.ntasks];

@@ -29,6 +29,35 @@ struct DSched {
   int max_items;        // largest item count in one block
 };
 
+// Schedule of level pairs over items (nodes or edges): lane i of warp w takes
+// the pair of item[32 w + i] whose first level is lev & kPairLevel, or none where
+// lev is kPairNone.  Items follow one another along a space-filling curve, so
+// that a block's pairs share their neighbours' columns in L1.  Edge pairs whose
+// levels all have both an up and a down triangle and those that have not
+// (kPairRing) are kept in warps apart, so that no warp mixes the two forms of
+// the MUSCL gradient.  kPairHalo: computed, stored by another warp.
+struct DPairs {
+  const int *item;
+  const unsigned short *lev;
+  int nwarps;
+};
+// blocks of `threads` threads that hold the schedule's warps, `per` to a warp
+inline int pair_blocks(const DPairs &s, int threads, int per) {
+  const int n = threads / 32 * per;
+  return (s.nwarps + n - 1) / n;
+}
+// Warps of a schedule that a warp takes one after the other, its loads running
+// ahead from one to the next: at most `most`, fewer where the device would not
+// fill (148 SMs x 16 warps).  Measured at 1000x1000x64: edges 1 / 2 / 4 / 8: FP64
+// 2.28 / 1.94 / 1.83 / 1.83 ms; columns (k_col1 + k_col2 + k_col3) 4.77 / 4.28 /
+// 4.62 / 4.87 ms.
+constexpr int kEdgeRun = 4, kColRun = 2;
+inline int pair_run(const DPairs &s, int most) {
+  const int n = s.nwarps / (148 * 16);
+  return n < 1 ? 1 : (n > most ? most : n);
+}
+constexpr unsigned kPairNone = 0xffffu, kPairHalo = 0x8000u, kPairRing = 0x4000u, kPairLevel = 0x3fffu;
+
 template <typename R>
 struct DMeshT {
   int N, T, E, nl, S;
@@ -49,7 +78,6 @@ struct DMeshT {
   const R *elem_area;       // (T)
   const int *ring_ptr;      // (N+1)
   const int *ring_elem;
-  const unsigned char *ring_full;  // (N) 1: the ring holds every element of the node
   const int *ne_ptr;        // (N+1)
   const int4 *ne4;          // per incidence, in ascending edge id:
                             // (slot << 1 | node is the edge's 2nd node, other node, edge levels,
@@ -66,6 +94,30 @@ struct DMeshT {
   // cells, S x N each, computed once per mesh (k_rcp_planes)
   const R *rcp;
   size_t rcp_plane;         // S * N
+  // Per-edge record of k_edge (slot order), read as vectors.  edge_idx: three
+  // int4, {n1 S, n2 S, u0 S, u1 S}, {u2 S, d0 S, d1 S, d2 S} (column bases of the
+  // edge's nodes and of its up and down triangles' nodes) and {levels with both
+  // triangles wet, levels where c_lo is 1 at n1, at n2, edge levels}.
+  // edge_geo: 16 reals, the up and down triangles' gradient_sca, edge_dxdy(1)
+  // * edge_a, edge_dxdy(2) * r_earth and two unused.
+  const int4 *edge_idx;
+  const R *edge_geo;
+  DPairs edge_pairs;        // items = edges
+  // Node records of the column kernels: nrec {nlevels | incident edges << 16,
+  // nlevels_nod2D_min | complete ring << 31, levels of the first three incident
+  // edges and of the next three in 10 bits each}; ne6: {slot x S, other node x
+  // S | node is the edge's second << 31} of the first six incident edges in
+  // ascending edge id (fewer: entries without levels).
+  const int4 *nrec;
+  const int4 *ne6;          // three int4 per node
+  DPairs node_pairs;        // items = nodes; whole columns, or overlapping pieces of
+                            // those deeper than a warp
+  // thicknesses and 1/hnode_new of cell (n, k) at [n hS + k]: the full arrays,
+  // or one column (hS = 0) where every node has the same at each wet level
+  const R *hT, *hnT, *yhnT;
+  int hS;
+  int uniform_h;            // the latter holds; ltab has the PPM weights
+  const R *ltab;            // level tables (advect_fused.cuh)
   DSched node_sched;        // items = nodes, levels = nlev_node - 1
   DSched edge_sched;        // items = edges, levels = edge levels
   // node-levels whose MUSCL gradient is the ring mean for some incident edge

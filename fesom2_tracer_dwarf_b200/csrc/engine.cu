@@ -119,6 +119,181 @@ void build_schedules(EngineImpl &P, DMeshT<R> &d, int cells_per_block) {
   d.grad_sched.nblk = (int)blk.size() - 1;
 }
 
+// Levels of an edge whose up and down triangles are both there and wet.
+int edge_tri_levels(const MeshHost &M, int e) {
+  if (M.up_dn_tri[2 * e] < 0 || M.up_dn_tri[2 * e + 1] < 0) return 0;
+  return std::max(0, std::min(M.nlev_node_min[M.edge_nodes[2 * e]], M.nlev_node_min[M.edge_nodes[2 * e + 1]]) - 1);
+}
+
+DPairs upload_pairs(EngineImpl &P, const std::vector<int> &item, const std::vector<unsigned short> &lev) {
+  DPairs d;
+  d.item = P.upload(item);
+  d.lev = P.upload(lev);
+  d.nwarps = (int)(item.size() / 32);
+  return d;
+}
+
+// Pair schedule of the edges, run by run of slots: the pairs with both triangles
+// at every wet level, then the others.
+DPairs build_edge_pairs(EngineImpl &P) {
+  const MeshHost &M = P.mesh;
+  const int E = M.edge2D, run = 2048;
+  std::vector<int> item;
+  std::vector<unsigned short> lev;
+  size_t pairs = 0;
+  for (int e = 0; e < E; e++) pairs += (M.edge_levels(e) + 1) / 2;
+  item.reserve(pairs + 128 * ((size_t)E / run + 1));
+  lev.reserve(item.capacity());
+  for (int s0 = 0; s0 < E; s0 += run)
+    for (unsigned ring = 0; ring <= kPairRing; ring += kPairRing) {
+      for (int s = s0; s < std::min(E, s0 + run); s++) {
+        const int e = P.slot_edge[s], nl = M.edge_levels(e), tri = edge_tri_levels(M, e);
+        for (int k = 0; k < nl; k += 2) {
+          if ((std::min(k + 2, nl) > tri) != (ring != 0)) continue;
+          item.push_back(s);
+          lev.push_back((unsigned short)(ring | k));
+        }
+      }
+      while (item.size() % 32) {
+        item.push_back(item.back());
+        lev.push_back((unsigned short)kPairNone);
+      }
+    }
+  return upload_pairs(P, item, lev);
+}
+
+// Per-edge records of k_edge (DMeshT::edge_idx, edge_geo).
+template <typename R>
+void build_edge_records(EngineImpl &P, DMeshT<R> &d) {
+  const MeshHost &M = P.mesh;
+  const int E = M.edge2D, S = P.S;
+  std::vector<int4> idx(3 * (size_t)E);
+  std::vector<R> geo(16 * (size_t)E, R(0));
+  for (int s = 0; s < E; s++) {
+    const int e = P.slot_edge[s], n1 = M.edge_nodes[2 * e], n2 = M.edge_nodes[2 * e + 1];
+    const int u = M.up_dn_tri[2 * e], w = M.up_dn_tri[2 * e + 1];
+    const bool pair = u >= 0 && w >= 0;
+    int un[3] = {n1, n1, n1}, dn[3] = {n2, n2, n2};
+    R *g = &geo[16 * (size_t)s];
+    if (pair)
+      for (int q = 0; q < 3; q++) {
+        un[q] = M.elem_nodes[3 * (size_t)u + q];
+        dn[q] = M.elem_nodes[3 * (size_t)w + q];
+      }
+    for (int q = 0; pair && q < 6; q++) {
+      g[q] = (R)M.grad_sca[6 * (size_t)u + q];
+      g[6 + q] = (R)M.grad_sca[6 * (size_t)w + q];
+    }
+    g[12] = (R)M.edge_dxdy[2 * (size_t)e] * (R)M.edge_a[e];
+    g[13] = (R)M.edge_dxdy[2 * (size_t)e + 1] * (R)kREarthD;
+    idx[3 * (size_t)s] = make_int4(n1 * S, n2 * S, un[0] * S, un[1] * S);
+    idx[3 * (size_t)s + 1] = make_int4(un[2] * S, dn[0] * S, dn[1] * S, dn[2] * S);
+    idx[3 * (size_t)s + 2] = make_int4(edge_tri_levels(M, e), M.nboundary_lay[n1], M.nboundary_lay[n2], M.edge_levels(e));
+  }
+  d.edge_idx = P.upload(idx);
+  d.edge_geo = P.upload(geo);
+}
+
+// Pair schedule of the columns.  A warp takes whole columns, so that their
+// vertical neighbours are the lanes beside; within a window of nodes they are
+// placed largest first into the fullest warp that still holds them (windows of 32
+// and 64 nodes leave more lanes idle: k_col1 5-10 % slower; a Morton order of the
+// nodes instead of their own was slower too).  Columns
+// of more than 32 pairs are cut into pieces that overlap by one pair at each cut
+// (halo lanes: computed, not stored).
+DPairs build_node_pairs(EngineImpl &P) {
+  const MeshHost &M = P.mesh;
+  struct Piece {
+    int node, first, n;  // pairs
+    bool lo, hi;         // its first / last pair is a halo
+  };
+  const int N = M.nod2D, window = 256;
+  std::vector<int> item;
+  std::vector<unsigned short> lev;
+  std::vector<Piece> pieces;
+  std::vector<std::vector<int>> by_n(33), warps, open(33);
+  for (int n0 = 0; n0 < N; n0 += window) {
+    pieces.clear();
+    warps.clear();
+    for (auto &v : by_n) v.clear();
+    for (auto &v : open) v.clear();
+    for (int n = n0; n < std::min(N, n0 + window); n++) {
+      const int np = M.nlev_node[n] / 2;  // pairs of nlev - 1 layers
+      for (int p = 0; p < np;) {
+        const bool lo = p > 0;
+        const int left = np - p + (lo ? 1 : 0);  // with the leading halo
+        const Piece c{n, lo ? p - 1 : 0, std::min(left, 32), lo, left > 32};
+        p = c.first + c.n - (c.hi ? 1 : 0);
+        by_n[c.n].push_back((int)pieces.size());
+        pieces.push_back(c);
+      }
+    }
+    for (int n = 32; n >= 1; n--)
+      for (int i : by_n[n]) {
+        int r = n;
+        while (r <= 32 && open[r].empty()) r++;
+        int w;
+        if (r > 32) {
+          w = (int)warps.size();
+          warps.emplace_back();
+          r = 32;
+        } else {
+          w = open[r].back();
+          open[r].pop_back();
+        }
+        warps[w].push_back(i);
+        if (r - n > 0) open[r - n].push_back(w);
+      }
+    for (auto &w : warps) {
+      for (int i : w) {
+        const Piece &c = pieces[i];
+        for (int q = 0; q < c.n; q++) {
+          const bool halo = (c.lo && q == 0) || (c.hi && q == c.n - 1);
+          item.push_back(c.node);
+          lev.push_back((unsigned short)((halo ? kPairHalo : 0u) | (unsigned)(2 * (c.first + q))));
+        }
+      }
+      while (item.size() % 32) {
+        item.push_back(item.back());
+        lev.push_back((unsigned short)kPairNone);
+      }
+    }
+  }
+  return upload_pairs(P, item, lev);
+}
+
+// Node records of the column kernels (DMeshT::nrec, ne6).
+template <typename R>
+void build_node_records(EngineImpl &P, DMeshT<R> &d, const std::vector<int> &edge_slot) {
+  const MeshHost &M = P.mesh;
+  const int N = M.nod2D, S = P.S;
+  std::vector<int> holds(N, 0);
+  for (int e = 0; e < M.elem2D; e++)
+    for (int q = 0; q < 3; q++) holds[M.elem_nodes[3 * (size_t)e + q]]++;
+  std::vector<int4> rec(N), ne(3 * (size_t)N);
+  for (int n = 0; n < N; n++) {
+    const int p0 = M.node_edge_ptr[n], deg = M.node_edge_ptr[n + 1] - p0;
+    const bool full = (M.ring_ptr[n + 1] - M.ring_ptr[n]) == holds[n];
+    if (deg > 0xffff) throw std::invalid_argument("a node has more than 65535 edges");
+    unsigned lev[2] = {0, 0}, r[12];
+    for (int i = 0; i < 6; i++) {
+      r[2 * i] = 0;
+      r[2 * i + 1] = (unsigned)n * (unsigned)S;
+      if (i >= deg) continue;
+      const int code = M.node_edge[p0 + i], e = code >> 1, second = code & 1;
+      r[2 * i] = (unsigned)edge_slot[e] * (unsigned)S;
+      r[2 * i + 1] = (unsigned)M.edge_nodes[2 * (size_t)e + (second ? 0 : 1)] * (unsigned)S | (unsigned)second << 31;
+      lev[i / 3] |= (unsigned)M.edge_levels(e) << (10 * (i % 3));
+    }
+    rec[n] = make_int4(M.nlev_node[n] | deg << 16, (int)((unsigned)M.nlev_node_min[n] | (full ? 0x80000000u : 0u)), (int)lev[0],
+                       (int)lev[1]);
+    for (int i = 0; i < 3; i++)
+      ne[3 * (size_t)n + i] = make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]);
+  }
+  d.nrec = P.upload(rec);
+  d.ne6 = P.upload(ne);
+}
+
 template <typename R>
 void build_dmesh(EngineImpl &P, DMeshT<R> &d, const std::vector<int> &slot_edge, const std::vector<int> &edge_slot) {
   const MeshHost &M = P.mesh;
@@ -152,16 +327,6 @@ void build_dmesh(EngineImpl &P, DMeshT<R> &d, const std::vector<int> &slot_edge,
   d.elem_area = upload_conv<R>(P, M.elem_area);
   d.ring_ptr = P.upload(M.ring_ptr);
   d.ring_elem = P.upload(M.ring_elem);
-  {
-    // complete rings: every element holding the node is listed (the
-    // reference's periodic compat lists are not, on the wrap rows)
-    std::vector<int> holds(N, 0);
-    for (int e = 0; e < T; e++)
-      for (int q = 0; q < 3; q++) holds[M.elem_nodes[3 * e + q]]++;
-    std::vector<unsigned char> full(N);
-    for (int n = 0; n < N; n++) full[n] = (M.ring_ptr[n + 1] - M.ring_ptr[n]) == holds[n];
-    d.ring_full = P.upload(full);
-  }
   d.ne_ptr = P.upload(M.node_edge_ptr);
   {
     std::vector<int4> ne4(M.node_edge.size());
@@ -182,6 +347,10 @@ void build_dmesh(EngineImpl &P, DMeshT<R> &d, const std::vector<int> &slot_edge,
   d.helem = upload_cols<R>(P, M.helem.data(), L, T, L);
 
   build_schedules(P, d, kCellsPerBlock);
+  build_edge_records(P, d);
+  d.edge_pairs = build_edge_pairs(P);
+  build_node_records(P, d, edge_slot);
+  d.node_pairs = build_node_pairs(P);
 }
 
 // Patch plan of the fused step kernel: built on the host, uploaded, host
@@ -225,6 +394,22 @@ void build_tiles(EngineImpl &P, const std::vector<int> &edge_slot, int owned) {
 }  // namespace
 
 static_assert(Engine::kDefaultCellsPerBlock == kCellsPerBlock, "one default schedule tile");
+
+bool uniform_levels(const MeshHost &M, int *deepest) {
+  const int N = M.nod2D, L = M.nl - 1;
+  int nd = 0;
+  for (int n = 1; n < N; n++)
+    if (M.nlev_node[n] > M.nlev_node[nd]) nd = n;
+  *deepest = nd;
+  if (N <= 0) return false;
+  const size_t w = sizeof(double);
+  const double *h = &M.hnode[(size_t)nd * L], *hn = &M.hnode_new[(size_t)nd * L];
+  for (int n = 0; n < N; n++) {
+    const size_t b = w * (M.nlev_node[n] - 1);
+    if (std::memcmp(&M.hnode[(size_t)n * L], h, b) || std::memcmp(&M.hnode_new[(size_t)n * L], hn, b)) return false;
+  }
+  return true;
+}
 
 std::vector<int> edge_slot_order(const MeshHost &M) {
   // slot order: edges sorted by their smaller node id (stable in edge id)
@@ -373,11 +558,11 @@ void Engine::allocate_tracers(int ntr, bool with_ab) {
 void Engine::release_work() {
   EngineImpl &P = *p_;
   CK(cudaStreamSynchronize(P.stream));
-  P.dfree(P.adfh[0]);  // the interleaved arrays: one allocation each
-  P.dfree(P.lo[0]);
-  P.dfree(P.adfv[0]);
+  for (void **q : {&P.adfh, &P.lo, &P.adfv}) {
+    P.dfree(*q);
+    *q = nullptr;
+  }
   for (int t = 0; t < P.slots; t++) {
-    P.adfh[t] = P.lo[t] = P.adfv[t] = nullptr;
     for (void **q : {&P.rpm[t], &P.gradn[t]}) {
       P.dfree(*q);
       *q = nullptr;
@@ -474,18 +659,15 @@ static void ensure_slots(EngineImpl &P, int n) {
   if (n <= P.slots) return;
   const size_t ns = (size_t)P.mesh.nod2D * P.S * P.r_bytes, es = (size_t)P.mesh.edge2D * P.S * P.r_bytes;
   if (!P.vflux) P.vflux = P.dalloc_bytes(es);
-  // adf_h, lo and adf_v are interleaved by tracer (a batch of NT tracers uses stride
-  // NT): one array each, reallocated for the larger batch
+  // adf_h, lo and adf_v hold a batch's tracers side by side: one array each,
+  // reallocated for the larger batch
   CK(cudaStreamSynchronize(P.stream));
-  P.dfree(P.adfh[0]);
-  P.dfree(P.lo[0]);
-  P.dfree(P.adfv[0]);
-  char *ah = (char *)P.dalloc_bytes(n * es), *lo = (char *)P.dalloc_bytes(n * ns), *av = (char *)P.dalloc_bytes(n * ns);
-  for (int t = 0; t < n; t++) {
-    P.adfh[t] = ah + t * P.r_bytes;
-    P.lo[t] = lo + t * P.r_bytes;
-    P.adfv[t] = av + t * P.r_bytes;
-  }
+  P.dfree(P.adfh);
+  P.dfree(P.lo);
+  P.dfree(P.adfv);
+  P.adfh = P.dalloc_bytes(n * es);
+  P.lo = P.dalloc_bytes(n * ns);
+  P.adfv = P.dalloc_bytes(n * ns);
   for (int t = P.slots; t < n; t++) {
     P.rpm[t] = P.dalloc_bytes(2 * ns);
     P.gradn[t] = P.dalloc_bytes(2 * ns);
@@ -520,9 +702,6 @@ static void run_batch(EngineImpl &P, int first, int nt, double dt, bool refresh_
     if (!refresh_ab && !tr.TAB) throw std::invalid_argument("tracer has no valuesAB array: advance with valuesAB := values");
     b.TAB[t] = refresh_ab ? tr.T : tr.TAB;
     b.T_out[t] = tr.Tout;
-    b.adf_h[t] = P.adfh[t];
-    b.adf_v[t] = P.adfv[t];
-    b.lo[t] = P.lo[t];
     b.rpm[t] = P.rpm[t];
     b.gradn[t] = P.gradn[t];
     if (learned_active(P) && tr.sch.hor == 1) learned_slot_buffers(P, t, &b.feat[t], &b.fscale[t]);
@@ -530,6 +709,9 @@ static void run_batch(EngineImpl &P, int first, int nt, double dt, bool refresh_
     b.seed[t] = mix32_host(P.sround_seed ^ mix32_host((uint32_t)(first + t) * 0x9e3779b9u + tr.nstep));
     tr.nstep++;
   }
+  b.adf_h = P.adfh;
+  b.adf_v = P.adfv;
+  b.lo = P.lo;
   b.sround = storage16(P) ? P.sround : 0;
   // the velocity only changes through set_velocity: the first launch after it
   // stores the edge volume fluxes, later ones load them
@@ -666,9 +848,9 @@ void Engine::step_with_scratch(int id, const double *T, const double *TAB, doubl
   b.TAB[0] = TAB;
   b.T_out[0] = T_out;
   b.vflux = scratch;
-  b.adf_h[0] = scratch + es;
-  b.adf_v[0] = scratch + 2 * es;
-  b.lo[0] = scratch + 2 * es + ns;
+  b.adf_h = scratch + es;
+  b.adf_v = scratch + 2 * es;
+  b.lo = scratch + 2 * es + ns;
   b.rpm[0] = scratch + 2 * es + 2 * ns;  // 2 ns
   b.gradn[0] = scratch + 2 * es + 4 * ns;
   dispatch(P, P.tr[id].sch, 1, b, dt);

@@ -28,9 +28,7 @@ struct BatchPtrs {
   const void *T[kBatchMax] = {};
   const void *TAB[kBatchMax] = {};
   void *T_out[kBatchMax] = {};
-  void *adf_h[kBatchMax] = {};
-  void *adf_v[kBatchMax] = {};
-  void *lo[kBatchMax] = {};
+  void *adf_h = nullptr, *adf_v = nullptr, *lo = nullptr;  // work arrays of the whole batch
   void *rpm[kBatchMax] = {};  // (2, S, node): R+ and R- side by side
   void *vflux = nullptr;
   int vflux_mode = 0;             // edge volume fluxes (FusedArgs::vflux_mode)
@@ -92,7 +90,7 @@ struct EngineImpl {
   TilePlanHost tplan;
   DTiles tiles{};
   int step_path = 1;
-  void *adfh[kBatchMax] = {}, *adfv[kBatchMax] = {}, *lo[kBatchMax] = {}, *rpm[kBatchMax] = {};
+  void *adfh = nullptr, *adfv = nullptr, *lo = nullptr, *rpm[kBatchMax] = {};
   void *gradn[kBatchMax] = {};
 
   // launch profiling: when prof is set, every launch is bracketed by events
@@ -171,7 +169,10 @@ void launch_batch_f64fma(EngineImpl &P, const TracerScheme &sc, int nt, const Ba
 // Whether the fused patch kernel runs a batch of this scheme (precision,
 // storage type, vertical scheme, learned flux and plan permitting).
 bool fused_step(const EngineImpl &P, const TracerScheme &sc, bool learned);
-// Geometry reciprocals of k_col3 (step_f64.cu / step_f32.cu).
+// Whether every node has the same hnode and hnode_new at each of its wet levels;
+// *deepest = a node with the most levels (engine.cu).
+bool uniform_levels(const MeshHost &M, int *deepest);
+// Geometry reciprocals and level tables (step_f64.cu / step_f32.cu).
 void build_rcp_f64(EngineImpl &P);
 void build_rcp_f32(EngineImpl &P);
 // Compensated FP64 sums of T and of T * areasvol * hnode_new over the wet

@@ -35,19 +35,22 @@ void set_smem(K kernel, size_t bytes) {
 template <typename R, typename TS, int NT, int HOR, int LIM>
 void launch_edge(EngineImpl &P, const FusedArgs<R, TS> &a) {
   const DMeshT<R> &m = dmesh<R>(P);
-  if (m.edge_sched.nblk <= 0) return;
+  if (m.edge_pairs.nwarps <= 0) return;
+  const int per = pair_run(m.edge_pairs, kEdgeRun), grid = pair_blocks(m.edge_pairs, kEdgeThreads, per);
   P.mark_begin(KK_EDGE);
-  k_edge<R, TS, NT, HOR, LIM><<<m.edge_sched.nblk, kThreads, smem_edge(), P.stream>>>(m, a);
+  if (a.vflux_mode == 2) k_edge<R, TS, NT, HOR, LIM, true><<<grid, kEdgeThreads, 0, P.stream>>>(m, a, per);
+  else k_edge<R, TS, NT, HOR, LIM, false><<<grid, kEdgeThreads, 0, P.stream>>>(m, a, per);
   P.mark_end();
 }
 
 template <typename R, typename TS, int NT, int VER, int LIM>
 void launch_col1(EngineImpl &P, const FusedArgs<R, TS> &a) {
   const DMeshT<R> &m = dmesh<R>(P);
-  const size_t sm = StageIncidence<R>::col1 ? smem_col_staged<R>(NT, 2) : smem_col<R>(NT, 2);
-  set_smem(k_col1<R, TS, NT, VER, LIM>, sm);
+  const int per = pair_run(m.node_pairs, kColRun);
+  const int grid = pair_blocks(m.node_pairs, kColThreads, per);
   P.mark_begin(KK_COL1);
-  k_col1<R, TS, NT, VER, LIM><<<m.node_sched.nblk, kThreads, sm, P.stream>>>(m, a);
+  if (VER != VER_PPM || m.uniform_h) k_col1<R, TS, NT, VER, LIM, true><<<grid, kColThreads, 0, P.stream>>>(m, a, per);
+  else k_col1<R, TS, NT, VER, LIM, VER != VER_PPM><<<grid, kColThreads, 0, P.stream>>>(m, a, per);
   P.mark_end();
 }
 
@@ -64,7 +67,15 @@ template <typename R, typename TS, int NT, int LIM>
 void run_group(EngineImpl &P, const TracerScheme &sc, const FusedArgs<R, TS> &a) {
   if (sc.hor != 0) launch_grad<R, TS, NT>(P, a);
   switch (sc.hor) {
-    case 1: launch_edge<R, TS, NT, HOR_MUSCL, LIM>(P, a); break;
+    case 1:
+      if constexpr (std::is_same<R, float>::value && std::is_same<TS, float>::value) {
+        if (a.feat[0]) {
+          launch_edge<R, TS, NT, HOR_MUSCL_FEAT, LIM>(P, a);
+          break;
+        }
+      }
+      launch_edge<R, TS, NT, HOR_MUSCL, LIM>(P, a);
+      break;
     case 2: launch_edge<R, TS, NT, HOR_MFCT, LIM>(P, a); break;
     default: launch_edge<R, TS, NT, HOR_UPW1, LIM>(P, a); break;
   }
@@ -78,21 +89,18 @@ void run_group(EngineImpl &P, const TracerScheme &sc, const FusedArgs<R, TS> &a)
     default: launch_col1<R, TS, NT, VER_UPW1, LIM>(P, a); break;
   }
   const DMeshT<R> &m = dmesh<R>(P);
+  const int per = pair_run(m.node_pairs, kColRun), nb = pair_blocks(m.node_pairs, kColThreads, per);
   if (LIM == LIM_FCT) {
-    const size_t sm2 = StageIncidence<R>::col2 ? smem_col_staged<R>(NT, 2) : smem_col<R>(NT, 2);
-    set_smem(k_col2<R, TS, NT>, sm2);
     P.mark_begin(KK_COL2);
-    k_col2<R, TS, NT><<<m.node_sched.nblk, kThreads, sm2, P.stream>>>(m, a);
+    k_col2<R, TS, NT><<<nb, kColThreads, 0, P.stream>>>(m, a, per);
     P.mark_end();
   }
-  const size_t sm3 = StageIncidence<R>::col3 ? smem_col_staged<R>(NT, 0) : smem_col<R>(NT, 0);
-  set_smem(k_col3<R, TS, NT, LIM>, sm3);
   P.mark_begin(KK_COL3);
-  k_col3<R, TS, NT, LIM><<<m.node_sched.nblk, kThreads, sm3, P.stream>>>(m, a);
+  k_col3<R, TS, NT, LIM><<<nb, kColThreads, 0, P.stream>>>(m, a, per);
   P.mark_end();
 }
 
-// Geometry reciprocals of k_col3 (k_rcp_planes), once per mesh.
+// Geometry reciprocals (k_rcp_planes) and level tables, once per mesh.
 template <typename R>
 void build_rcp_planes_t(EngineImpl &P, DMeshT<R> &d) {
   const size_t plane = (size_t)d.S * d.N;
@@ -100,9 +108,22 @@ void build_rcp_planes_t(EngineImpl &P, DMeshT<R> &d) {
   const int grid = (int)std::min<size_t>((plane + 255) / 256, (size_t)148 * 32);
   k_rcp_planes<R><<<std::max(grid, 1), 256, 0, P.stream>>>(d, rcp);
   CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(P.stream));
   d.rcp = rcp;
   d.rcp_plane = plane;
+  // the deepest column stands for every one where the levels are uniform
+  int nd = 0;
+  const bool uni = uniform_levels(P.mesh, &nd);
+  const size_t base = uni ? (size_t)nd * d.S : 0;
+  d.uniform_h = uni;
+  d.hS = uni ? 0 : d.S;
+  d.hT = d.hnode + base;
+  d.hnT = d.hnode_new + base;
+  d.yhnT = rcp + plane + base;
+  R *lt = (R *)P.dalloc_bytes((size_t)LT_COUNT * d.S * sizeof(R));
+  if (d.N > 0) k_level_tables<R><<<1, 256, 0, P.stream>>>(d, nd, lt);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(P.stream));
+  d.ltab = lt;
 }
 
 // Edge volume fluxes of every edge level (the values k_edge computes and
@@ -156,8 +177,25 @@ void run_tiles(EngineImpl &P, const TracerScheme &sc, int nt, const BatchPtrs &b
   }
 }
 
+// A batch of one FP64 tracer on caller-owned buffers that are only 8-byte
+// aligned (tracer_advect_device_noalloc) runs the kernels built without
+// vector accesses of the tracer columns.
+inline bool pair_aligned(const BatchPtrs &b, int nt, size_t ts_bytes) {
+  for (int t = 0; t < nt; t++)
+    for (const void *p : {b.T[t], b.TAB[t], (const void *)b.T_out[t]})
+      if (((uintptr_t)p) % (2 * ts_bytes)) return false;
+  return true;
+}
+
 template <typename R, typename TS>
 void launch_batch_t(EngineImpl &P, const TracerScheme &sc, int nt, const BatchPtrs &b, double dt) {
+  if constexpr (std::is_same<TS, double>::value) {
+    if (!pair_aligned(b, nt, sizeof(TS)) && !fused_step(P, sc, false)) {
+      if (nt != 1) throw std::invalid_argument("unaligned tracer buffers: one tracer at a time");
+      launch_batch_t<R, f64u>(P, sc, nt, b, dt);
+      return;
+    }
+  }
   if constexpr (std::is_same<R, TS>::value) {
     if (fused_step(P, sc, b.feat[0] != nullptr)) {
       run_tiles<R>(P, sc, nt, b, dt);
@@ -169,14 +207,14 @@ void launch_batch_t(EngineImpl &P, const TracerScheme &sc, int nt, const BatchPt
     a.T[t] = (const TS *)b.T[t];
     a.TAB[t] = (const TS *)b.TAB[t];
     a.T_out[t] = (TS *)b.T_out[t];
-    a.adf_h[t] = (R *)b.adf_h[t];
-    a.adf_v[t] = (R *)b.adf_v[t];
-    a.lo[t] = (R *)b.lo[t];
     a.rpm[t] = (R *)b.rpm[t];
     a.gradn[t] = (R *)b.gradn[t];
     a.feat[t] = (__nv_bfloat16 *)b.feat[t];
     a.fscale[t] = (float *)b.fscale[t];
   }
+  a.adf_h = (R *)b.adf_h;
+  a.adf_v = (R *)b.adf_v;
+  a.lo = (R *)b.lo;
   a.vflux = (R *)b.vflux;
   a.vel = (const R *)P.vel;
   a.W = (const R *)P.W;
@@ -191,7 +229,11 @@ void launch_batch_t(EngineImpl &P, const TracerScheme &sc, int nt, const BatchPt
   a.vflux_mode = b.vflux_mode;
   a.nonfinite = P.nonfinite_d;
   const bool fct = sc.lim == 1;
-  if (nt == 4) fct ? run_group<R, TS, 4, LIM_FCT>(P, sc, a) : run_group<R, TS, 4, LIM_NONE>(P, sc, a);
+  if constexpr (std::is_same<TS, f64u>::value) {
+    fct ? run_group<R, TS, 1, LIM_FCT>(P, sc, a) : run_group<R, TS, 1, LIM_NONE>(P, sc, a);
+    return;
+  }
+  else if (nt == 4) fct ? run_group<R, TS, 4, LIM_FCT>(P, sc, a) : run_group<R, TS, 4, LIM_NONE>(P, sc, a);
   else if (nt == 2) fct ? run_group<R, TS, 2, LIM_FCT>(P, sc, a) : run_group<R, TS, 2, LIM_NONE>(P, sc, a);
   else fct ? run_group<R, TS, 1, LIM_FCT>(P, sc, a) : run_group<R, TS, 1, LIM_NONE>(P, sc, a);
 }

@@ -605,16 +605,16 @@ struct LearnedState {
 
 namespace {
 
-// adf: tracer t's slot of the batch's tracer-interleaved antidiffusive fluxes
-// (stride nt)
-__global__ void __launch_bounds__(kThreads) k_learn_apply(DMeshT<float> m, float *adf, int nt, const float *scale,
+// tracer t of the batch's antidiffusive fluxes (NT tracers side by side)
+template <int NT>
+__global__ void __launch_bounds__(kThreads) k_learn_apply(DMeshT<float> m, float *adf, int t, const float *scale,
                                                          const float *y) {
   extern __shared__ int smem[];
   int *s_off = smem, *s_item = smem + kMaxItemsPerBlock + 1;
   const CellMap cm = map_cells(m.edge_sched, blockIdx.x, s_off, s_item);
   for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
     const int j = s_item[lc], e = cm.i0 + j, k = lc - (s_off[j] - cm.c0), cell = cm.c0 + lc;
-    adf[((size_t)e * m.S + k) * nt] += scale[cell] * y[cell];
+    il<NT>(adf, t, (cix)e * m.S + k) += scale[cell] * y[cell];
   }
 }
 
@@ -819,9 +819,10 @@ void learned_correct_f32(EngineImpl &P, int nt, const FusedArgs<float, float> &a
   for (int t = 0; t < nt; t++) {
     if (mlp_forward_dev(L.mlp, a.feat[t], L.ncells, L.y[t], P.stream) != 0)
       throw std::runtime_error("learned flux: MLP forward launch failed");
-    if (P.dm32.edge_sched.nblk > 0)
-      k_learn_apply<<<P.dm32.edge_sched.nblk, kThreads, smem_edge(), P.stream>>>(P.dm32, a.adf_h[t], nt, a.fscale[t],
-                                                                                  L.y[t]);
+    if (P.dm32.edge_sched.nblk > 0) {
+      auto *apply = nt == 4 ? k_learn_apply<4> : (nt == 2 ? k_learn_apply<2> : k_learn_apply<1>);
+      apply<<<P.dm32.edge_sched.nblk, kThreads, smem_edge(), P.stream>>>(P.dm32, a.adf_h, t, a.fscale[t], L.y[t]);
+    }
     CK(cudaGetLastError());
   }
 }
@@ -926,15 +927,15 @@ double Engine::learn_step(const double *T_in, const double *T_target, double dt,
         L.hm = dmalloc<float>((size_t)P.mesh.nod2D * P.S);
       }
       k_learn_fct_g<<<m.node_sched.nblk, kThreads, smem_edge(), P.stream>>>(
-          m, T, L.target, c, (const float *)P.adfh[0], (const float *)P.adfv[0], (const float *)P.rpm[0],
+          m, T, L.target, c, (const float *)P.adfh, (const float *)P.adfv, (const float *)P.rpm[0],
           (const float *)P.rpm[0] + 1, (float)dt, L.hp, L.hm);
       CK(cudaGetLastError());
       k_learn_dy_fct<<<m.edge_sched.nblk, kThreads, smem_edge(), P.stream>>>(
-          m, T, L.target, c, L.fscale[0], (const float *)P.adfh[0], (const float *)P.rpm[0], (const float *)P.rpm[0] + 1,
+          m, T, L.target, c, L.fscale[0], (const float *)P.adfh, (const float *)P.rpm[0], (const float *)P.rpm[0] + 1,
           L.hp, L.hm, L.dy);
     } else {
       k_learn_dy<<<m.edge_sched.nblk, kThreads, smem_edge(), P.stream>>>(
-          m, T, L.target, L.fscale[0], c, (const float *)P.adfh[0], fct ? (const float *)P.rpm[0] : nullptr,
+          m, T, L.target, L.fscale[0], c, (const float *)P.adfh, fct ? (const float *)P.rpm[0] : nullptr,
           fct ? (const float *)P.rpm[0] + 1 : nullptr, L.dy);
     }
     CK(cudaGetLastError());
