@@ -46,6 +46,12 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
          | ((uint32_t)(M >> 4) << 24);    // M / 16
 }
 
+// operand read transposed: stored with its M (N) dimension contiguous.  In the
+// no-swizzle layout the descriptor's SBO then steps 8 elements of M (N) and its
+// LBO 8 of K, so a K-major tile of C columns holding [k][m] has LBO = C / 8 x 128,
+// SBO = 128.
+constexpr uint32_t kAMnMajor = 1u << 15, kBMnMajor = 1u << 16;
+
 // --- TMEM allocation (one full warp executes each) -----------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t *smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)),
