@@ -285,6 +285,25 @@ __device__ __forceinline__ R div6(R x, bool &bad) { return div_3k<6>(x, bad); }
 template <typename R>
 __device__ __forceinline__ R div3(R x, bool &bad) { return div_3k<3>(x, bad); }
 
+// a / b given y = RN(1 / b), correctly rounded (see div_rcp), straight-line:
+// numerators outside [2^-900, 2^900] other than zero set `bad` and the caller
+// divides again.  The sign of a zero result is not kept (no output of the step
+// depends on the sign of a zero quotient).
+__device__ __forceinline__ double div_fast(double a, double b, double y, bool &bad) {
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  const unsigned u = 2u * (unsigned)__double2hiint(a);
+  bad |= (u - 0x0f600000u > 0xf0800000u - 0x0f600000u) && u != 0u;
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+__device__ __forceinline__ float div_fast(float a, float b, float y, bool &bad) {
+  float q = a * y;
+  q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+  const unsigned u = 2u * __float_as_uint(a);
+  bad |= (u - 0x1b000000u > 0xe3000000u - 0x1b000000u) && u != 0u;
+  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
 // learned flux: 16 features of one MUSCL edge level in the flow's frame, in
 // units of the local variation sig, and the scale of the network's output
 template <typename TS>
@@ -298,9 +317,21 @@ __device__ __forceinline__ void edge_features(const DMeshT<float> &m, const Fuse
   const float xu = fwd ? x1 : -x2, xd = fwd ? x2 : -x1;
   const float face = 0.5f * (Tmean1 + Tmean2);
   const float sig = fabsf(td - tu) + (fabsf(xu) + fabsf(xd)) * sixth + 1e-6f * (fabsf(tu) + fabsf(td)) + 1e-20f;
-  const float inv = 1.0f / sig;
+  // the two quotients straight-line: an approximate reciprocal within a unit in
+  // the last place and one Newton step round 1 / x (see div_any), Markstein's
+  // correction the quotient
+  auto rcp = [](float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return __fmaf_rn(__fmaf_rn(-x, y, 1.0f), y, y);
+  };
+  const float inv = rcp(sig);
   const cix ou = fwd ? o1 : o2;
-  const float cour = fminf(fabsf(vflux) * a.dt / (m.areasvol[ou] * m.hnode_new[ou]), 4.0f);
+  bool bad = false;
+  const float num = fabsf(vflux) * a.dt, vol = m.areasvol[ou] * m.hnode_new[ou];
+  float cour = div_fast(num, vol, rcp(vol), bad);
+  if (bad) cour = num / vol;
+  cour = fminf(cour, 4.0f);
   const float gx = fwd ? gux : gdx, gy = fwd ? guy : gdy;
   const float trans = (-eyr * gx + exa * gy) * inv;
   float f[16];
@@ -589,25 +620,6 @@ __device__ __forceinline__ void for_edges(const DMeshT<R> &m, int n, int k, cons
       f((cix)(q.x >> 1) * m.S + k, (cix)q.w + k, (q.x & 1) != 0, q.z);
     }
   }
-}
-
-// a / b given y = RN(1 / b), correctly rounded (see div_rcp), straight-line:
-// numerators outside [2^-900, 2^900] other than zero set `bad` and the caller
-// divides again.  The sign of a zero result is not kept (no output of the step
-// depends on the sign of a zero quotient).
-__device__ __forceinline__ double div_fast(double a, double b, double y, bool &bad) {
-  double q = a * y;
-  q = __fma_rn(__fma_rn(-b, q, a), y, q);
-  const unsigned u = 2u * (unsigned)__double2hiint(a);
-  bad |= (u - 0x0f600000u > 0xf0800000u - 0x0f600000u) && u != 0u;
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-__device__ __forceinline__ float div_fast(float a, float b, float y, bool &bad) {
-  float q = a * y;
-  q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-  const unsigned u = 2u * __float_as_uint(a);
-  bad |= (u - 0x1b000000u > 0xe3000000u - 0x1b000000u) && u != 0u;
-  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
 // PPM weights of one column level (lib/oce_adv_tra_ver.F90:525-553): c1, c2, c3

@@ -95,12 +95,37 @@ __device__ __forceinline__ float tanh_fast(float x) {
   return y;
 }
 constexpr float kGeluC = 0.7978845608028654f, kGeluA = 0.044715f;
-// acc + GELU(z) w3 with hw3 = w3 / 2, i.e. acc + hw3 z (1 + tanh u):
-// u = z (c + c a z^2), then one add and one FMA
-__device__ __forceinline__ float gelu_out(float z, float hw3, float acc) {
-  const float t = tanh_fast(z * fmaf(kGeluC * kGeluA, z * z, kGeluC));
-  const float hz = z * hw3;
-  return fmaf(hz, t, acc + hz);
+// Packed pairs of FP32 values: one instruction for two operations on sm_100.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// acc + GELU(z) w3 with hw3 = w3 / 2, i.e. acc + hw3 z (1 + tanh u), for two hidden
+// units: u = z (c + c a z^2), then one add and one FMA
+__device__ __forceinline__ f32x2 gelu_out2(f32x2 z, f32x2 hw3, f32x2 acc) {
+  const f32x2 ca = pack2(kGeluC * kGeluA, kGeluC * kGeluA), c = pack2(kGeluC, kGeluC);
+  float u0, u1;
+  unpack2(mul2(z, fma2(ca, mul2(z, z), c)), u0, u1);
+  const f32x2 hz = mul2(z, hw3);
+  return fma2(hz, pack2(tanh_fast(u0), tanh_fast(u1)), add2(acc, hz));
 }
 
 // The first inference epilogue evaluates GELU on packed FP16 pairs (two
@@ -123,15 +148,19 @@ __device__ __forceinline__ __half2 gelu2(__half2 z) {
   return __hfma2(hz, tanh_fast2(u), hz);             // z/2 (1 + tanh u)
 }
 // 16 FP32 pre-activations (bias added) -> GELU -> 16 BF16 in two 16-byte stores
-// (bias: 16-byte aligned shared memory, read as four 16-byte vectors)
+// (bias: 16-byte aligned shared memory)
 __device__ __forceinline__ void gelu_store16(unsigned char *base, uint32_t off_lo, uint32_t off_hi, const float *v,
                                              const float *bias_s) {
   __align__(16) __nv_bfloat162 o[8];
-  float bias[16];
-  for (int i = 0; i < 4; i++) reinterpret_cast<float4 *>(bias)[i] = reinterpret_cast<const float4 *>(bias_s)[i];
-  for (int i = 0; i < 8; i++) {
-    const __half2 g = gelu2(__floats2half2_rn(v[2 * i] + bias[2 * i], v[2 * i + 1] + bias[2 * i + 1]));
-    o[i] = __float22bfloat162_rn(__half22float2(g));
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const ulonglong2 b = reinterpret_cast<const ulonglong2 *>(bias_s)[i];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      float z0, z1;
+      unpack2(add2(pack2(v[4 * i + 2 * j], v[4 * i + 2 * j + 1]), j == 0 ? b.x : b.y), z0, z1);
+      o[2 * i + j] = __float22bfloat162_rn(__half22float2(gelu2(__floats2half2_rn(z0, z1))));
+    }
   }
   *reinterpret_cast<uint4 *>(base + off_lo) = *reinterpret_cast<const uint4 *>(o);
   *reinterpret_cast<uint4 *>(base + off_hi) = *reinterpret_cast<const uint4 *>(o + 4);
@@ -210,8 +239,35 @@ __device__ __forceinline__ void smem_to_tc() {
 // side; their tiles' load, MMA and epilogue phases overlap one another.
 constexpr uint32_t kFwdTmemCols = 64;
 
-__global__ void __launch_bounds__(128, 1)
-    k_mlp_fwd(const __nv_bfloat16 *X, long long S, MlpDev w, float *y, int *status) {
+// Where the network's output of a sample goes: begin() at the start of its tile,
+// load() ahead of the last epilogue and store() after it, so that what the store
+// needs is there by then.
+struct StoreY {
+  float *y;
+  __device__ __forceinline__ void begin(long long, bool) {}
+  __device__ __forceinline__ void load(bool) {}
+  __device__ __forceinline__ void store(long long s, float v) const { y[s] = v; }
+};
+// scale x output added to tracer t's antidiffusive flux of the sample's edge cell
+// (NT tracers side by side)
+template <int NT>
+struct AddFlux {
+  float *adf;
+  const float *scale;
+  const unsigned *cell;  // slot x S + level of every sample
+  int t;
+  cix o;
+  float f, c;
+  __device__ __forceinline__ void begin(long long s, bool on) {
+    o = on ? cell[s] : 0u;
+    c = on ? scale[s] : 0.f;
+  }
+  __device__ __forceinline__ void load(bool on) { f = on ? il<NT>(adf, t, o) : 0.f; }
+  __device__ __forceinline__ void store(long long, float v) { il<NT>(adf, t, o) = f + c * v; }
+};
+
+template <typename Out>
+__global__ void __launch_bounds__(128, 7) k_mlp_fwd(const __nv_bfloat16 *X, long long S, MlpDev w, Out out, int *status) {
   extern __shared__ __align__(1024) unsigned char sm[];
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tbase;
@@ -246,12 +302,14 @@ __global__ void __launch_bounds__(128, 1)
   uint32_t phase = 0;
   bool ok = true;
   const long long ntiles = (S + 127) / 128;
+  uint4 lo, hi;  // the next tile's sample, loaded a tile ahead
+  load_sample(X, S, blockIdx.x * 128ll + tid, lo, hi);
   for (long long t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
     const long long sample = t * 128 + tid;
-    uint4 lo, hi;
-    load_sample(X, S, sample, lo, hi);
     *reinterpret_cast<uint4 *>(sm + FwdSmem::X + umma::kmajor_offset(tid, 0, kF)) = lo;
     *reinterpret_cast<uint4 *>(sm + FwdSmem::X + umma::kmajor_offset(tid, 8, kF)) = hi;
+    load_sample(X, S, sample + gridDim.x * 128ll, lo, hi);
+    out.begin(sample, sample < S);
     smem_to_tc();
     if (tid == 0) {
       mma_tiles(D1, aX, aW1, kF, kH, false);
@@ -268,19 +326,26 @@ __global__ void __launch_bounds__(128, 1)
       mma_tiles(D2, aH1, aW2, kH, kH, false);
       umma::mma_commit(&mbar);
     }
+    out.load(sample < S);
     if (!(ok = wait_all(&mbar, phase))) break;
-    float acc = 0.f;
+    f32x2 acc = pack2(b3, 0.f);
+#pragma unroll 1
     for (int c = 0; c < kH; c += 16) {
       float v[16];
       umma::tmem_ld16(D2 + lane + c, v);
-      float b[16], hw[16];
-      for (int i = 0; i < 4; i++) {
-        reinterpret_cast<float4 *>(b)[i] = reinterpret_cast<const float4 *>(sb2 + c)[i];
-        reinterpret_cast<float4 *>(hw)[i] = reinterpret_cast<const float4 *>(shw3 + c)[i];
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(sb2 + c + i);
+        const ulonglong2 hw = *reinterpret_cast<const ulonglong2 *>(shw3 + c + i);
+        acc = gelu_out2(add2(pack2(v[i], v[i + 1]), b.x), hw.x, acc);
+        acc = gelu_out2(add2(pack2(v[i + 2], v[i + 3]), b.y), hw.y, acc);
       }
-      for (int i = 0; i < 16; i++) acc = gelu_out(v[i] + b[i], hw[i], acc);
     }
-    if (sample < S) y[sample] = acc + b3;
+    if (sample < S) {
+      float y0, y1;
+      unpack2(acc, y0, y1);
+      out.store(sample, y0 + y1);
+    }
     umma::tc_fence_before();
     __syncthreads();
     umma::tc_fence_after();
@@ -299,11 +364,9 @@ __global__ void __launch_bounds__(128, 1)
 
 // GELU and its derivative from one hardware tanh
 __device__ __forceinline__ void gelu_both(float z, float &g, float &dg) {
-  const float z2 = z * z;
-  const float t = tanh_fast(kGeluC * (z + kGeluA * z2 * z));
-  const float hz = 0.5f * z, ht = 0.5f * (1.0f + t);
-  g = z * ht;
-  dg = ht + hz * (1.0f - t * t) * kGeluC * (1.0f + 3.0f * kGeluA * z2);
+  const float t = tanh_fast(kGeluC * (z + kGeluA * z * z * z));
+  g = 0.5f * z * (1.0f + t);
+  dg = 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * kGeluC * (1.0f + 3.0f * kGeluA * z * z);
 }
 
 // Sums of 16 columns over the 32 rows (lanes) of a warp: each exchange halves the
@@ -550,11 +613,13 @@ static size_t fwd_smem() { return FwdSmem::END; }
 static size_t train_smem() { return TrainSmem::END; }
 
 // y[S] = MLP(X[S][16]) on the device (X BF16, 16-byte aligned rows)
-int mlp_forward_dev(const MlpState &s, const __nv_bfloat16 *X, long long S, float *y, cudaStream_t st) {
+// (out: StoreY, or AddFlux to add it to the edge fluxes)
+template <typename Out>
+static int mlp_forward_dev(const MlpState &s, const __nv_bfloat16 *X, long long S, const Out &out, cudaStream_t st) {
   static bool attr = false;
   static int per_sm = 1;
   if (!attr) {
-    if (cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem()) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_mlp_fwd<Out>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem()) != cudaSuccess)
       return -1;
     // A CTA's tile loop is grid-strided, so the grid is exactly the CTAs that
     // are resident together (a CTA started after another one's exit would run
@@ -562,12 +627,12 @@ int mlp_forward_dev(const MlpState &s, const __nv_bfloat16 *X, long long S, floa
     // threads hold, at most 512 / kFwdTmemCols for TMEM.  (Counted here from
     // the kernel's attributes: the runtime's occupancy query answered one CTA
     // per SM for this kernel, which the shared memory does not require.)
-    if (cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributePreferredSharedMemoryCarveout,
+    if (cudaFuncSetAttribute(k_mlp_fwd<Out>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
       return -1;
     cudaFuncAttributes fa{};
     int dev = 0, smem_sm = 0, resv = 0, regs_sm = 0, thr_sm = 0;
-    if (cudaFuncGetAttributes(&fa, k_mlp_fwd) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+    if (cudaFuncGetAttributes(&fa, k_mlp_fwd<Out>) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&resv, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev) != cudaSuccess ||
@@ -583,7 +648,7 @@ int mlp_forward_dev(const MlpState &s, const __nv_bfloat16 *X, long long S, floa
   if (S <= 0) return 0;
   const long long tiles = (S + 127) / 128;
   const int grid = (int)std::min<long long>(tiles, (long long)s.sms * per_sm);
-  k_mlp_fwd<<<grid, 128, fwd_smem(), st>>>(X, S, mlp_view(s), y, s.status);
+  k_mlp_fwd<Out><<<grid, 128, fwd_smem(), st>>>(X, S, mlp_view(s), out, s.status);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -621,7 +686,8 @@ struct LearnedState {
   bool on = false;
   long long ncells = 0;  // edge cells of the dense edge schedule
   __nv_bfloat16 *feat[kBatchMax] = {};
-  float *fscale[kBatchMax] = {}, *y[kBatchMax] = {};
+  float *fscale[kBatchMax] = {};
+  unsigned *cell = nullptr;  // slot x S + level of every edge cell
   float *dy = nullptr, *target = nullptr, *hp = nullptr, *hm = nullptr;
   double *red = nullptr;  // per-block partial sums
   double volume = 0.0;    // sum of areasvol * hnode_new over wet cells
@@ -629,19 +695,6 @@ struct LearnedState {
 };
 
 namespace {
-
-// tracer t of the batch's antidiffusive fluxes (NT tracers side by side)
-template <int NT>
-__global__ void __launch_bounds__(kThreads) k_learn_apply(DMeshT<float> m, float *adf, int t, const float *scale,
-                                                         const float *y) {
-  extern __shared__ int smem[];
-  int *s_off = smem, *s_item = smem + kMaxItemsPerBlock + 1;
-  const CellMap cm = map_cells(m.edge_sched, blockIdx.x, s_off, s_item);
-  for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
-    const int j = s_item[lc], e = cm.i0 + j, k = lc - (s_off[j] - cm.c0), cell = cm.c0 + lc;
-    il<NT>(adf, t, (cix)e * m.S + k) += scale[cell] * y[cell];
-  }
-}
 
 // dL/dy for L = sum_n V_n (T_n - target_n)^2 / sum V after an unlimited step:
 // an edge flux f enters T_n1 with +dt/V and T_n2 with -dt/V, f = base + scale y
@@ -828,8 +881,8 @@ void learned_release(EngineImpl &P) {
   for (int t = 0; t < kBatchMax; t++) {
     cudaFree(L.feat[t]);
     cudaFree(L.fscale[t]);
-    cudaFree(L.y[t]);
   }
+  cudaFree(L.cell);
   cudaFree(L.dy);
   cudaFree(L.target);
   cudaFree(L.hp);
@@ -841,15 +894,13 @@ void learned_release(EngineImpl &P) {
 
 void learned_correct_f32(EngineImpl &P, int nt, const FusedArgs<float, float> &a) {
   LearnedState &L = *P.learn;
-  for (int t = 0; t < nt; t++) {
-    if (mlp_forward_dev(L.mlp, a.feat[t], L.ncells, L.y[t], P.stream) != 0)
-      throw std::runtime_error("learned flux: MLP forward launch failed");
-    if (P.dm32.edge_sched.nblk > 0) {
-      auto *apply = nt == 4 ? k_learn_apply<4> : (nt == 2 ? k_learn_apply<2> : k_learn_apply<1>);
-      apply<<<P.dm32.edge_sched.nblk, kThreads, smem_edge(), P.stream>>>(P.dm32, a.adf_h, t, a.fscale[t], L.y[t]);
-    }
-    CK(cudaGetLastError());
-  }
+  auto forward = [&](int t) {
+    if (nt == 4) return mlp_forward_dev(L.mlp, a.feat[t], L.ncells, AddFlux<4>{a.adf_h, a.fscale[t], L.cell, t, 0u, 0.f, 0.f}, P.stream);
+    if (nt == 2) return mlp_forward_dev(L.mlp, a.feat[t], L.ncells, AddFlux<2>{a.adf_h, a.fscale[t], L.cell, t, 0u, 0.f, 0.f}, P.stream);
+    return mlp_forward_dev(L.mlp, a.feat[t], L.ncells, AddFlux<1>{a.adf_h, a.fscale[t], L.cell, t, 0u, 0.f, 0.f}, P.stream);
+  };
+  for (int t = 0; t < nt; t++)
+    if (forward(t) != 0) throw std::runtime_error("learned flux: MLP forward launch failed");
 }
 
 // feature / scale buffers of the batch slots, for the run_batch of engine.cu
@@ -858,7 +909,6 @@ void learned_slot_buffers(EngineImpl &P, int t, void **feat, void **scale) {
   if (!L.feat[t]) {
     L.feat[t] = dmalloc<__nv_bfloat16>((size_t)L.ncells * kF);
     L.fscale[t] = dmalloc<float>(L.ncells);
-    L.y[t] = dmalloc<float>(L.ncells);
   }
   *feat = L.feat[t];
   *scale = L.fscale[t];
@@ -883,6 +933,12 @@ void Engine::set_learned(const float *params, bool on) {
       for (int k = 0; k < M.nlev_node[n] - 1; k++)
         vol += M.areasvol[(size_t)n * M.nl + k] * M.hnode_new[(size_t)n * L1 + k];
     L.volume = vol;
+    std::vector<unsigned> cell;
+    cell.reserve(cells);
+    for (int s = 0; s < M.edge2D; s++)
+      for (int k = 0; k < M.edge_levels(P.slot_edge[s]); k++) cell.push_back((unsigned)s * (unsigned)P.S + (unsigned)k);
+    L.cell = dmalloc<unsigned>(cell.size());
+    CK(cudaMemcpy(L.cell, cell.data(), cell.size() * sizeof(unsigned), cudaMemcpyHostToDevice));
     L.dy = dmalloc<float>(L.ncells);
     L.target = dmalloc<float>((size_t)M.nod2D * P.S);
     CK(cudaMemset(L.target, 0, (size_t)M.nod2D * P.S * sizeof(float)));
@@ -996,7 +1052,7 @@ extern "C" int tracer_mlp_forward(const uint16_t *X, long long S, const float *p
       cudaMemcpy(s.p, params, kParams * 4, cudaMemcpyHostToDevice) == cudaSuccess &&
       cudaMemcpy(dX, X, (size_t)S * kF * 2, cudaMemcpyHostToDevice) == cudaSuccess) {
     mlp_sync_bf16(s, 0);
-    if (mlp_forward_dev(s, dX, S, dy, 0) == 0 && cudaDeviceSynchronize() == cudaSuccess &&
+    if (mlp_forward_dev(s, dX, S, StoreY{dy}, 0) == 0 && cudaDeviceSynchronize() == cudaSuccess &&
         cudaMemcpy(y, dy, (size_t)S * 4, cudaMemcpyDeviceToHost) == cudaSuccess)
       rc = mlp_status(s);
   }
