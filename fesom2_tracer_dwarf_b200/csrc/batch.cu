@@ -275,6 +275,7 @@ struct BatchImpl {
   int ntasks = 0, nwaves = 0;
   std::vector<void *> work;  // work arrays of every (member, wave slot)
   long long work_bytes = 0;
+  long long tile_bytes = 0;  // work arrays of the configured tile
   BatchKernel kernel = nullptr;
   int grid = 0;
   cudaGraph_t graph = nullptr;
@@ -284,6 +285,10 @@ struct BatchImpl {
   cudaGraph_t sep_graph = nullptr;
   cudaGraphExec_t sep_exec = nullptr;
   std::vector<cudaEvent_t> sep_events;
+  const void *sep_key = nullptr;  // the first tracer's buffer at capture
+  // path 2 holds the members' own work arrays (and the graph) from call to call
+  // and the batch's are released meanwhile; set_tile changes back
+  bool separate = false;
 
   // step path: 0 one cooperative launch per step, 1 one persistent launch
   // per phase and wave, 2 the members' own launches
@@ -330,6 +335,7 @@ struct BatchImpl {
     if (sep_graph) cudaGraphDestroy(sep_graph);
     sep_exec = nullptr;
     sep_graph = nullptr;
+    sep_key = nullptr;
     for (auto e : sep_events) cudaEventDestroy(e);
     sep_events.clear();
   }
@@ -492,9 +498,9 @@ void Batch::configure(const TracerScheme &sch, const std::vector<double> &dt, bo
 }
 
 BatchTile Batch::tile() const { return p_->tile; }
-long long Batch::work_bytes() const { return p_->work_bytes; }
+long long Batch::work_bytes() const { return p_->tile_bytes; }
 bool Batch::graph_captured() const {
-  if (p_->mode == 2) return p_->sep_exec != nullptr;
+  if (p_->mode == 2) return false;  // the persistent paths' graph
   return p_->mode == 1 ? p_->ph_exec != nullptr : p_->graph_exec != nullptr;
 }
 
@@ -512,6 +518,11 @@ void Batch::set_tile(const BatchTile &tile) {
   for (auto &m : B.members) m->synchronize();
   CK(cudaStreamSynchronize(B.stream));
   B.release();
+  if (B.separate) {
+    B.release_sep();
+    for (auto &m : B.members) m->release_work();
+    B.separate = false;
+  }
   B.tile = tile;
   B.kernel = pick_kernel(B.sch, tile.threads, tile.blocks_per_sm);
   phase_kernels(B.sch, B.phk);
@@ -559,6 +570,7 @@ void Batch::set_tile(const BatchTile &tile) {
       }
     }
   }
+  B.tile_bytes = B.work_bytes;
   refresh_vflux(B);
   make_tasks(B);
   std::vector<int> prefix((size_t)PH_COUNT * (B.ntasks + 1), 0);
@@ -763,6 +775,7 @@ void Batch::set_learned(const float *params, bool on) {
   BatchImpl &B = *p_;
   CK(cudaStreamSynchronize(B.stream));
   for (auto &m : B.members) m->set_learned(params, on);
+  B.release_sep();  // captured with the other sequence of launches
   B.learned = on;
   if (on) B.mode = 2;
 }
@@ -775,6 +788,7 @@ void Batch::step(int nsteps, bool use_graph) {
     step_separate(nsteps, use_graph);
     return;
   }
+  if (B.configured && B.separate) set_tile(B.tile);
   begin_steps(B);
   run_steps(B, nsteps, use_graph);
   CK(cudaGetLastError());
@@ -787,6 +801,7 @@ double Batch::time_steps(int nsteps, bool use_graph) {
   BatchImpl &B = *p_;
   if (B.learned && B.mode != 2) throw std::logic_error("batch: the learned flux runs on path 2 only");
   if (B.mode == 2) return time_separate(nsteps, use_graph);
+  if (B.configured && B.separate) set_tile(B.tile);
   begin_steps(B);
   // capture (and the device table upload) outside the timed region
   if (use_graph && B.mode == 1 && nsteps >= 2) capture_phases(B);
@@ -812,18 +827,25 @@ double Batch::time_steps(int nsteps, bool use_graph) {
 }
 
 // The separate path uses the member engines' own work arrays; the batch's are
-// released meanwhile (device memory) and rebuilt with the task table after.
-// Members launch on their own streams; with use_graph the launches of two
-// steps (so that every engine's buffer ping-pong returns to where it started)
-// are captured once as a graph forked from and joined into the batch stream.
+// released meanwhile (device memory) and rebuilt with the task table when a
+// persistent path runs next (set_tile).  Both the arrays and the graph stay from
+// call to call: allocating, capturing and rebuilding the batch's task table on
+// each call cost 70-90 ms (3 members of up to 233x233x38, 8 tracers, against
+// 24 ms for 30 steps).  Members launch on their own streams; with use_graph the
+// launches of two steps (so that every engine's buffer ping-pong returns to where
+// it started) are captured as a graph forked from and joined into the batch
+// stream, valid while the buffers are those of its capture or their swap.
 namespace {
 void separate_steps_direct(BatchImpl &B, int nsteps) {
   for (int s = 0; s < nsteps; s++)
     for (size_t m = 0; m < B.members.size(); m++) B.members[m]->step(B.dt[m], B.refresh_ab);
 }
 
+const void *first_buffer(BatchImpl &B) { return B.members.empty() ? nullptr : B.members[0]->impl()->tr[0].T; }
+
 void capture_separate(BatchImpl &B) {
-  if (B.sep_exec) return;
+  if (B.sep_exec && B.sep_key == first_buffer(B)) return;
+  B.release_sep();
   const size_t M = B.members.size();
   B.sep_events.resize(M + 1);
   for (auto &e : B.sep_events) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -839,6 +861,30 @@ void capture_separate(BatchImpl &B) {
   CK(cudaStreamEndCapture(B.stream, &g));
   B.sep_graph = g;
   CK(cudaGraphInstantiate(&B.sep_exec, g, 0));
+  B.sep_key = first_buffer(B);
+}
+
+// Changes to the separate path, and takes one step of `nsteps` directly where
+// that must come first: it allocates the work arrays and fills the edge volume
+// fluxes, which no capture or replay may do, or swaps the buffers back to those
+// the graph was captured with.  Returns the steps left.
+int begin_separate(BatchImpl &B, int nsteps, bool use_graph, bool always) {
+  if (!B.configured) throw std::runtime_error("configure the batch first");
+  CK(cudaStreamSynchronize(B.stream));
+  for (auto &m : B.members) m->synchronize();
+  if (!B.separate) {
+    B.release();
+    B.separate = true;
+  }
+  bool direct = always || (B.sep_exec && B.sep_key != first_buffer(B));
+  for (auto &m : B.members) direct = direct || !m->impl()->vflux_valid || m->impl()->slots < kNT;
+  if (nsteps > 0 && (direct || !use_graph)) {
+    separate_steps_direct(B, 1);
+    nsteps--;
+    CK(cudaDeviceSynchronize());
+  }
+  if (use_graph && nsteps >= 2) capture_separate(B);
+  return nsteps;
 }
 
 // nsteps separate steps (graph-replayed in pairs when use_graph)
@@ -857,36 +903,18 @@ void separate_steps(BatchImpl &B, int nsteps, bool use_graph) {
 
 void Batch::step_separate(int nsteps, bool use_graph) {
   BatchImpl &B = *p_;
-  CK(cudaStreamSynchronize(B.stream));
-  B.release();
-  // one direct step allocates the engines' work arrays and kernel attributes
-  // before any capture
-  const int first = nsteps > 0 ? 1 : 0;
-  separate_steps_direct(B, first);
+  const int left = begin_separate(B, nsteps, use_graph, false);
+  separate_steps(B, left, use_graph);
   CK(cudaDeviceSynchronize());
-  if (use_graph) capture_separate(B);
-  separate_steps(B, nsteps - first, use_graph);
-  CK(cudaDeviceSynchronize());
-  B.release_sep();
-  for (auto &m : B.members) m->release_work();
-  set_tile(B.tile);
 }
 
 double Batch::time_separate(int nsteps, bool use_graph) {
   BatchImpl &B = *p_;
-  CK(cudaStreamSynchronize(B.stream));
-  B.release();
-  // one untimed step allocates the engines' work arrays
-  separate_steps_direct(B, 1);
-  CK(cudaDeviceSynchronize());
-  if (use_graph) capture_separate(B);
+  begin_separate(B, nsteps + 1, use_graph, true);  // one untimed step
   const auto t0 = std::chrono::steady_clock::now();
   separate_steps(B, nsteps, use_graph);
   CK(cudaDeviceSynchronize());
   const auto t1 = std::chrono::steady_clock::now();
-  B.release_sep();
-  for (auto &m : B.members) m->release_work();
-  set_tile(B.tile);
   return std::chrono::duration<double, std::milli>(t1 - t0).count();
 }
 
