@@ -33,6 +33,14 @@ FESOM_VARIANT_BEGIN
 constexpr int NTMAX = 4;
 constexpr int kThreads = 256;
 constexpr int kEdgeThreads = 128, kColThreads = 128;
+
+// Programmatic dependent launch: each step kernel lets the next one start as soon
+// as its own blocks run, and waits, after reading its schedule and tables, for
+// the kernel before it to be complete.  Both are no-ops in a kernel launched without
+// the attribute.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 // Resident 128-thread blocks per SM that each step kernel's register budget is
 // cut for.  The kernels are bound by the latency of their gathers; a lane issues the
 // loads of its whole stencil before it uses the first, so what hides the latency
@@ -52,6 +60,12 @@ constexpr int kEdgeThreads = 128, kColThreads = 128;
 #ifndef FESOM_MINB_COL3
 #define FESOM_MINB_COL3 4
 #endif
+#ifndef FESOM_MINB_GRAD
+#define FESOM_MINB_GRAD 7
+#endif
+#ifndef FESOM_MINB32_GRAD
+#define FESOM_MINB32_GRAD 9
+#endif
 #ifndef FESOM_MINB32_EDGE
 #define FESOM_MINB32_EDGE 5
 #endif
@@ -66,11 +80,11 @@ constexpr int kEdgeThreads = 128, kColThreads = 128;
 #endif
 template <typename R, int NT>
 struct StepBlocks {
-  static constexpr int edge = FESOM_MINB_EDGE, col1 = FESOM_MINB_COL1, col2 = FESOM_MINB_COL2, col3 = FESOM_MINB_COL3;
+  static constexpr int grad = FESOM_MINB_GRAD, edge = FESOM_MINB_EDGE, col1 = FESOM_MINB_COL1, col2 = FESOM_MINB_COL2, col3 = FESOM_MINB_COL3;
 };
 template <int NT>
 struct StepBlocks<float, NT> {  // four tracers a lane: 128 registers
-  static constexpr int edge = NT == 4 ? 4 : FESOM_MINB32_EDGE, col1 = NT == 4 ? 4 : FESOM_MINB32_COL1,
+  static constexpr int grad = FESOM_MINB32_GRAD, edge = NT == 4 ? 4 : FESOM_MINB32_EDGE, col1 = NT == 4 ? 4 : FESOM_MINB32_COL1,
                        col2 = NT == 4 ? 4 : FESOM_MINB32_COL2, col3 = NT == 4 ? 4 : FESOM_MINB32_COL3;
 };
 // Tracers of a batch of NT that a lane advances together; it takes the groups one
@@ -81,9 +95,9 @@ struct StepBlocks<float, NT> {  // four tracers a lane: 128 registers
 template <typename R, int NT>
 struct LaneTracers {
   static constexpr int cap(int g) { return g < NT ? g : NT; }
-  static constexpr int col1 = cap(sizeof(R) == 8 ? 2 : 4), col2 = cap(sizeof(R) == 8 ? 1 : 4), col3 = col1;
+  static constexpr int col1 = cap(sizeof(R) == 8 ? 2 : 4), col2 = cap(sizeof(R) == 8 ? 1 : 4), col3 = col1,
+                       grad = cap(sizeof(R) == 8 ? 2 : 4);
 };
-constexpr int kGradBlocks = 5;  // k_grad: 256-thread blocks
 constexpr int kCellsPerBlock = 512;      // schedule cap: wet cells per block (two per thread)
 constexpr int kMaxCellsPerBlock = 576;   // upper bound (target + deepest column)
 constexpr int kMaxItemsPerBlock = 512;
@@ -198,66 +212,152 @@ __device__ __forceinline__ void st_pair(float *p, float x, float y) {
   *reinterpret_cast<float2 *>(p) = make_float2(x, y);
 }
 
+// a / b given y = RN(1 / b), correctly rounded (see div_rcp), straight-line:
+// numerators outside [2^-900, 2^900] other than zero set `bad` and the caller
+// divides again.  The sign of a zero result is not kept (no output of the step
+// depends on the sign of a zero quotient).
+__device__ __forceinline__ double div_fast(double a, double b, double y, bool &bad) {
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  const unsigned u = 2u * (unsigned)__double2hiint(a);
+  bad |= (u - 0x0f600000u > 0xf0800000u - 0x0f600000u) && u != 0u;
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+__device__ __forceinline__ float div_fast(float a, float b, float y, bool &bad) {
+  float q = a * y;
+  q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+  const unsigned u = 2u * __float_as_uint(a);
+  bad |= (u - 0x1b000000u > 0xe3000000u - 0x1b000000u) && u != 0u;
+  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
+// RN(1 / b), straight-line: the hardware's approximate reciprocal refined by
+// Newton steps y += y (1 - b y), the last of which rounds correctly unless b's
+// significand is all ones (Markstein).  That significand, and magnitudes outside
+// [2^-500, 2^500] (FP32: [2^-60, 2^60]), set `bad`.
+__device__ __forceinline__ double rcp_newton(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));  // about 2^-20
+  y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+  return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+}
+__device__ __forceinline__ double rcp_exact(double b, bool &bad) {
+  const double y = rcp_newton(b);
+  const unsigned u = 2u * (unsigned)__double2hiint(b);
+  bad |= u - 0x41600000u > 0xbe600000u - 0x41600000u || ((unsigned)__double2hiint(b) | 0xfff00000u) == 0xffffffffu;
+  return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+}
+__device__ __forceinline__ float rcp_exact(float b, bool &bad) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));  // within a unit in the last place
+  const unsigned u = 2u * __float_as_uint(b);
+  bad |= u - 0x43000000u > 0xbb000000u - 0x43000000u || (__float_as_uint(b) | 0xff800000u) == 0xffffffffu;
+  return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
+}
+// a / b for any divisor: the limiter ratios (numerators below 2^-500 other than
+// zero set `bad` too, so that no quotient underflows)
+__device__ __forceinline__ double div_any(double a, double b, bool &bad) {
+  const unsigned u = 2u * (unsigned)__double2hiint(a);
+  bad |= u < 0x41600000u && u != 0u;
+  return div_fast(a, b, rcp_exact(b, bad), bad);
+}
+
+// One pair of node levels: the ring's elements one after the other (a level an
+// element does not reach adds nothing).  The pairs are the few bottom levels of
+// each column, so every load of a warp touches as many lines as it has nodes:
+// the kernel is bound by those lines, and more resident warps hide more of them
+// than more loads per warp (400x400x64: one element at a time in 56-72 registers
+// FP64 0.088, FP32 0.059 ms; two in 78-120 0.095, 0.062; three 0.098, 0.062; the cell-mapped
+// kernel before 0.091, 0.071).
 template <typename R, typename TS, int NT>
-__device__ __forceinline__ void grad_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk, int *smem) {
-  int *s_off = smem, *s_item = smem + kMaxItemsPerBlock + 1;
-  const CellMap cm = map_cells(m.grad_sched, blk, s_off, s_item);
-  for (int lc = threadIdx.x; lc < cm.nc; lc += blockDim.x) {
-    const int j = s_item[lc], n = cm.i0 + j, k = m.grad_lev0[n] + lc - (s_off[j] - cm.c0);
-    R gx[NTMAX], gy[NTMAX];
-    ring_mean_n(m, a.TAB, a.off, NT, n, k, gx, gy);
-    const cix o = (cix)n * m.S + k;
-    for (int t = 0; t < NT; t++) st_pair(a.gradn[t] + 2 * o, gx[t], gy[t]);
+__device__ __forceinline__ void grad_pair(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int n, int k) {
+  const int p0 = m.ring_ptr[n], p1 = m.ring_ptr[n + 1], nln = m.nlev_node[n] - 1;
+  R vol[2] = {R(0), R(0)}, sx[NT][2], sy[NT][2];
+#pragma unroll
+  for (int t = 0; t < NT; t++) sx[t][0] = sx[t][1] = sy[t][0] = sy[t][1] = R(0);
+#pragma unroll 1
+  for (int p = p0; p < p1; p++) {
+    const int el = m.ring_elem[p];
+    const int4 r = m.elem_idx[el];
+    R g[8], v[NT][3][2];
+    ldv8(m.elem_geo + 8 * (size_t)el, g);
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      ld_pair_T(a.TAB[t], (cix)r.x + k, a.off[t], v[t][0]);
+      ld_pair_T(a.TAB[t], (cix)r.y + k, a.off[t], v[t][1]);
+      ld_pair_T(a.TAB[t], (cix)r.z + k, a.off[t], v[t][2]);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const bool wet = k + q < r.w;
+      vol[q] = wet ? vol[q] + g[6] : vol[q];
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        const R gx = (g[0] * v[t][0][q] + g[1] * v[t][1][q]) + g[2] * v[t][2][q];
+        const R gy = (g[3] * v[t][0][q] + g[4] * v[t][1][q]) + g[5] * v[t][2][q];
+        sx[t][q] = wet ? sx[t][q] + gx * g[6] : sx[t][q];
+        sy[t][q] = wet ? sy[t][q] + gy * g[6] : sy[t][q];
+      }
+    }
+  }
+  const cix o = (cix)n * m.S + k;
+  if (k + 1 >= nln) vol[1] = R(1);  // dry
+  bool bad = false;
+  const R y[2] = {rcp_exact(vol[0], bad), rcp_exact(vol[1], bad)};
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    R out[4];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      out[2 * q] = div_fast(sx[t][q], vol[q], y[q], bad);
+      out[2 * q + 1] = div_fast(sy[t][q], vol[q], y[q], bad);
+    }
+    if (bad)
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        out[2 * q] = sx[t][q] / vol[q];
+        out[2 * q + 1] = sy[t][q] / vol[q];
+      }
+    stv4(a.gradn[t] + 2 * (size_t)o, out);
   }
 }
 
 template <typename R, typename TS, int NT>
-__global__ void __launch_bounds__(kThreads, kGradBlocks) k_grad(DMeshT<R> m, FusedArgs<R, TS> a) {
-  extern __shared__ int smem[];
-  grad_block<R, TS, NT>(m, a, blockIdx.x, smem);
+__device__ __forceinline__ void grad_block(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int blk) {
+  const int warp = blk * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
+  if (warp >= m.grad_pairs.nwarps) return;
+  const PairLane l = pair_lane(m.grad_pairs, warp);
+  if (l.on) prefetch(m.ring_elem + m.ring_ptr[l.item]);
+  pdl_wait();
+  if (!l.on) return;
+  constexpr int G = LaneTracers<R, NT>::grad;
+  if constexpr (G == NT) {
+    grad_pair<R, TS, NT>(m, a, l.item, l.k);
+  } else {
+    FusedArgs<R, TS> b;  // the pointers grad_pair reads, of one group of tracers at a time
+#pragma unroll
+    for (int t0 = 0; t0 < NT; t0 += G) {
+#pragma unroll
+      for (int t = 0; t < G; t++) {
+        b.TAB[t] = a.TAB[t0 + t];
+        b.off[t] = a.off[t0 + t];
+        b.gradn[t] = a.gradn[t0 + t];
+      }
+      grad_pair<R, TS, G>(m, b, l.item, l.k);
+    }
+  }
+}
+
+template <typename R, typename TS, int NT>
+__global__ void __launch_bounds__(kColThreads, StepBlocks<R, NT>::grad)
+    k_grad(const __grid_constant__ DMeshT<R> m, const __grid_constant__ FusedArgs<R, TS> a) {
+  pdl_launch();
+  grad_block<R, TS, NT>(m, a, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
 // k_edge
 // ---------------------------------------------------------------------------
-template <typename R, typename TS>
-__device__ __forceinline__ void trxy_n(const DMeshT<R> &m, const TS *const *tab, const R *off, int NT, int elem, int k,
-                                       R *gx, R *gy) {
-  const int *en = m.elem_nodes + 3 * elem;
-  const int a = en[0], b = en[1], c = en[2];
-  const R *gs = m.grad_sca + 6 * elem;
-  const R g0 = gs[0], g1 = gs[1], g2 = gs[2], g3 = gs[3], g4 = gs[4], g5 = gs[5];
-  for (int t = 0; t < NT; t++) {
-    const R t1 = ldT(tab[t], (cix)a * m.S + k, off[t]), t2 = ldT(tab[t], (cix)b * m.S + k, off[t]), t3 = ldT(tab[t], (cix)c * m.S + k, off[t]);
-    gx[t] = (g0 * t1 + g1 * t2) + g2 * t3;
-    gy[t] = (g3 * t1 + g4 * t2) + g5 * t3;
-  }
-}
-
-template <typename R, typename TS>
-__device__ __forceinline__ void ring_mean_n(const DMeshT<R> &m, const TS *const *tab, const R *off, int NT, int n, int k,
-                                            R *gx, R *gy) {
-  R tvol = R(0), tx[NTMAX], ty[NTMAX];
-  for (int t = 0; t < NT; t++) { tx[t] = R(0); ty[t] = R(0); }
-  const int nz = k + 1;
-  for (int p = m.ring_ptr[n]; p < m.ring_ptr[n + 1]; p++) {
-    const int el = m.ring_elem[p];
-    if (m.nlev_elem[el] - 1 < nz) continue;
-    R ax[NTMAX], ay[NTMAX];
-    trxy_n(m, tab, off, NT, el, k, ax, ay);
-    const R a = m.elem_area[el];
-    tvol = tvol + a;
-    for (int t = 0; t < NT; t++) {
-      tx[t] = tx[t] + ax[t] * a;
-      ty[t] = ty[t] + ay[t] * a;
-    }
-  }
-  for (int t = 0; t < NT; t++) {
-    gx[t] = tx[t] / tvol;
-    gy[t] = ty[t] / tvol;
-  }
-}
-
 // x / 6 and x / 3, correctly rounded.  The reciprocals of 3 and 6 round with a
 // relative error of 2^-54 (FP32: 2^-25), so q = RN(x y) is already a faithful
 // quotient and one Markstein correction rounds it (div_rcp needs two).  The
@@ -284,25 +384,6 @@ template <typename R>
 __device__ __forceinline__ R div6(R x, bool &bad) { return div_3k<6>(x, bad); }
 template <typename R>
 __device__ __forceinline__ R div3(R x, bool &bad) { return div_3k<3>(x, bad); }
-
-// a / b given y = RN(1 / b), correctly rounded (see div_rcp), straight-line:
-// numerators outside [2^-900, 2^900] other than zero set `bad` and the caller
-// divides again.  The sign of a zero result is not kept (no output of the step
-// depends on the sign of a zero quotient).
-__device__ __forceinline__ double div_fast(double a, double b, double y, bool &bad) {
-  double q = a * y;
-  q = __fma_rn(__fma_rn(-b, q, a), y, q);
-  const unsigned u = 2u * (unsigned)__double2hiint(a);
-  bad |= (u - 0x0f600000u > 0xf0800000u - 0x0f600000u) && u != 0u;
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-__device__ __forceinline__ float div_fast(float a, float b, float y, bool &bad) {
-  float q = a * y;
-  q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-  const unsigned u = 2u * __float_as_uint(a);
-  bad |= (u - 0x1b000000u > 0xe3000000u - 0x1b000000u) && u != 0u;
-  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-}
 
 // learned flux: 16 features of one MUSCL edge level in the flow's frame, in
 // units of the local variation sig, and the scale of the network's output
@@ -554,6 +635,7 @@ __device__ __forceinline__ void edge_block(const DMeshT<R> &m, const FusedArgs<R
   PairLane nxt = pair_lane(s, warp);
   EdgeIdx idx = edge_idx(m, nxt.item);
   PairLane nn = warp + 1 < end ? pair_lane(s, warp + 1) : nxt;
+  pdl_wait();
   do {
     const PairLane c = nxt;
     const EdgeIdx x = idx;
@@ -572,6 +654,7 @@ __device__ __forceinline__ void edge_block(const DMeshT<R> &m, const FusedArgs<R
 template <typename R, typename TS, int NT, int HOR, int LIM, bool LOADV>
 __global__ void __launch_bounds__(kEdgeThreads, StepBlocks<R, NT>::edge)
     k_edge(const __grid_constant__ DMeshT<R> m, const __grid_constant__ FusedArgs<R, TS> a, int per) {
+  pdl_launch();
   edge_block<R, TS, NT, HOR, LIM, LOADV>(m, a, blockIdx.x, per);
 }
 
@@ -977,6 +1060,9 @@ __device__ __forceinline__ void col_warps(const DMeshT<R> &m, int blk, int per, 
   const int end = min(warp + per, s.nwarps);
   if (warp >= end) return;
   PairLane nxt = pair_lane(s, warp);
+  prefetch(m.nrec + nxt.item);
+  prefetch(m.ne6 + 3 * (size_t)nxt.item);
+  pdl_wait();
   do {
     const PairLane c = nxt;
     if (++warp < end) nxt = pair_lane(s, warp);
@@ -995,34 +1081,13 @@ __device__ __forceinline__ void col1_block(const DMeshT<R> &m, const FusedArgs<R
 template <typename R, typename TS, int NT, int VER, int LIM, bool UNI>
 __global__ void __launch_bounds__(kColThreads, StepBlocks<R, NT>::col1)
     k_col1(const __grid_constant__ DMeshT<R> m, const __grid_constant__ FusedArgs<R, TS> a, int per) {
+  pdl_launch();
   col1_block<R, TS, NT, VER, LIM, UNI>(m, a, blockIdx.x, per);
 }
 
 // ---------------------------------------------------------------------------
 // k_col2: bounds, in/out sums, ratios (lib/oce_adv_tra_fct.F90:105-374)
 // ---------------------------------------------------------------------------
-// Quotients of the limiter ratios, straight-line.  FP64: the hardware's
-// approximate reciprocal (about 2^-20) refined by Newton steps y += y (1 - b y), the
-// last of which rounds 1 / b correctly unless b's significand is all ones, then
-// the quotient by Markstein's correction (see div_rcp).  Operands outside [2^-500,
-// 2^500] (other than a zero numerator) and that significand set `bad`, and the
-// caller divides again.
-__device__ __forceinline__ double rcp_newton(double b) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
-  return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
-}
-__device__ __forceinline__ double div_any(double a, double b, bool &bad) {
-  double y = rcp_newton(b);
-  y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
-  double q = a * y;
-  q = __fma_rn(__fma_rn(-b, q, a), y, q);
-  const unsigned ua = 2u * (unsigned)__double2hiint(a), ub = 2u * (unsigned)__double2hiint(b);
-  bad |= ub - 0x41600000u > 0xbe600000u - 0x41600000u || (ua - 0x41600000u > 0xbe600000u - 0x41600000u && ua != 0u) ||
-         ((unsigned)__double2hiint(b) | 0xfff00000u) == 0xffffffffu;
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
 // Reciprocal for FP64 quotients that are rounded to FP32 afterwards: one Newton
 // step (error about 2^-40).
 __device__ __forceinline__ double rcp_newton1(double b) {
@@ -1221,6 +1286,7 @@ __device__ __forceinline__ void col2_block(const DMeshT<R> &m, const FusedArgs<R
 template <typename R, typename TS, int NT>
 __global__ void __launch_bounds__(kColThreads, StepBlocks<R, NT>::col2)
     k_col2(const __grid_constant__ DMeshT<R> m, const __grid_constant__ FusedArgs<R, TS> a, int per) {
+  pdl_launch();
   col2_block<R, TS, NT>(m, a, blockIdx.x, per);
 }
 
@@ -1378,6 +1444,7 @@ __device__ __forceinline__ void col3_block(const DMeshT<R> &m, const FusedArgs<R
 template <typename R, typename TS, int NT, int LIM>
 __global__ void __launch_bounds__(kColThreads, StepBlocks<R, NT>::col3)
     k_col3(const __grid_constant__ DMeshT<R> m, const __grid_constant__ FusedArgs<R, TS> a, int per) {
+  pdl_launch();
   col3_block<R, TS, NT, LIM>(m, a, blockIdx.x, per);
 }
 

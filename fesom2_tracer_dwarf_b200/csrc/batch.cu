@@ -63,7 +63,7 @@ enum { PH_GRAD = 0, PH_EDGE, PH_COL1, PH_COL2, PH_COL3, PH_COUNT };
 
 constexpr size_t kTaskSmem = (sizeof(BatchTask) + 15) / 16 * 16;
 size_t batch_smem() {
-  return kTaskSmem + smem_edge();
+  return kTaskSmem;
 }
 
 // prefix: PH_COUNT rows of (ntasks + 1) running totals of each task's blocks;
@@ -75,7 +75,6 @@ __global__ void __launch_bounds__(256, MINB)
                  long long spin_limit, int refresh_ab) {
   extern __shared__ __align__(16) int smem[];
   BatchTask &st = *reinterpret_cast<BatchTask *>(smem);
-  int *work = smem + kTaskSmem / sizeof(int);
   const unsigned nb = gridDim.x;
   for (int w = 0; w < nwaves; w++) {
     const int t0 = wave_first[w], t1 = wave_first[w + 1];
@@ -97,7 +96,7 @@ __global__ void __launch_bounds__(256, MINB)
         }
         const int vblk = g - pre[task];
         switch (ph) {
-          case PH_GRAD: grad_block<float, float, kNT>(st.m, st.a, vblk, work); break;
+          case PH_GRAD: grad_block<float, float, kNT>(st.m, st.a, vblk); break;
           case PH_EDGE: edge_block<float, float, kNT, HOR, LIM, true>(st.m, st.a, vblk, kEdgeRun); break;
           case PH_COL1: col1_block<float, float, kNT, VER, LIM, true>(st.m, st.a, vblk, kColRun); break;
           case PH_COL2: col2_block<float, float, kNT>(st.m, st.a, vblk, kColRun); break;
@@ -196,16 +195,13 @@ __global__ void __launch_bounds__(kThreads, PhaseBudget<PH>::v) k_batch_phase(co
     if (g != (int)blockIdx.x) __syncthreads();  // the previous item is done with shared memory
     const int vblk = g - p.prefix[task];
     const BatchTask &st = p.t[task];
-    if (PH == PH_GRAD) grad_block<float, float, kNT>(st.m, st.a, vblk, smem);
+    if (PH == PH_GRAD) grad_block<float, float, kNT>(st.m, st.a, vblk);
     else if (PH == PH_EDGE) edge_block<float, float, kNT, HOR, LIM, true>(st.m, st.a, vblk, kEdgeRun);
     else if (PH == PH_COL1) col1_block<float, float, kNT, VER, LIM, true>(st.m, st.a, vblk, kColRun);
     else if (PH == PH_COL2) col2_block<float, float, kNT>(st.m, st.a, vblk, kColRun);
     else col3_block<float, float, kNT, LIM>(st.m, st.a, vblk, kColRun);
   }
 }
-
-// dynamic shared memory of each phase
-size_t phase_smem(int ph) { return ph == PH_GRAD ? smem_edge() : 0; }
 
 struct PhaseKernel {
   const void *fn = nullptr;
@@ -398,7 +394,7 @@ void refresh_vflux(BatchImpl &B) {
 // the batch's work-array slots.
 int phase_blocks(const BatchImpl &B, const DMeshT<float> &m, int ph, int threads) {
   switch (ph) {
-    case PH_GRAD: return B.sch.hor == HOR_UPW1 ? 0 : m.grad_sched.nblk;
+    case PH_GRAD: return B.sch.hor == HOR_UPW1 ? 0 : pair_blocks(m.grad_pairs, threads, 1);
     case PH_EDGE: return pair_blocks(m.edge_pairs, threads, kEdgeRun);
     case PH_COL2: return B.sch.lim == LIM_FCT ? pair_blocks(m.node_pairs, threads, kColRun) : 0;
     default: return pair_blocks(m.node_pairs, threads, kColRun);
@@ -590,10 +586,8 @@ void Batch::set_tile(const BatchTile &tile) {
   for (int ph = 0; ph < PH_COUNT; ph++) {
     B.phgrid[ph] = 0;
     if (!B.phk[ph].fn) continue;
-    const size_t sm = phase_smem(ph);
-    CK(cudaFuncSetAttribute(B.phk[ph].fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     int pocc = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pocc, B.phk[ph].fn, kThreads, sm));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pocc, B.phk[ph].fn, kThreads, 0));
     if (pocc < 1) throw std::runtime_error("batched phase kernel cannot be resident");
     B.phgrid[ph] = B.sms * pocc;
   }
@@ -693,7 +687,7 @@ void phase_step(BatchImpl &B) {
           }
           const int total = p.prefix[p.ntasks];
           if (total == 0) continue;
-          B.phk[ph].launch(p, std::min(total, B.phgrid[ph]), phase_smem(ph), st);
+          B.phk[ph].launch(p, std::min(total, B.phgrid[ph]), 0, st);
         }
       }
     }
@@ -852,7 +846,9 @@ void capture_separate(BatchImpl &B) {
   CK(cudaStreamBeginCapture(B.stream, cudaStreamCaptureModeRelaxed));
   CK(cudaEventRecord(B.sep_events[M], B.stream));
   for (size_t m = 0; m < M; m++) CK(cudaStreamWaitEvent((cudaStream_t)B.members[m]->stream(), B.sep_events[M], 0));
+  for (auto &m : B.members) m->impl()->pdl = false;  // forked streams: plain dependencies
   separate_steps_direct(B, 2);
+  for (auto &m : B.members) m->impl()->pdl = true;
   for (size_t m = 0; m < M; m++) {
     CK(cudaEventRecord(B.sep_events[m], (cudaStream_t)B.members[m]->stream()));
     CK(cudaStreamWaitEvent(B.stream, B.sep_events[m], 0));

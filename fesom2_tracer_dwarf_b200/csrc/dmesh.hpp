@@ -120,10 +120,11 @@ struct DMeshT {
   const R *ltab;            // level tables (advect_fused.cuh)
   DSched node_sched;        // items = nodes, levels = nlev_node - 1
   DSched edge_sched;        // items = edges, levels = edge levels
-  // node-levels whose MUSCL gradient is the ring mean for some incident edge
-  // (levels grad_lev0[n] .. nlev_node[n]-2 of node n)
-  const int *grad_lev0;
-  DSched grad_sched;        // items = nodes, levels = nlev_node - 1 - grad_lev0
+  // Element record of the ring means: {column bases (node x S) of its nodes,
+  // layers} and 8 reals, gradient_sca, area and one unused.
+  const int4 *elem_idx;
+  const R *elem_geo;
+  DPairs grad_pairs;        // node-level pairs some incident edge takes the ring mean of
 };
 
 }  // namespace fesom

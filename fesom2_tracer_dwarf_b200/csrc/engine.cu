@@ -73,7 +73,7 @@ R *upload_conv(EngineImpl &P, const std::vector<double> &h) {
   return P.upload(st);
 }
 
-// Work schedules (node, edge and gradient cells) for a cap on the wet
+// Work schedules (node and edge cells, of the learned flux) for a cap on the wet
 // cells per block; the arrays of a previous tiling are released.
 template <typename R>
 void build_schedules(EngineImpl &P, DMeshT<R> &d, int cells_per_block) {
@@ -81,9 +81,7 @@ void build_schedules(EngineImpl &P, DMeshT<R> &d, int cells_per_block) {
   const int N = M.nod2D, E = M.edge2D;
   const std::vector<int> &slot_edge = P.slot_edge;
   for (const void *q : {(const void *)d.node_sched.cell_off, (const void *)d.node_sched.blk,
-                        (const void *)d.edge_sched.cell_off, (const void *)d.edge_sched.blk,
-                        (const void *)d.grad_sched.cell_off, (const void *)d.grad_sched.blk,
-                        (const void *)d.grad_lev0})
+                        (const void *)d.edge_sched.cell_off, (const void *)d.edge_sched.blk})
     P.dfree(const_cast<void *>(q));
   std::vector<int> cnt(N), off, blk;
   for (int n = 0; n < N; n++) cnt[n] = M.nlev_node[n] - 1;
@@ -97,26 +95,6 @@ void build_schedules(EngineImpl &P, DMeshT<R> &d, int cells_per_block) {
   d.edge_sched.cell_off = P.upload(off);
   d.edge_sched.blk = P.upload(blk);
   d.edge_sched.nblk = (int)blk.size() - 1;
-
-  // ring-mean gradient levels: an edge uses the node ring means from level
-  // k = min(nlevels_nod2D_min(n1), nlevels_nod2D_min(n2)) - 1 down (from the
-  // surface when it lacks an up or down triangle)
-  std::vector<int> lev0(N);
-  for (int n = 0; n < N; n++) lev0[n] = std::max(0, M.nlev_node[n] - 1);
-  for (int e = 0; e < E; e++) {
-    const int n1 = M.edge_nodes[2 * e], n2 = M.edge_nodes[2 * e + 1];
-    const bool pair = M.up_dn_tri[2 * e] >= 0 && M.up_dn_tri[2 * e + 1] >= 0;
-    const int thr = pair ? std::max(0, std::min(M.nlev_node_min[n1], M.nlev_node_min[n2]) - 1) : 0;
-    lev0[n1] = std::min(lev0[n1], thr);
-    lev0[n2] = std::min(lev0[n2], thr);
-  }
-  d.grad_lev0 = P.upload(lev0);
-  for (int n = 0; n < N; n++) cnt[n] = std::max(0, M.nlev_node[n] - 1 - lev0[n]);
-  cnt.resize(N);
-  build_sched(cnt, off, blk, d.grad_sched.max_items, cells_per_block);
-  d.grad_sched.cell_off = P.upload(off);
-  d.grad_sched.blk = P.upload(blk);
-  d.grad_sched.nblk = (int)blk.size() - 1;
 }
 
 // Levels of an edge whose up and down triangles are both there and wet.
@@ -160,6 +138,50 @@ DPairs build_edge_pairs(EngineImpl &P) {
       }
     }
   return upload_pairs(P, item, lev);
+}
+
+// Pair schedule of the ring-mean gradients: an edge uses its nodes' ring means from
+// level edge_tri_levels down.
+DPairs build_grad_pairs(EngineImpl &P) {
+  const MeshHost &M = P.mesh;
+  const int N = M.nod2D;
+  std::vector<int> lev0(N), item;
+  std::vector<unsigned short> lev;
+  for (int n = 0; n < N; n++) lev0[n] = std::max(0, M.nlev_node[n] - 1);
+  for (int e = 0; e < M.edge2D; e++) {
+    const int thr = edge_tri_levels(M, e);
+    for (int q = 0; q < 2; q++) {
+      int &l = lev0[M.edge_nodes[2 * (size_t)e + q]];
+      l = std::min(l, thr);
+    }
+  }
+  for (int n = 0; n < N; n++)
+    for (int k = lev0[n] / 2 * 2; lev0[n] < M.nlev_node[n] - 1 && k < M.nlev_node[n] - 1; k += 2) {
+      item.push_back(n);
+      lev.push_back((unsigned short)k);
+    }
+  while (item.size() % 32) {
+    item.push_back(item.back());
+    lev.push_back((unsigned short)kPairNone);
+  }
+  return upload_pairs(P, item, lev);
+}
+
+// Element records of the ring means (DMeshT::elem_idx, elem_geo).
+template <typename R>
+void build_elem_records(EngineImpl &P, DMeshT<R> &d) {
+  const MeshHost &M = P.mesh;
+  const int T = M.elem2D, S = P.S;
+  std::vector<int4> idx(T);
+  std::vector<R> geo(8 * (size_t)T, R(0));
+  for (int e = 0; e < T; e++) {
+    const int *en = &M.elem_nodes[3 * (size_t)e];
+    idx[e] = make_int4(en[0] * S, en[1] * S, en[2] * S, M.nlev_elem[e] - 1);
+    for (int q = 0; q < 6; q++) geo[8 * (size_t)e + q] = (R)M.grad_sca[6 * (size_t)e + q];
+    geo[8 * (size_t)e + 6] = (R)M.elem_area[e];
+  }
+  d.elem_idx = P.upload(idx);
+  d.elem_geo = P.upload(geo);
 }
 
 // Per-edge records of k_edge (DMeshT::edge_idx, edge_geo).
@@ -349,6 +371,8 @@ void build_dmesh(EngineImpl &P, DMeshT<R> &d, const std::vector<int> &slot_edge,
   build_schedules(P, d, kCellsPerBlock);
   build_edge_records(P, d);
   d.edge_pairs = build_edge_pairs(P);
+  build_elem_records(P, d);
+  d.grad_pairs = build_grad_pairs(P);
   build_node_records(P, d, edge_slot);
   d.node_pairs = build_node_pairs(P);
 }

@@ -32,14 +32,30 @@ void set_smem(K kernel, size_t bytes) {
   done[(const void *)kernel] = bytes;
 }
 
+// Launch of a step kernel on the engine's stream, overlapping its prologue with
+// the kernel before it (pdl_wait) unless the launches are being captured.
+template <typename... P, typename... A>
+void launch_step(EngineImpl &E, void (*kernel)(P...), int grid, int threads, const A &...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = E.stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = E.pdl ? 1 : 0;
+  CK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
 template <typename R, typename TS, int NT, int HOR, int LIM>
 void launch_edge(EngineImpl &P, const FusedArgs<R, TS> &a) {
   const DMeshT<R> &m = dmesh<R>(P);
   if (m.edge_pairs.nwarps <= 0) return;
   const int per = pair_run(m.edge_pairs, kEdgeRun), grid = pair_blocks(m.edge_pairs, kEdgeThreads, per);
   P.mark_begin(KK_EDGE);
-  if (a.vflux_mode == 2) k_edge<R, TS, NT, HOR, LIM, true><<<grid, kEdgeThreads, 0, P.stream>>>(m, a, per);
-  else k_edge<R, TS, NT, HOR, LIM, false><<<grid, kEdgeThreads, 0, P.stream>>>(m, a, per);
+  if (a.vflux_mode == 2) launch_step(P, k_edge<R, TS, NT, HOR, LIM, true>, grid, kEdgeThreads, m, a, per);
+  else launch_step(P, k_edge<R, TS, NT, HOR, LIM, false>, grid, kEdgeThreads, m, a, per);
   P.mark_end();
 }
 
@@ -49,17 +65,17 @@ void launch_col1(EngineImpl &P, const FusedArgs<R, TS> &a) {
   const int per = pair_run(m.node_pairs, kColRun);
   const int grid = pair_blocks(m.node_pairs, kColThreads, per);
   P.mark_begin(KK_COL1);
-  if (VER != VER_PPM || m.uniform_h) k_col1<R, TS, NT, VER, LIM, true><<<grid, kColThreads, 0, P.stream>>>(m, a, per);
-  else k_col1<R, TS, NT, VER, LIM, VER != VER_PPM><<<grid, kColThreads, 0, P.stream>>>(m, a, per);
+  if (VER != VER_PPM || m.uniform_h) launch_step(P, k_col1<R, TS, NT, VER, LIM, true>, grid, kColThreads, m, a, per);
+  else launch_step(P, k_col1<R, TS, NT, VER, LIM, VER != VER_PPM>, grid, kColThreads, m, a, per);
   P.mark_end();
 }
 
 template <typename R, typename TS, int NT>
 void launch_grad(EngineImpl &P, const FusedArgs<R, TS> &a) {
   const DMeshT<R> &m = dmesh<R>(P);
-  if (m.grad_sched.nblk <= 0) return;
+  if (m.grad_pairs.nwarps <= 0) return;
   P.mark_begin(KK_GRAD);
-  k_grad<R, TS, NT><<<m.grad_sched.nblk, kThreads, smem_edge(), P.stream>>>(m, a);
+  launch_step(P, k_grad<R, TS, NT>, pair_blocks(m.grad_pairs, kColThreads, 1), kColThreads, m, a);
   P.mark_end();
 }
 
@@ -92,11 +108,11 @@ void run_group(EngineImpl &P, const TracerScheme &sc, const FusedArgs<R, TS> &a)
   const int per = pair_run(m.node_pairs, kColRun), nb = pair_blocks(m.node_pairs, kColThreads, per);
   if (LIM == LIM_FCT) {
     P.mark_begin(KK_COL2);
-    k_col2<R, TS, NT><<<nb, kColThreads, 0, P.stream>>>(m, a, per);
+    launch_step(P, k_col2<R, TS, NT>, nb, kColThreads, m, a, per);
     P.mark_end();
   }
   P.mark_begin(KK_COL3);
-  k_col3<R, TS, NT, LIM><<<nb, kColThreads, 0, P.stream>>>(m, a, per);
+  launch_step(P, k_col3<R, TS, NT, LIM>, nb, kColThreads, m, a, per);
   P.mark_end();
 }
 
