@@ -921,7 +921,6 @@ void Engine::volume_sum(int id, double out[2]) const {
 void Engine::stats(int id, double out[4]) const {
   EngineImpl &P = *p_;
   check_id(P, id);
-  CK(cudaStreamSynchronize(P.stream));
   tracer_stats(P, P.tr[id].T, P.tr[id].off, out);
 }
 

@@ -71,7 +71,7 @@ struct EngineImpl {
   // (nl-1, nod2D) FP64 layout, and a ring of pinned host slots
   static constexpr int kRing = 4;
   double *stage_d = nullptr;
-  double *stats_d = nullptr;  // per-block partial statistics (tracer_stats)
+  double *stats_h = nullptr;  // per-block partial statistics, page-locked (tracer_stats)
   // pipelined host-I/O step (Engine::step_io): per-tracer device buffers of
   // the host layout, the two copy streams and their events
   std::vector<double *> io_in, io_out;

@@ -219,17 +219,26 @@ constexpr int kGrid = 148 * 8, kBlock = 256;
 // back (wet cells T = storage + off, dry cells the storage itself): per block
 // the minimum and maximum of the non-NaN values, the NaN count and a
 // Neumaier-compensated sum, in a fixed assignment of cells to threads and a
-// fixed reduction order, so the result does not depend on scheduling.
+// fixed reduction order, so the result does not depend on scheduling.  The
+// partial results (and the first raw value) go straight to page-locked host
+// memory: the call waits for the kernel alone instead of two copies after it
+// (42 -> 17 us a call at 20x20x10).
 constexpr int kStatBlocks = 296, kStatThreads = 256;
 template <typename TS>
 __global__ void __launch_bounds__(kStatThreads) k_stats(const TS *__restrict__ s, const int *__restrict__ nlev,
                                                         int L, int S, long long N, double off, double *out) {
   double mn = INFINITY, mx = -INFINITY, nan = 0.0, sm = 0.0, c = 0.0;
   const long long total = N * L;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long n = i / L;
-    const int k = (int)(i - n * L);
+  const int step = gridDim.x * blockDim.x, dn = step / L, dk = step - dn * L;
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  long long n = i0 / L;
+  int k = i0 - (int)n * L;
+  for (; n * L + k < total; n += dn, k += dk) {  // cell index i0 + j step as (node, level), without divisions
+    if (k >= L) {
+      k -= L;
+      n++;
+      if (n * L + k >= total) break;
+    }
     const double raw = from_ts<TS>(s[n * S + k]);
     const double v = k < nlev[n] - 1 ? raw + off : raw;
     if (v != v) {
@@ -260,6 +269,7 @@ __global__ void __launch_bounds__(kStatThreads) k_stats(const TS *__restrict__ s
     __syncthreads();
   }
   if (tid < 5) out[5 * blockIdx.x + tid] = sh[tid][0];
+  if (blockIdx.x == 0 && tid == 0 && total > 0) out[5 * kStatBlocks] = from_ts<TS>(s[0]);
 }
 
 template <typename TS>
@@ -368,44 +378,39 @@ void stage_unpack(EngineImpl &P, const void *s, double off) {
 }
 
 void tracer_stats(EngineImpl &P, const void *s, double off, double out[4]) {
-  if (!P.stats_d) P.stats_d = P.dalloc<double>(5 * kStatBlocks + 1);
+  if (!P.stats_h) CK(cudaHostAlloc((void **)&P.stats_h, (5 * kStatBlocks + 1) * sizeof(double), cudaHostAllocMapped));
+  double *out_d = nullptr;
+  CK(cudaHostGetDevicePointer((void **)&out_d, P.stats_h, 0));
+  const double *h = P.stats_h;
   const int L = P.mesh.nl - 1;
   const long long N = P.mesh.nod2D;
+  // blocks without a cell would add nothing
+  const int nblk = (int)std::max<long long>(1, std::min<long long>(kStatBlocks, (N * L + kStatThreads - 1) / kStatThreads));
   switch (P.prec) {
     case Precision::FP32:
-      k_stats<float><<<kStatBlocks, kStatThreads, 0, P.stream>>>((const float *)s, nlev_dev(P), L, P.S, N, off, P.stats_d);
+      k_stats<float><<<nblk, kStatThreads, 0, P.stream>>>((const float *)s, nlev_dev(P), L, P.S, N, off, out_d);
       break;
     case Precision::BF16:
-      k_stats<__nv_bfloat16><<<kStatBlocks, kStatThreads, 0, P.stream>>>((const __nv_bfloat16 *)s, nlev_dev(P), L, P.S,
-                                                                        N, off, P.stats_d);
+      k_stats<__nv_bfloat16><<<nblk, kStatThreads, 0, P.stream>>>((const __nv_bfloat16 *)s, nlev_dev(P), L, P.S,
+                                                                        N, off, out_d);
       break;
     case Precision::FP16:
-      k_stats<__half><<<kStatBlocks, kStatThreads, 0, P.stream>>>((const __half *)s, nlev_dev(P), L, P.S, N, off,
-                                                                 P.stats_d);
+      k_stats<__half><<<nblk, kStatThreads, 0, P.stream>>>((const __half *)s, nlev_dev(P), L, P.S, N, off,
+                                                                 out_d);
       break;
     default:
-      k_stats<double><<<kStatBlocks, kStatThreads, 0, P.stream>>>((const double *)s, nlev_dev(P), L, P.S, N, off,
-                                                                 P.stats_d);
+      k_stats<double><<<nblk, kStatThreads, 0, P.stream>>>((const double *)s, nlev_dev(P), L, P.S, N, off,
+                                                                 out_d);
       break;
   }
   CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(P.stream));
   // the first cell as the host reads it: a NaN there makes min and max NaN,
   // like a host loop seeded with the first value
-  std::vector<double> h(5 * kStatBlocks);
-  P.d2h(h.data(), P.stats_d, h.size() * sizeof(double));
   double first = 0.0;
-  if (L > 0 && N > 0) {
-    double raw = 0.0;
-    switch (P.prec) {
-      case Precision::FP32: { float f; P.d2h(&f, s, 4); raw = f; break; }
-      case Precision::BF16: { __nv_bfloat16 b; P.d2h(&b, s, 2); raw = (double)__bfloat162float(b); break; }
-      case Precision::FP16: { __half b; P.d2h(&b, s, 2); raw = (double)__half2float(b); break; }
-      default: P.d2h(&raw, s, 8); break;
-    }
-    first = (P.mesh.nlev_node[0] - 1 > 0) ? raw + off : raw;
-  }
+  if (L > 0 && N > 0) first = (P.mesh.nlev_node[0] - 1 > 0) ? h[5 * kStatBlocks] + off : h[5 * kStatBlocks];
   double mn = INFINITY, mx = -INFINITY, nan = 0.0, sm = 0.0, c = 0.0;
-  for (int b = 0; b < kStatBlocks; b++) {
+  for (int b = 0; b < nblk; b++) {
     mn = std::fmin(mn, h[5 * b]);
     mx = std::fmax(mx, h[5 * b + 1]);
     nan += h[5 * b + 2];
@@ -449,6 +454,8 @@ void storage_reoffset(EngineImpl &P, void *s, double off_old, double off_new) {
 }
 
 void release_ring(EngineImpl &P) {
+  if (P.stats_h) cudaFreeHost(P.stats_h);
+  P.stats_h = nullptr;
   for (int s = 0; s < EngineImpl::kRing; s++) {
     if (P.ring_ev[s]) cudaEventDestroy(P.ring_ev[s]);
     if (P.ring[s]) cudaFreeHost(P.ring[s]);
