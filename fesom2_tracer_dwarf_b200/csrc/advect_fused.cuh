@@ -47,7 +47,8 @@ __device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch
 // is the loads in flight per warp: 16 warps of 128 registers per SM beat 20-24
 // with fewer (FP64, 400x400x64, two tracers: k_edge 0.30 ms at 4 blocks, 0.33 at 3; k_col1
 // 0.225 at 4, 0.256 / 0.30 at 3 / 5; k_col3 0.236 at 4, 0.237 / 0.32; FP32 k_edge 0.184 at 5, 0.193
-// / 0.188 at 4 / 6; k_col2 0.138 at 6, 0.152 at 5).  Build-time knobs.
+// / 0.188 at 4 / 6; k_col1 0.133 at 7, 0.141 at 5, and with BF16 storage at 500x500x48
+// 0.152, 0.172; k_col2 0.138 at 6, 0.148 at 8).  Build-time knobs.
 #ifndef FESOM_MINB_EDGE
 #define FESOM_MINB_EDGE 4
 #endif
@@ -70,22 +71,27 @@ __device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch
 #define FESOM_MINB32_EDGE 5
 #endif
 #ifndef FESOM_MINB32_COL1
-#define FESOM_MINB32_COL1 5
+#define FESOM_MINB32_COL1 7
 #endif
 #ifndef FESOM_MINB32_COL2
 #define FESOM_MINB32_COL2 6
 #endif
 #ifndef FESOM_MINB32_COL3
-#define FESOM_MINB32_COL3 5
+#define FESOM_MINB32_COL3 7
 #endif
 template <typename R, int NT>
 struct StepBlocks {
-  static constexpr int grad = FESOM_MINB_GRAD, edge = FESOM_MINB_EDGE, col1 = FESOM_MINB_COL1, col2 = FESOM_MINB_COL2, col3 = FESOM_MINB_COL3;
+  // (k_col1 of one tracer: 6 blocks 0.148, 4 blocks 0.161 ms)
+  static constexpr int grad = FESOM_MINB_GRAD, edge = FESOM_MINB_EDGE, col1 = NT == 1 ? 6 : FESOM_MINB_COL1,
+                       col2 = FESOM_MINB_COL2, col3 = FESOM_MINB_COL3;
 };
 template <int NT>
-struct StepBlocks<float, NT> {  // four tracers a lane: 128 registers
-  static constexpr int grad = FESOM_MINB32_GRAD, edge = NT == 4 ? 4 : FESOM_MINB32_EDGE, col1 = NT == 4 ? 4 : FESOM_MINB32_COL1,
-                       col2 = NT == 4 ? 4 : FESOM_MINB32_COL2, col3 = NT == 4 ? 4 : FESOM_MINB32_COL3;
+struct StepBlocks<float, NT> {
+  // four tracers a lane: 128 registers; one: more blocks (k_col1 0.093 ms at 9, 0.105
+  // at 5; BF16 storage 0.105, 0.138)
+  static constexpr int pick(int n1, int n2) { return NT == 4 ? 4 : (NT == 1 ? n1 : n2); }
+  static constexpr int grad = FESOM_MINB32_GRAD, edge = pick(6, FESOM_MINB32_EDGE), col1 = pick(9, FESOM_MINB32_COL1),
+                       col2 = pick(8, FESOM_MINB32_COL2), col3 = pick(7, FESOM_MINB32_COL3);
 };
 // Tracers of a batch of NT that a lane advances together; it takes the groups one
 // after the other.  Two FP64 tracers share a column's records and geometry
