@@ -333,12 +333,12 @@ __device__ __forceinline__ void grad_block(const DMeshT<R> &m, const FusedArgs<R
   const int warp = blk * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
   if (warp >= m.grad_pairs.nwarps) return;
   const PairLane l = pair_lane(m.grad_pairs, warp);
-  if (l.on) prefetch(m.ring_elem + m.ring_ptr[l.item]);
+  if (l.on()) prefetch(m.ring_elem + m.ring_ptr[l.item]);
   pdl_wait();
-  if (!l.on) return;
+  if (!l.on()) return;
   constexpr int G = LaneTracers<R, NT>::grad;
   if constexpr (G == NT) {
-    grad_pair<R, TS, NT>(m, a, l.item, l.k);
+    grad_pair<R, TS, NT>(m, a, l.item, l.k());
   } else {
     FusedArgs<R, TS> b;  // the pointers grad_pair reads, of one group of tracers at a time
 #pragma unroll
@@ -349,7 +349,7 @@ __device__ __forceinline__ void grad_block(const DMeshT<R> &m, const FusedArgs<R
         b.off[t] = a.off[t0 + t];
         b.gradn[t] = a.gradn[t0 + t];
       }
-      grad_pair<R, TS, G>(m, b, l.item, l.k);
+      grad_pair<R, TS, G>(m, b, l.item, l.k());
     }
   }
 }
@@ -650,9 +650,9 @@ __device__ __forceinline__ void edge_block(const DMeshT<R> &m, const FusedArgs<R
       idx = edge_idx(m, nxt.item);
       if (warp + 1 < end) nn = pair_lane(s, warp + 1);
     }
-    if (c.on) {
-      if (HOR != HOR_UPW1 && c.ring) edge_pair<R, TS, NT, HOR, LIM, LOADV, true>(m, a, c.item, c.k, x);
-      else edge_pair<R, TS, NT, HOR, LIM, LOADV, false>(m, a, c.item, c.k, x);
+    if (c.on()) {
+      if (HOR != HOR_UPW1 && c.ring()) edge_pair<R, TS, NT, HOR, LIM, LOADV, true>(m, a, c.item, c.k(), x);
+      else edge_pair<R, TS, NT, HOR, LIM, LOADV, false>(m, a, c.item, c.k(), x);
     }
   } while (warp < end);
 }
@@ -853,7 +853,7 @@ __device__ __noinline__ void col1_vert_slow(const DMeshT<R> &m, const FusedArgs<
 // and reciprocal thicknesses; otherwise they are formed here.
 template <typename R, typename TS, int NT, int G, int VER, int LIM, bool UNI>
 __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, const PairLane &l) {
-  const int n = l.item, k = l.k, S = m.S;
+  const int n = l.item, k = l.k(), S = m.S;
   const cix col = (cix)n * S, o = col + k;
   const NodeRec rec = node_rec(m, n);
   const int nln = rec.nlev() - 1;
@@ -1021,7 +1021,7 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
         hov[2 * t + q] = kk >= nln ? R(0) : v;
       }
   }
-  const bool st = l.on && !l.halo;
+  const bool st = l.stores();
   if (st) {
     st_pair_il<NT, G>(a.adf_v, t0, o, hov);
     if (k + 2 == nln)  // the bottom interface of a column of whole pairs
@@ -1137,7 +1137,7 @@ __device__ __noinline__ Bounds<R> ring_bounds(const DMeshT<R> &m, const FusedArg
 
 template <typename R, typename TS, int NT, int G>
 __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, const PairLane &l) {
-  const int n = l.item, k = l.k, S = m.S;
+  const int n = l.item, k = l.k(), S = m.S;
   const cix o = (cix)n * S + k;
   const NodeRec rec = node_rec(m, n);
   const int nln = rec.nlev() - 1;
@@ -1258,7 +1258,7 @@ __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R,
       }
     }
     if (k + 1 >= nln) out[2] = out[3] = R(0);  // dry: read by k_col3 against a zero flux
-    if (l.on && !l.halo) {
+    if (l.stores()) {
       stv4(a.rpm[t0 + t] + 2 * (size_t)o, out);
       if (bad) {
         for (int q = 0; q < 2; q++) {
@@ -1424,8 +1424,8 @@ __device__ __noinline__ void col3_pair_slow(const DMeshT<R> &m, const FusedArgs<
 
 template <typename R, typename TS, int NT, int G, int LIM>
 __device__ __forceinline__ void col3_pair(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, const PairLane &l) {
-  if (!l.on || l.halo) return;
-  const int n = l.item, k = l.k;
+  if (!l.stores()) return;
+  const int n = l.item, k = l.k();
   const NodeRec rec = node_rec(m, n);
   const int wet = min(rec.nlev() - 1 - k, 2);
   bool bad = false;

@@ -163,19 +163,16 @@ __device__ __forceinline__ void ld_pair_T_if(const TS *p, cix o, R off, bool on,
 // A lane's entry of a pair schedule (DPairs in dmesh.hpp).  Lanes without a
 // pair hold some item and level 0.
 struct PairLane {
-  int item, k;
-  bool on, halo, ring;
+  int item;
+  unsigned code;
+  __device__ __forceinline__ bool on() const { return code != kPairNone; }
+  __device__ __forceinline__ bool stores() const { return code < kPairHalo; }
+  __device__ __forceinline__ bool ring() const { return (code & kPairRing) != 0; }
+  __device__ __forceinline__ int k() const { return on() ? (int)(code & kPairLevel) : 0; }
 };
 __device__ __forceinline__ PairLane pair_lane(const DPairs &s, int warp) {
   const int i = warp * 32 + (int)(threadIdx.x & 31);
-  const unsigned c = s.lev[i];
-  PairLane p;
-  p.item = s.item[i];
-  p.on = c != kPairNone;
-  p.halo = (c & kPairHalo) != 0;
-  p.ring = (c & kPairRing) != 0;
-  p.k = p.on ? (int)(c & kPairLevel) : 0;
-  return p;
+  return PairLane{s.item[i], s.lev[i]};
 }
 
 FESOM_VARIANT_END
