@@ -3,17 +3,20 @@
 // into four passes and batched over up to NTMAX tracers that share a mesh,
 // a flow and a scheme.
 //
-//   k_edge  [edge cells]  volume flux of every edge level (stored once for all
+//   k_edge  [edge pairs]  volume flux of every edge level (stored once for all
 //                         tracers) and, per tracer, the antidiffusive flux
 //                         HO(T_AB) - LO(T) (MUSCL/MFCT/UPW1), or HO alone
 //                         without FCT
-//   k_col1  [node cells]  horizontal LO gather, vertical LO and HO fluxes
-//                         (PPM slopes and interface values staged in shared
-//                         memory, geometry coefficients shared by the tracers),
-//                         LO solution
-//   k_col2  [node cells]  FCT cluster bounds (a1-a3), antidiffusive in/out
+//   k_col1  [node pairs]  horizontal LO gather, vertical LO and HO fluxes
+//                         (PPM slopes and interface values of the neighbouring
+//                         levels by shuffle, geometry coefficients shared by the
+//                         tracers), LO solution
+//   k_col2  [node pairs]  FCT cluster bounds (a1-a3), antidiffusive in/out
 //                         sums (b1) and limiter ratios (b2)
-//   k_col3  [node cells]  limiting (b3), flux2dtracer, T += del / h_new
+//   k_col3  [node pairs]  limiting (b3), flux2dtracer, T += del / h_new
+//
+// A lane advances a pair of levels (2j+1, 2j+2) of its column or edge for every
+// tracer of its group; warps are packed with whole columns (pairs.cuh).
 //
 // Edge scatters of the reference become node-centric gathers over the
 // node's incident edges in ascending edge id: every node sums its
@@ -104,7 +107,7 @@ struct LaneTracers {
   static constexpr int col1 = cap(sizeof(R) == 8 ? 2 : 4), col2 = cap(sizeof(R) == 8 ? 1 : 4), col3 = col1,
                        grad = cap(sizeof(R) == 8 ? 2 : 4);
 };
-constexpr int kCellsPerBlock = 512;      // schedule cap: wet cells per block (two per thread)
+constexpr int kCellsPerBlock = 512;      // cell maps (learned flux): wet cells per block, two per thread
 constexpr int kMaxCellsPerBlock = 576;   // upper bound (target + deepest column)
 constexpr int kMaxItemsPerBlock = 512;
 

@@ -154,13 +154,9 @@ struct PhasePack {
 };
 static_assert(sizeof(PhasePack) <= 32000, "phase pack must fit the kernel parameter space");
 
-// resident 256-thread blocks per SM each phase kernel's register budget is
-// cut for (build-time knobs).  One block fewer than the standalone FP32
-// kernels: the task lookup and the descriptor loads from parameter space
-// need registers of their own.  Measured on the 48-tracer x 8-member
-// ensemble: 424 ms per step against 456 with the standalone budgets.
-// (Copying the descriptor into shared memory instead was slower still:
-// 491-525 ms, the pointers then occupy registers.)
+// Resident 256-thread blocks per SM each phase kernel's register budget is
+// cut for (build-time knobs): 16 warps of 128 registers, the budget of the
+// standalone kernels of four FP32 tracers.
 #ifndef FESOM_PHASE_MINB_GRAD
 #define FESOM_PHASE_MINB_GRAD 5
 #endif
@@ -187,12 +183,10 @@ struct PhaseBudget {
 
 template <int PH, int HOR, int VER, int LIM>
 __global__ void __launch_bounds__(kThreads, PhaseBudget<PH>::v) k_batch_phase(const __grid_constant__ PhasePack p) {
-  extern __shared__ __align__(16) int smem[];
   const int total = p.prefix[p.ntasks];
   int task = 0;
   for (int g = blockIdx.x; g < total; g += gridDim.x) {
     while (p.prefix[task + 1] <= g) task++;
-    if (g != (int)blockIdx.x) __syncthreads();  // the previous item is done with shared memory
     const int vblk = g - p.prefix[task];
     const BatchTask &st = p.t[task];
     if (PH == PH_GRAD) grad_block<float, float, kNT>(st.m, st.a, vblk);

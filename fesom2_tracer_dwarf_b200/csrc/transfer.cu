@@ -222,7 +222,7 @@ constexpr int kGrid = 148 * 8, kBlock = 256;
 // fixed reduction order, so the result does not depend on scheduling.  The
 // partial results (and the first raw value) go straight to page-locked host
 // memory: the call waits for the kernel alone instead of two copies after it
-// (42 -> 17 us a call at 20x20x10).
+// (42 -> 24 us a call at 20x20x10).
 constexpr int kStatBlocks = 296, kStatThreads = 256;
 template <typename TS>
 __global__ void __launch_bounds__(kStatThreads) k_stats(const TS *__restrict__ s, const int *__restrict__ nlev,
