@@ -68,7 +68,7 @@ def parse():
     p.add_argument("--step-path", default="five", choices=["fused", "five"],
                    help="the five-kernel path (default) or the fused patch kernel")
     p.add_argument("--cells-per-block", type=int, default=0,
-                   help="most wet cells per block of the five-kernel schedules (0: the default, 512)")
+                   help="most wet cells per block of the learned flux's training schedules (0: the default, 512)")
     p.add_argument("--learned", action="store_true",
                    help="FP32 with the learned antidiffusive flux (shipped parameters) ahead of FCT")
     p.add_argument("--config", default="c2", choices=["c2", "c3", "c4", "dd"],
@@ -170,10 +170,10 @@ def measured_peaks():
 
 def committed_traffic(args):
     """DRAM bytes per step of the plain FP64 step at 1000x1000x64 from the
-    committed ncu summary (profiles/step_c2_fp64.md, line
+    committed ncu summary (profiles/level_pairs_300x64.md, line
     'dram_bytes_per_step_scaled: X'); None for any other workload or
     precision, which that capture does not cover."""
-    p = ROOT / "profiles" / "step_c2_fp64.md"
+    p = ROOT / "profiles" / "level_pairs_300x64.md"
     if (args.precision != "fp64" or args.learned or args.nx != 1000 or args.nl != 64 or args.step_path != "five"
             or not p.exists()):
         return None
@@ -379,7 +379,7 @@ def run_ours(args):
                          "frac": achieved / peak, "traffic": traffic,
                          "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the five step "
                                             "kernels of one step on the 300x300x64 case of this workload, scaled by "
-                                            "wet cells (x11.17) to this size; profiles/step_c2_fp64.md"
+                                            "wet cells (x11.17) to this size; profiles/level_pairs_300x64.md"
                                             if traffic else None),
                          "kernel": f"full step (all kernels of one step, {BYTES_PER_CELL[args.precision]} B/cell algorithmic)",
                          "peak_source": f"{peak_kind} hbm_gbs"},

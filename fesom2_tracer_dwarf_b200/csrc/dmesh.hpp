@@ -31,8 +31,9 @@ struct DSched {
 
 // Schedule of level pairs over items (nodes or edges): lane i of warp w takes
 // the pair of item[32 w + i] whose first level is lev & kPairLevel, or none where
-// lev is kPairNone.  Items follow one another along a space-filling curve, so
-// that a block's pairs share their neighbours' columns in L1.  Edge pairs whose
+// lev is kPairNone.  Items follow one another in the order of their slots or
+// (within windows of 256) nodes, so that a block's pairs share their neighbours'
+// columns in L1.  Edge pairs whose
 // levels all have both an up and a down triangle and those that have not
 // (kPairRing) are kept in warps apart, so that no warp mixes the two forms of
 // the MUSCL gradient.  kPairHalo: computed, stored by another warp.

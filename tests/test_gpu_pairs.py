@@ -32,11 +32,11 @@ def run_both(api, m, tracers, uv, w, dt, scheme, steps, refresh=True):
             assert_bitwise(api.get_tracer_values(i + 1), T, f"tracer {i + 1} step {s + 1}")
 
 
-@pytest.mark.parametrize("nl", [3, 4, 5, 34, 64, 65, 66, 67, 96, 130, 200])
+@pytest.mark.parametrize("nl", [3, 4, 5, 34, 64, 65, 66, 67, 96, 130, 200, 577])
 @pytest.mark.parametrize("ntr", [1, 2])
 def test_column_depths(api, oracle, nl, ntr):
-    """2 to 199 layers over random bathymetry: odd and even columns, columns that
-    just fill a warp and those cut into two, three and four overlapping pieces."""
+    """2 to 576 layers (the most that a mesh may have) over random bathymetry: odd and even columns, columns that
+    just fill a warp and those cut into two and up to ten overlapping pieces."""
     K, uv, w, T, S, dt = synth_case(api, 9, 8, nl, True, nl)
     K[:4] = [nl, max(3, nl - 1), max(3, nl - 2), 3]
     api.init_analytic(9, 8, nl, periodic=True, full_rings=True, node_K=K)
