@@ -73,6 +73,9 @@ __device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch
 #ifndef FESOM_MINB32_EDGE
 #define FESOM_MINB32_EDGE 5
 #endif
+#ifndef FESOM_MINB32_FEAT
+#define FESOM_MINB32_FEAT 4
+#endif
 #ifndef FESOM_MINB32_COL1
 #define FESOM_MINB32_COL1 7
 #endif
@@ -85,7 +88,7 @@ __device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch
 template <typename R, int NT>
 struct StepBlocks {
   // (k_col1 of one tracer: 6 blocks 0.148, 4 blocks 0.161 ms)
-  static constexpr int grad = FESOM_MINB_GRAD, edge = FESOM_MINB_EDGE, col1 = NT == 1 ? 6 : FESOM_MINB_COL1,
+  static constexpr int grad = FESOM_MINB_GRAD, edge = FESOM_MINB_EDGE, feat = edge, col1 = NT == 1 ? 6 : FESOM_MINB_COL1,
                        col2 = FESOM_MINB_COL2, col3 = FESOM_MINB_COL3;
 };
 template <int NT>
@@ -93,6 +96,9 @@ struct StepBlocks<float, NT> {
   // four tracers a lane: 128 registers; one: more blocks (k_col1 0.093 ms at 9, 0.105
   // at 5; BF16 storage 0.105, 0.138)
   static constexpr int pick(int n1, int n2) { return NT == 4 ? 4 : (NT == 1 ? n1 : n2); }
+  // k_edge with the learned flux's features of two tracers: 0.666 ms at 4, 0.784 at 5,
+  // 0.726 at 3 (500x500x64); of one: 0.418 at 6, 0.437 at 4
+  static constexpr int feat = pick(6, FESOM_MINB32_FEAT);
   static constexpr int grad = FESOM_MINB32_GRAD, edge = pick(6, FESOM_MINB32_EDGE), col1 = pick(9, FESOM_MINB32_COL1),
                        col2 = pick(8, FESOM_MINB32_COL2), col3 = pick(7, FESOM_MINB32_COL3);
 };
@@ -394,34 +400,38 @@ __device__ __forceinline__ R div6(R x, bool &bad) { return div_3k<6>(x, bad); }
 template <typename R>
 __device__ __forceinline__ R div3(R x, bool &bad) { return div_3k<3>(x, bad); }
 
+// Reciprocals of the learned flux's features, straight-line: an approximate
+// reciprocal within a unit in the last place and one Newton step round 1 / x
+// (see div_any).
+__device__ __forceinline__ float rcp_newton(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return __fmaf_rn(__fmaf_rn(-x, y, 1.0f), y, y);
+}
+// Courant number of an edge level's volume flux in the upwind node's cell, of
+// volume vol; the same for every tracer.
+__device__ __forceinline__ float edge_courant(float vflux, float dt, float vol) {
+  bool bad = false;
+  const float num = fabsf(vflux) * dt;
+  float cour = div_fast(num, vol, rcp_newton(vol), bad);
+  if (bad) cour = num / vol;
+  return fminf(cour, 4.0f);
+}
+
 // learned flux: 16 features of one MUSCL edge level in the flow's frame, in
 // units of the local variation sig, and the scale of the network's output
 template <typename TS>
 __device__ __forceinline__ void edge_features(const DMeshT<float> &m, const FusedArgs<float, TS> &a, int t, int cell,
-                                              int k, float vflux, float t1, float t2, float x1, float x2, float Tmean1,
+                                              int k, float vflux, float cour, float t1, float t2, float x1, float x2, float Tmean1,
                                               float Tmean2, float gux, float guy, float gdx, float gdy, float exa,
-                                              float eyr, float c_lo1, float c_lo2, cix o1, cix o2, bool shared) {
+                                              float eyr, float c_lo1, float c_lo2, bool shared) {
   const float sixth = 1.0f / 6.0f;
   const bool fwd = vflux >= 0.0f;
   const float tu = fwd ? t1 : t2, td = fwd ? t2 : t1;
   const float xu = fwd ? x1 : -x2, xd = fwd ? x2 : -x1;
   const float face = 0.5f * (Tmean1 + Tmean2);
   const float sig = fabsf(td - tu) + (fabsf(xu) + fabsf(xd)) * sixth + 1e-6f * (fabsf(tu) + fabsf(td)) + 1e-20f;
-  // the two quotients straight-line: an approximate reciprocal within a unit in
-  // the last place and one Newton step round 1 / x (see div_any), Markstein's
-  // correction the quotient
-  auto rcp = [](float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return __fmaf_rn(__fmaf_rn(-x, y, 1.0f), y, y);
-  };
-  const float inv = rcp(sig);
-  const cix ou = fwd ? o1 : o2;
-  bool bad = false;
-  const float num = fabsf(vflux) * a.dt, vol = m.areasvol[ou] * m.hnode_new[ou];
-  float cour = div_fast(num, vol, rcp(vol), bad);
-  if (bad) cour = num / vol;
-  cour = fminf(cour, 4.0f);
+  const float inv = rcp_newton(sig);
   const float gx = fwd ? gux : gdx, gy = fwd ? guy : gdy;
   const float trans = (-eyr * gx + exa * gy) * inv;
   float f[16];
@@ -497,9 +507,12 @@ __device__ __noinline__ void edge_pair_slow(const DMeshT<R> &m, const FusedArgs<
       const R ho = -(R(0.5) * (R(1) - a.ph) * cHO) - vf * a.ph * R(0.5) * (Tmean1 + Tmean2);
       const R flo = (LIM == LIM_FCT) ? upw1_flux(vf, ldT<R>(a.T[t], o1, a.off[t]), ldT<R>(a.T[t], o2, a.off[t])) : R(0);
       il<NT>(a.adf_h, t, o) = ho - flo;
-      if constexpr (HOR == HOR_MUSCL_FEAT)
-        edge_features(m, a, t, m.edge_sched.cell_off[e] + k, k, vf, b1, b2, x1, x2, Tmean1, Tmean2, gux, guy, gdx, gdy,
-                      g[12], g[13], c1, c2, o1, o2, k < x.tri_levels());
+      if constexpr (HOR == HOR_MUSCL_FEAT) {
+        const cix ou = vf >= R(0) ? o1 : o2;
+        edge_features(m, a, t, m.edge_sched.cell_off[e] + k, k, vf,
+                      edge_courant(vf, a.dt, m.areasvol[ou] * m.hnode_new[ou]), b1, b2, x1, x2, Tmean1, Tmean2, gux, guy,
+                      gdx, gdy, g[12], g[13], c1, c2, k < x.tri_levels());
+      }
     }
   }
 }
@@ -546,6 +559,16 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
     bool bad = false;
     // the loads of G tracers are all issued before the first is used
     constexpr int G = NT > 2 ? 2 : NT;
+    [[maybe_unused]] int cell = 0;
+    [[maybe_unused]] R vol[2] = {R(1), R(1)};
+    if constexpr (HOR == HOR_MUSCL_FEAT) {
+      cell = m.edge_sched.cell_off[e] + k;
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const cix ou = (vf[q] >= R(0) ? o1 : o2) + q;
+        vol[q] = m.areasvol[ou] * m.hnode_new[ou];
+      }
+    }
 #pragma unroll
     for (int t0 = 0; t0 < NT; t0 += G) {
       R b1[G][2], b2[G][2], u[G][3][2], d[G][3][2], p1[G][4], p2[G][4];
@@ -576,6 +599,11 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
       }
       const R exa = g[12], eyr = g[13];
       const R hph = R(0.5) * (R(1) - a.ph);
+      [[maybe_unused]] R cour[2];
+      if constexpr (HOR == HOR_MUSCL_FEAT) {
+        cour[0] = edge_courant(vf[0], a.dt, vol[0]);
+        cour[1] = edge_courant(vf[1], a.dt, vol[1]);
+      }
       R out[2 * G];
 #pragma unroll
       for (int i = 0; i < G; i++) {
@@ -616,8 +644,8 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
           out[2 * i + q] = ho - flo;
           if constexpr (HOR == HOR_MUSCL_FEAT) {
             if (k + q < x.levels())
-              edge_features(m, a, t, m.edge_sched.cell_off[e] + k + q, k + q, vf[q], b1[i][q], b2[i][q], x1, x2, Tmean1,
-                            Tmean2, gux, guy, gdx, gdy, exa, eyr, c1, c2, o1 + q, o2 + q, sh);
+              edge_features(m, a, t, cell + q, k + q, vf[q], cour[q], b1[i][q], b2[i][q], x1, x2, Tmean1, Tmean2, gux,
+                            guy, gdx, gdy, exa, eyr, c1, c2, sh);
           }
         }
       }
@@ -661,7 +689,7 @@ __device__ __forceinline__ void edge_block(const DMeshT<R> &m, const FusedArgs<R
 }
 
 template <typename R, typename TS, int NT, int HOR, int LIM, bool LOADV>
-__global__ void __launch_bounds__(kEdgeThreads, StepBlocks<R, NT>::edge)
+__global__ void __launch_bounds__(kEdgeThreads, HOR == HOR_MUSCL_FEAT ? StepBlocks<R, NT>::feat : StepBlocks<R, NT>::edge)
     k_edge(const __grid_constant__ DMeshT<R> m, const __grid_constant__ FusedArgs<R, TS> a, int per) {
   pdl_launch();
   edge_block<R, TS, NT, HOR, LIM, LOADV>(m, a, blockIdx.x, per);
