@@ -689,7 +689,8 @@ struct LearnedState {
   float *fscale[kBatchMax] = {};
   unsigned *cell = nullptr;  // slot x S + level of every edge cell
   float *dy = nullptr, *target = nullptr, *hp = nullptr, *hm = nullptr;
-  double *red = nullptr;  // per-block partial sums
+  double *red = nullptr;  // per-block partial sums, red_cap of them
+  int red_cap = 0;
   double volume = 0.0;    // sum of areasvol * hnode_new over wet cells
   float adam_b1 = 0.9f, adam_b2 = 0.999f;
 };
@@ -942,7 +943,6 @@ void Engine::set_learned(const float *params, bool on) {
     L.dy = dmalloc<float>(L.ncells);
     L.target = dmalloc<float>((size_t)M.nod2D * P.S);
     CK(cudaMemset(L.target, 0, (size_t)M.nod2D * P.S * sizeof(float)));
-    L.red = dmalloc<double>(std::max(1, P.dm32.node_sched.nblk));
   }
   LearnedState &L = *P.learn;
   if (params) {
@@ -996,6 +996,16 @@ double Engine::learn_step(const double *T_in, const double *T_target, double dt,
   stage_pack(P, 0.0, L.target, nullptr, nullptr);
   const DMeshT<float> &m = P.dm32;
   const float *T = (const float *)P.tr[0].T;
+  // one partial sum per block of the node schedule, whose tile may have changed
+  // since the last step (set_cells_per_block)
+  if (m.node_sched.nblk > L.red_cap) {
+    CK(cudaStreamSynchronize(P.stream));
+    cudaFree(L.red);
+    L.red = nullptr;
+    L.red_cap = 0;
+    L.red = dmalloc<double>(m.node_sched.nblk);
+    L.red_cap = m.node_sched.nblk;
+  }
   k_learn_loss<<<m.node_sched.nblk, kThreads, smem_edge(), P.stream>>>(m, T, L.target, L.red);
   CK(cudaGetLastError());
   std::vector<double> part(std::max(1, m.node_sched.nblk));
