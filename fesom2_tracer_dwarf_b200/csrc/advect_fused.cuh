@@ -227,6 +227,10 @@ __device__ __forceinline__ void st_pair(float *p, float x, float y) {
   *reinterpret_cast<float2 *>(p) = make_float2(x, y);
 }
 
+// Whether a is not a zero, given u = 2 x its high word: subnormals below 2^-1042
+// have a high word of zero and a low word that is not.
+__device__ __forceinline__ bool not_zero(double a, unsigned u) { return (u | (unsigned)__double2loint(a)) != 0u; }
+
 // a / b given y = RN(1 / b), correctly rounded (see div_rcp), straight-line:
 // numerators outside [2^-900, 2^900] other than zero set `bad` and the caller
 // divides again.  The sign of a zero result is not kept (no output of the step
@@ -235,7 +239,7 @@ __device__ __forceinline__ double div_fast(double a, double b, double y, bool &b
   double q = a * y;
   q = __fma_rn(__fma_rn(-b, q, a), y, q);
   const unsigned u = 2u * (unsigned)__double2hiint(a);
-  bad |= (u - 0x0f600000u > 0xf0800000u - 0x0f600000u) && u != 0u;
+  bad |= (u - 0x0f600000u > 0xf0800000u - 0x0f600000u) && not_zero(a, u);
   return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 __device__ __forceinline__ float div_fast(float a, float b, float y, bool &bad) {
@@ -273,7 +277,7 @@ __device__ __forceinline__ float rcp_exact(float b, bool &bad) {
 // zero set `bad` too, so that no quotient underflows)
 __device__ __forceinline__ double div_any(double a, double b, bool &bad) {
   const unsigned u = 2u * (unsigned)__double2hiint(a);
-  bad |= u < 0x41600000u && u != 0u;
+  bad |= u < 0x41600000u && not_zero(a, u);
   return div_fast(a, b, rcp_exact(b, bad), bad);
 }
 
@@ -384,7 +388,7 @@ __device__ __forceinline__ double div_3k(double x, bool &bad) {
   const double y = 1.0 / B;
   const double q = x * y;
   const unsigned u = 2u * (unsigned)__double2hiint(x);
-  bad |= (u - 0x0f600000u >= 0xffe00000u - 0x0f600000u) && u != 0u;
+  bad |= (u - 0x0f600000u >= 0xffe00000u - 0x0f600000u) && not_zero(x, u);
   return __fma_rn(__fma_rn(-(double)B, q, x), y, q);
 }
 template <int B>
