@@ -91,6 +91,7 @@ SIGNATURES = {
     "tracer_launches_per_step": (ctypes.c_int, []),
     "tracer_device_bytes": (ctypes.c_longlong, []),
     "tracer_selftest_division": (ctypes.c_int, [ctypes.c_longlong, ctypes.c_uint64, _vp, _vp]),
+    "tracer_selftest_quotients": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_uint64, _vp, _vp, _vp]),
     "tracer_selftest_sround": (ctypes.c_int, [ctypes.c_int, ctypes.c_longlong, ctypes.c_int, ctypes.c_uint32,
                                               ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_double)]),
     "tracer_batch_create": (ctypes.c_int, []),

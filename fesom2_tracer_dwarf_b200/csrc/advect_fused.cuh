@@ -273,12 +273,25 @@ __device__ __forceinline__ float rcp_exact(float b, bool &bad) {
   bad |= u - 0x43000000u > 0xbb000000u - 0x43000000u || (__float_as_uint(b) | 0xff800000u) == 0xffffffffu;
   return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
 }
-// a / b for any divisor: the limiter ratios (numerators below 2^-500 other than
-// zero set `bad` too, so that no quotient underflows)
-__device__ __forceinline__ double div_any(double a, double b, bool &bad) {
+// a / b for any divisor: the limiter ratios and the ring means.  Numerators below
+// 2^-500 (FP32: 2^-60) other than zero set `bad` too, so that no quotient underflows.
+__device__ __forceinline__ bool tiny(double a) {
   const unsigned u = 2u * (unsigned)__double2hiint(a);
-  bad |= u < 0x41600000u && not_zero(a, u);
-  return div_fast(a, b, rcp_exact(b, bad), bad);
+  return u < 0x41600000u && not_zero(a, u);
+}
+__device__ __forceinline__ bool tiny(float a) {
+  const unsigned u = 2u * __float_as_uint(a);
+  return u < 0x43000000u && u != 0u;
+}
+// the same given y = RN(1 / b) of rcp_exact
+template <typename R>
+__device__ __forceinline__ R div_any(R a, R b, R y, bool &bad) {
+  bad |= tiny(a);
+  return div_fast(a, b, y, bad);
+}
+template <typename R>
+__device__ __forceinline__ R div_any(R a, R b, bool &bad) {
+  return div_any(a, b, rcp_exact(b, bad), bad);
 }
 
 // One pair of node levels: the ring's elements one after the other (a level an
@@ -328,8 +341,8 @@ __device__ __forceinline__ void grad_pair(const DMeshT<R> &m, const FusedArgs<R,
     R out[4];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
-      out[2 * q] = div_fast(sx[t][q], vol[q], y[q], bad);
-      out[2 * q + 1] = div_fast(sy[t][q], vol[q], y[q], bad);
+      out[2 * q] = div_any(sx[t][q], vol[q], y[q], bad);
+      out[2 * q + 1] = div_any(sy[t][q], vol[q], y[q], bad);
     }
     if (bad)
 #pragma unroll

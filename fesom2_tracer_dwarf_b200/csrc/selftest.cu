@@ -1,7 +1,10 @@
 // Device self-tests of arithmetic primitives of the step kernels:
-//  * the reciprocal-based correctly rounded division of the FP64 kernels:
+//  * the reciprocal-based correctly rounded division of the fused patch kernel:
 //    div_rcp(a, b, 1/b) must return the bits of the IEEE quotient a / b for
 //    every operand pair (Markstein's correction; see advect_fused.cuh);
+//  * the straight-line divisions of the five step kernels (div_fast, div_any,
+//    rcp_exact, div_3k): every result that is not flagged `bad` has the bits of the
+//    IEEE quotient, the sign of a zero aside;
 //  * the stochastic rounding of 16-bit tracer stores (advect_ops.cuh): every
 //    result is one of the two storage neighbours of the input, and the
 //    fraction rounded up matches (remainder / spacing) without bias.
@@ -47,6 +50,106 @@ __global__ void k_div_check(long long n, uint64_t seed, unsigned long long *bad,
     if (__double_as_longlong(q) != __double_as_longlong(ref)) {
       unsigned long long k = atomicAdd(bad, 1ull);
       if (k == 0) { first[0] = a; first[1] = b; first[2] = q; first[3] = ref; }
+    }
+  }
+}
+
+// Operands of the straight-line divisions.  mode 0: ordinary (the flag must stay
+// down); 1: exponents up to 4 beside the edges of the ranges that set the flag, and
+// beyond the largest and smallest ones; 2: significands of all ones, or but a few of
+// them, and powers of two; 3: subnormals of a few bits, zeros, infinities, NaN.
+template <typename R> struct Bits;
+template <> struct Bits<double> {
+  using U = uint64_t;
+  static constexpr int mant = 52, bias = 1023, emax = 2047;
+  __device__ static double make(U u) { return __longlong_as_double((long long)u); }
+  __device__ static U get(double x) { return (U)__double_as_longlong(x); }
+};
+template <> struct Bits<float> {
+  using U = uint32_t;
+  static constexpr int mant = 23, bias = 127, emax = 255;
+  __device__ static float make(U u) { return __uint_as_float(u); }
+  __device__ static U get(float x) { return __float_as_uint(x); }
+};
+template <typename R>
+__device__ R special(uint64_t r, int mode, int lo, int hi, int edge) {
+  using B = Bits<R>;
+  using U = typename B::U;
+  U m = (U)r & (((U)1 << B::mant) - 1);
+  int e = lo + (int)((r >> 52) % (uint64_t)(hi - lo + 1));
+  const uint64_t h = mix64(r);
+  if (mode == 1) e = ((h >> 1) & 1 ? edge : -edge) + (int)((h >> 2) % 9) - 4;
+  if (mode == 2) {
+    const int few = (int)((h >> 8) % 4);
+    m = few == 0 ? ((U)1 << B::mant) - 1 : (few == 1 ? ((U)1 << B::mant) - 1 - ((U)(h >> 16) & 7) : (few == 2 ? (U)(h >> 16) & 7 : (U)0));
+  }
+  int eb = e + B::bias;
+  if (mode == 3) {
+    const int kind = (int)(h % 8);
+    eb = kind == 6 ? B::emax : 0;
+    if (kind == 7) m = 0;
+    else if (kind == 6) m = (h >> 32) & 1 ? m : 0;
+    else m >>= (h >> 32) % B::mant;
+  }
+  eb = max(0, min(B::emax, eb));
+  return B::make(((U)(r >> 63) << (B::mant + (sizeof(R) == 8 ? 11 : 8))) | ((U)eb << B::mant) | m);
+}
+template <typename R>
+__device__ bool same_quotient(R q, R ref) {
+  return Bits<R>::get(q) == Bits<R>::get(ref) || (q == R(0) && ref == R(0)) || (q != q && ref != ref);
+}
+
+enum { Q_DIV_FAST = 0, Q_DIV_ANY, Q_RCP, Q_DIV3, Q_DIV6, Q_COUNT };
+// out: results that are neither flagged nor the quotient's bits; flagged results of
+// ordinary operands
+template <typename R>
+__global__ void k_quotients(int kind, long long n, uint64_t seed, unsigned long long *out, double *first) {
+  // edges of the flagged ranges (advect_fused.cuh): numerators of div_fast and
+  // div_3k, divisors (and numerators of div_any)
+  constexpr int ea = sizeof(R) == 8 ? 900 : 100, eb = sizeof(R) == 8 ? 500 : 60;
+  constexpr int ord = sizeof(R) == 8 ? 80 : 40;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const uint64_t r1 = mix64(seed ^ (uint64_t)(2 * i)), r2 = mix64(seed ^ (uint64_t)(2 * i + 1));
+    const int ma = (int)(i & 3), mb = (int)((i >> 2) & 3);
+    bool bad = false, plain = ma == 0 && mb == 0;
+    R a = special<R>(r1, ma, -ord, ord, kind == Q_DIV_ANY ? eb : ea), b, q, ref;
+    switch (kind) {
+      case Q_DIV_FAST:
+        // divisors that leave the quotient of an unflagged numerator normal
+        b = special<R>(r2, mb & 2, -20, 20, 0);
+        plain = ma == 0;
+        q = fesom::div_fast(a, b, R(1) / b, bad);
+        ref = a / b;
+        break;
+      case Q_DIV_ANY:
+        b = special<R>(r2, mb, -ord, ord, eb);
+        q = fesom::div_any(a, b, bad);
+        ref = a / b;
+        break;
+      case Q_RCP:
+        b = special<R>(r2, mb, -ord, ord, eb);
+        a = R(1);
+        plain = mb == 0;
+        q = fesom::rcp_exact(b, bad);
+        ref = R(1) / b;
+        break;
+      case Q_DIV3:
+        b = R(3);
+        plain = ma == 0;
+        q = fesom::div3(a, bad);
+        ref = a / b;
+        break;
+      default:
+        b = R(6);
+        plain = ma == 0;
+        q = fesom::div6(a, bad);
+        ref = a / b;
+        break;
+    }
+    if (bad && plain) atomicAdd(&out[1], 1ull);
+    if (!bad && !same_quotient(q, ref) && atomicAdd(&out[0], 1ull) == 0) {
+      first[0] = a; first[1] = b; first[2] = q; first[3] = ref;
     }
   }
 }
@@ -123,6 +226,30 @@ extern "C" int tracer_selftest_sround(int fmt, long long n, int draws, uint32_t 
   if (e != cudaSuccess) return -1;
   if (outside) *outside = (long long)bad;
   if (z) *z = acc[1] > 0.0 ? acc[0] / sqrt(acc[1]) : 0.0;
+  return 0;
+}
+
+extern "C" int tracer_selftest_quotients(int kind, int fp32, long long n, uint64_t seed, long long *wrong, long long *flagged,
+                                         double *example4) {
+  if (kind < 0 || kind >= Q_COUNT || n < 1) return -1;
+  unsigned long long *d = nullptr, h[2] = {0, 0};
+  double *d_first = nullptr, first[4] = {0, 0, 0, 0};
+  if (cudaMalloc(&d, sizeof(h)) != cudaSuccess) return -1;
+  if (cudaMalloc(&d_first, sizeof(first)) != cudaSuccess) { cudaFree(d); return -1; }
+  cudaMemset(d, 0, sizeof(h));
+  cudaMemset(d_first, 0, sizeof(first));
+  if (fp32) k_quotients<float><<<148 * 8, 256>>>(kind, n, seed, d, d_first);
+  else k_quotients<double><<<148 * 8, 256>>>(kind, n, seed, d, d_first);
+  cudaError_t e = cudaDeviceSynchronize();
+  if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(first, d_first, sizeof(first), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  cudaFree(d_first);
+  if (e != cudaSuccess) return -1;
+  if (wrong) *wrong = (long long)h[0];
+  if (flagged) *flagged = (long long)h[1];
+  if (example4)
+    for (int k = 0; k < 4; k++) example4[k] = first[k];
   return 0;
 }
 

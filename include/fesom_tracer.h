@@ -276,11 +276,21 @@ int tracer_set_device(int device);
 int tracer_launches_per_step(void);
 /* Device memory held by the engine, in bytes. */
 long long tracer_device_bytes(void);
-/* Checks on the GPU that the reciprocal-based division of the FP64 kernels
+/* Checks on the GPU that the reciprocal-based division of the fused patch kernel
  * returns the same bits as IEEE a / b for n random operand pairs;
  * *mismatches = number of differing results, example4 = (a, b, got,
  * expected) of the first one. */
 int tracer_selftest_division(long long n, uint64_t seed, long long *mismatches, double *example4);
+/* Checks on the GPU the straight-line divisions of the five step kernels on n
+ * operand pairs, in FP64 or FP32: kind 0 a / b given RN(1 / b), 1 a / b for any
+ * divisor, 2 1 / b, 3 a / 3, 4 a / 6.  A quarter of the operands each is ordinary,
+ * lies beside the edges of the ranges a kernel flags for a plain division, has
+ * (nearly) all-ones or all-zero significands, and is subnormal, zero, infinite or
+ * NaN.  *wrong = results not flagged whose bits differ from the IEEE quotient's
+ * (zeros of either sign are one), *flagged = results flagged though their operands
+ * were ordinary; example4 = (a, b, got, expected) of the first wrong one. */
+int tracer_selftest_quotients(int kind, int fp32, long long n, uint64_t seed, long long *wrong, long long *flagged,
+                              double *example4);
 /* Checks on the GPU the stochastic rounding of 16-bit stores (fmt 0 BF16,
  * 1 FP16) on n random inputs with `draws` roundings each: *outside = results
  * that are not one of the input's two storage neighbours; *z = standardized

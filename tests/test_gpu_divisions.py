@@ -1,5 +1,7 @@
-"""The step kernels' divisions: fields of subnormal values, whose high words are
-zero like a zero's."""
+"""The step kernels' divisions: the device functions on operands where they can go
+wrong, and fields of subnormal values, whose high words are zero like a zero's."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -25,3 +27,25 @@ def test_subnormal_fields(api, oracle, scale, scheme, path):
         run_both(api, m, [T, S], uv, w, dt, scheme, 3)
     finally:
         api.set_step_path("five")
+
+
+QUOTIENTS = ["div_fast", "div_any", "rcp", "div3", "div6"]
+
+
+def quotients(lib, kind, fp32, n, seed):
+    wrong, flagged, ex = ctypes.c_longlong(-1), ctypes.c_longlong(-1), np.zeros(4)
+    assert lib.tracer_selftest_quotients(QUOTIENTS.index(kind), fp32, n, seed, ctypes.byref(wrong), ctypes.byref(flagged),
+                                         ex.ctypes.data_as(ctypes.c_void_p)) == 0
+    return wrong.value, flagged.value, ex
+
+
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("kind", QUOTIENTS)
+def test_straight_line_quotients(lib, kind, fp32):
+    """Every result that is not flagged for a plain division is the IEEE quotient, on
+    2^26 operand pairs; ordinary operands are flagged only for a divisor whose
+    significand's high word (FP32: whole significand) is all ones, 1 in 2^20 (2^23)."""
+    n = 1 << 26
+    wrong, flagged, ex = quotients(lib, kind, fp32, n, 77 + fp32)
+    assert wrong == 0, f"a={ex[0]!r} b={ex[1]!r} got={ex[2]!r} expected={ex[3]!r}"
+    assert flagged <= (4 * n / 2 ** 20 if kind in ("div_any", "rcp") else 0)
