@@ -235,12 +235,15 @@ __device__ __forceinline__ bool not_zero(double a, unsigned u) { return (u | (un
 // numerators outside [2^-900, 2^900] other than zero set `bad` and the caller
 // divides again.  The sign of a zero result is not kept (no output of the step
 // depends on the sign of a zero quotient).
-__device__ __forceinline__ double div_fast(double a, double b, double y, bool &bad) {
+__device__ __forceinline__ double div_near(double a, double b, double y) {  // numerator known to be in range
   double q = a * y;
   q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+__device__ __forceinline__ double div_fast(double a, double b, double y, bool &bad) {
   const unsigned u = 2u * (unsigned)__double2hiint(a);
   bad |= (u - 0x0f600000u > 0xf0800000u - 0x0f600000u) && not_zero(a, u);
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
+  return div_near(a, b, y);
 }
 __device__ __forceinline__ float div_fast(float a, float b, float y, bool &bad) {
   float q = a * y;
@@ -253,7 +256,8 @@ __device__ __forceinline__ float div_fast(float a, float b, float y, bool &bad) 
 // RN(1 / b), straight-line: the hardware's approximate reciprocal refined by
 // Newton steps y += y (1 - b y), the last of which rounds correctly unless b's
 // significand is all ones (Markstein).  That significand, and magnitudes outside
-// [2^-500, 2^500] (FP32: [2^-60, 2^60]), set `bad`.
+// [2^-500, 2^500] (FP32: [2^-EXP, 2^EXP]: 2^60 where quotients are formed with it),
+// set `bad`.
 __device__ __forceinline__ double rcp_newton(double b) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));  // about 2^-20
@@ -266,11 +270,13 @@ __device__ __forceinline__ double rcp_exact(double b, bool &bad) {
   bad |= u - 0x41600000u > 0xbe600000u - 0x41600000u || ((unsigned)__double2hiint(b) | 0xfff00000u) == 0xffffffffu;
   return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
 }
+template <int EXP = 60>
 __device__ __forceinline__ float rcp_exact(float b, bool &bad) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));  // within a unit in the last place
+  constexpr unsigned lo = (unsigned)(127 - EXP) << 24, hi = (unsigned)(127 + EXP) << 24;
   const unsigned u = 2u * __float_as_uint(b);
-  bad |= u - 0x43000000u > 0xbb000000u - 0x43000000u || (__float_as_uint(b) | 0xff800000u) == 0xffffffffu;
+  bad |= u - lo > hi - lo || (__float_as_uint(b) | 0xff800000u) == 0xffffffffu;
   return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
 }
 // a / b for any divisor: the limiter ratios and the ring means.  Numerators below
@@ -417,28 +423,28 @@ __device__ __forceinline__ R div6(R x, bool &bad) { return div_3k<6>(x, bad); }
 template <typename R>
 __device__ __forceinline__ R div3(R x, bool &bad) { return div_3k<3>(x, bad); }
 
-// Reciprocals of the learned flux's features, straight-line: an approximate
-// reciprocal within a unit in the last place and one Newton step round 1 / x
-// (see div_any).
-__device__ __forceinline__ float rcp_newton(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return __fmaf_rn(__fmaf_rn(-x, y, 1.0f), y, y);
-}
+// Divisions of the learned flux's features, correctly rounded: straight-line, or
+// plain again for the lanes that set `bad`.
+struct FeatFast {
+  bool &bad;
+  __device__ __forceinline__ float rcp(float x) { return rcp_exact<100>(x, bad); }
+  __device__ __forceinline__ float div(float a, float b) { return div_fast(a, b, rcp_exact(b, bad), bad); }
+};
+struct FeatPlain {
+  __device__ __forceinline__ float rcp(float x) { return 1.0f / x; }
+  __device__ __forceinline__ float div(float a, float b) { return a / b; }
+};
 // Courant number of an edge level's volume flux in the upwind node's cell, of
 // volume vol; the same for every tracer.
-__device__ __forceinline__ float edge_courant(float vflux, float dt, float vol) {
-  bool bad = false;
-  const float num = fabsf(vflux) * dt;
-  float cour = div_fast(num, vol, rcp_newton(vol), bad);
-  if (bad) cour = num / vol;
-  return fminf(cour, 4.0f);
+template <typename D>
+__device__ __forceinline__ float edge_courant(float vflux, float dt, float vol, D d) {
+  return fminf(d.div(fabsf(vflux) * dt, vol), 4.0f);
 }
 
 // learned flux: 16 features of one MUSCL edge level in the flow's frame, in
 // units of the local variation sig, and the scale of the network's output
-template <typename TS>
-__device__ __forceinline__ void edge_features(const DMeshT<float> &m, const FusedArgs<float, TS> &a, int t, int cell,
+template <typename TS, typename D>
+__device__ __forceinline__ void edge_features(const DMeshT<float> &m, const FusedArgs<float, TS> &a, D d, int t, int cell,
                                               int k, float vflux, float cour, float t1, float t2, float x1, float x2, float Tmean1,
                                               float Tmean2, float gux, float guy, float gdx, float gdy, float exa,
                                               float eyr, float c_lo1, float c_lo2, bool shared) {
@@ -448,7 +454,7 @@ __device__ __forceinline__ void edge_features(const DMeshT<float> &m, const Fuse
   const float xu = fwd ? x1 : -x2, xd = fwd ? x2 : -x1;
   const float face = 0.5f * (Tmean1 + Tmean2);
   const float sig = fabsf(td - tu) + (fabsf(xu) + fabsf(xd)) * sixth + 1e-6f * (fabsf(tu) + fabsf(td)) + 1e-20f;
-  const float inv = rcp_newton(sig);
+  const float inv = d.rcp(sig);
   const float gx = fwd ? gux : gdx, gy = fwd ? guy : gdy;
   const float trans = (-eyr * gx + exa * gy) * inv;
   float f[16];
@@ -526,8 +532,8 @@ __device__ __noinline__ void edge_pair_slow(const DMeshT<R> &m, const FusedArgs<
       il<NT>(a.adf_h, t, o) = ho - flo;
       if constexpr (HOR == HOR_MUSCL_FEAT) {
         const cix ou = vf >= R(0) ? o1 : o2;
-        edge_features(m, a, t, m.edge_sched.cell_off[e] + k, k, vf,
-                      edge_courant(vf, a.dt, m.areasvol[ou] * m.hnode_new[ou]), b1, b2, x1, x2, Tmean1, Tmean2, gux, guy,
+        edge_features(m, a, FeatPlain{}, t, m.edge_sched.cell_off[e] + k, k, vf,
+                      edge_courant(vf, a.dt, m.areasvol[ou] * m.hnode_new[ou], FeatPlain{}), b1, b2, x1, x2, Tmean1, Tmean2, gux, guy,
                       gdx, gdy, g[12], g[13], c1, c2, k < x.tri_levels());
       }
     }
@@ -585,6 +591,7 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
         const cix ou = (vf[q] >= R(0) ? o1 : o2) + q;
         vol[q] = m.areasvol[ou] * m.hnode_new[ou];
       }
+      if (k + 1 >= x.levels()) vol[1] = R(1);  // dry
     }
 #pragma unroll
     for (int t0 = 0; t0 < NT; t0 += G) {
@@ -618,8 +625,8 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
       const R hph = R(0.5) * (R(1) - a.ph);
       [[maybe_unused]] R cour[2];
       if constexpr (HOR == HOR_MUSCL_FEAT) {
-        cour[0] = edge_courant(vf[0], a.dt, vol[0]);
-        cour[1] = edge_courant(vf[1], a.dt, vol[1]);
+        cour[0] = edge_courant(vf[0], a.dt, vol[0], FeatFast{bad});
+        cour[1] = edge_courant(k + 1 < x.levels() ? vf[1] : R(0), a.dt, vol[1], FeatFast{bad});
       }
       R out[2 * G];
 #pragma unroll
@@ -661,7 +668,7 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
           out[2 * i + q] = ho - flo;
           if constexpr (HOR == HOR_MUSCL_FEAT) {
             if (k + q < x.levels())
-              edge_features(m, a, t, cell + q, k + q, vf[q], cour[q], b1[i][q], b2[i][q], x1, x2, Tmean1, Tmean2, gux,
+              edge_features(m, a, FeatFast{bad}, t, cell + q, k + q, vf[q], cour[q], b1[i][q], b2[i][q], x1, x2, Tmean1, Tmean2, gux,
                             guy, gdx, gdy, exa, eyr, c1, c2, sh);
           }
         }
@@ -1142,12 +1149,23 @@ __global__ void __launch_bounds__(kColThreads, StepBlocks<R, NT>::col1)
 // ---------------------------------------------------------------------------
 // k_col2: bounds, in/out sums, ratios (lib/oce_adv_tra_fct.F90:105-374)
 // ---------------------------------------------------------------------------
-// Reciprocal for FP64 quotients that are rounded to FP32 afterwards: one Newton
-// step (error about 2^-40).
-__device__ __forceinline__ double rcp_newton1(double b) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+// Denominator of a limiter ratio, P dt / V +- eps (y = RN(1 / V)), and the ratio of
+// a bound q to it: FP64 quotients in every precision.  FP32 operands, products of two
+// of them and denominators of at least 1e-16 lie inside the exact range, or are not
+// finite: an infinite or NaN P leaves a NaN denominator, which rcp_exact flags.
+template <typename R>
+__device__ __forceinline__ double ratio_den(R P, R dt, R V, double y, double eps, bool &bad) {
+  if constexpr (sizeof(R) == 8) return div_fast(P * dt, V, y, bad) + eps;
+  else return div_near((double)P * (double)dt, (double)V, y) + eps;
+}
+template <typename R>
+__device__ __forceinline__ R ratio(R q, double den, bool &bad) {
+  if constexpr (sizeof(R) == 8) {
+    return fmin2(1.0, div_any(q, den, bad));
+  } else {
+    bad |= !(fabsf(q) < INFINITY);
+    return (R)fmin2(1.0, div_near((double)q, den, rcp_exact(den, bad)));
+  }
 }
 
 // FCT bounds of one cell from the ring elements, for nodes whose ring list is
@@ -1250,10 +1268,13 @@ __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R,
   ldv2(m.areasvol + o, asv);
   ldv2(m.rcp + o, yas);  // 1/areasvol plane (k_rcp_planes)
   if (k + 1 >= nln) asv[1] = yas[1] = R(1);  // dry
-  double dtv[2];
-  if constexpr (sizeof(R) == 4) {
-    dtv[0] = (double)a.dt * rcp_newton1((double)asv[0]);
-    dtv[1] = (double)a.dt * rcp_newton1((double)asv[1]);
+  // FP64 reciprocals of areasvol (FP64: the plane's)
+  bool badv = false;
+  double yv[2];
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    if constexpr (sizeof(R) == 8) yv[q] = yas[q];
+    else yv[q] = rcp_exact((double)asv[q], badv);
   }
   __syncwarp();
 #pragma unroll
@@ -1273,36 +1294,26 @@ __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R,
     }
     // R+ = min(1, bmax / (P+ dt / V + eps)), R- likewise; flux_eps is a
     // default-real literal.  In FP32 the denominators, where cancellation with it
-    // matters, and the quotients are formed in FP64.  A quotient of a positive
-    // denominator not above bmax is at least 1: where that holds for the warp (limiting
-    // is local) the FP32 kernels do not divide (FP64: the test costs more than it
-    // saves, 0.277 against 0.258 ms at 400x400x64).
+    // matters, and the quotients are formed in FP64 too.  A quotient of a positive
+    // denominator not above bmax is at least 1: a lane where that holds of all its
+    // quotients (limiting is local) does not divide in the FP32 kernels (FP64: the
+    // test costs more than it saves, 0.277 against 0.258 ms at 400x400x64).
     const double eps = (double)1e-16f;
-    bool bad = false, need = false;
+    bool bad = badv, need = false;
     double up[2], um[2];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const int i = 2 * t + q;
-      if constexpr (sizeof(R) == 8) {
-        up[q] = div_fast(fp[i] * a.dt, asv[q], yas[q], bad) + eps;
-        um[q] = div_fast(fm[i] * a.dt, asv[q], yas[q], bad) - eps;
-      } else {
-        up[q] = (double)fp[i] * dtv[q] + eps;
-        um[q] = (double)fm[i] * dtv[q] - eps;
-        bad |= !(fabs(up[q]) < 1e200) || !(fabs(um[q]) < 1e200);
-      }
+      up[q] = ratio_den(fp[i], a.dt, asv[q], yv[q], eps, bad);
+      um[q] = ratio_den(fm[i], a.dt, asv[q], yv[q], -eps, bad);
       out[2 * q] = out[2 * q + 1] = R(1);
       need |= k + q < nln && (!(up[q] > 0.0 && (double)bx[q] >= up[q]) || !(um[q] < 0.0 && (double)bn[q] <= um[q]));
     }
     if (sizeof(R) == 8 || need) {
-      auto div = [&](double x, double y) {
-        if constexpr (sizeof(R) == 8) return div_any(x, y, bad);
-        else return x * rcp_newton1(y);
-      };
 #pragma unroll
       for (int q = 0; q < 2; q++) {
-        out[2 * q] = (R)fmin2(1.0, div((double)bx[q], up[q]));
-        out[2 * q + 1] = (R)fmin2(1.0, div((double)bn[q], um[q]));
+        out[2 * q] = ratio(bx[q], up[q], bad);
+        out[2 * q + 1] = ratio(bn[q], um[q], bad);
       }
     }
     if (k + 1 >= nln) out[2] = out[3] = R(0);  // dry: read by k_col3 against a zero flux
@@ -1311,14 +1322,7 @@ __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R,
       if (bad) {
         for (int q = 0; q < 2; q++) {
           const int i = 2 * t + q;
-          double u, v;
-          if constexpr (sizeof(R) == 8) {
-            u = fp[i] * a.dt / asv[q];
-            v = fm[i] * a.dt / asv[q];
-          } else {
-            u = (double)fp[i] * (double)a.dt / (double)asv[q];
-            v = (double)fm[i] * (double)a.dt / (double)asv[q];
-          }
+          const double u = (double)fp[i] * (double)a.dt / (double)asv[q], v = (double)fm[i] * (double)a.dt / (double)asv[q];
           out[2 * q] = (R)fmin2(1.0, (double)bx[q] / (u + eps));
           out[2 * q + 1] = (R)fmin2(1.0, (double)bn[q] / (v - eps));
         }

@@ -99,7 +99,7 @@ __device__ bool same_quotient(R q, R ref) {
   return Bits<R>::get(q) == Bits<R>::get(ref) || (q == R(0) && ref == R(0)) || (q != q && ref != ref);
 }
 
-enum { Q_DIV_FAST = 0, Q_DIV_ANY, Q_RCP, Q_DIV3, Q_DIV6, Q_COUNT };
+enum { Q_DIV_FAST = 0, Q_DIV_ANY, Q_RCP, Q_DIV3, Q_DIV6, Q_RATIO, Q_COURANT, Q_SCALE, Q_COUNT };
 // out: results that are neither flagged nor the quotient's bits; flagged results of
 // ordinary operands
 template <typename R>
@@ -140,11 +140,45 @@ __global__ void k_quotients(int kind, long long n, uint64_t seed, unsigned long 
         q = fesom::div3(a, bad);
         ref = a / b;
         break;
-      default:
+      case Q_DIV6:
         b = R(6);
         plain = ma == 0;
         q = fesom::div6(a, bad);
         ref = a / b;
+        break;
+      case Q_RATIO: {
+        // min(1, a / (P dt / V + eps)) of values in the model's range: P and V of
+        // any significand, bounds from 2^-40 to 2 times the denominator
+        const double eps = (double)1e-16f;
+        const R dt = (R)(100.0 + (double)(r1 % 1000));
+        const R P = fabs(special<R>(r1, ma == 3 ? 3 : 0, -60, 30, 0)), V = fabs(special<R>(r2, mb & 2, 10, 40, 0));
+        const double den = (double)P * (double)dt / (double)V + eps;
+        a = (R)(den * ldexp(1.0 + (double)(mix64(r1) >> 12) * 0x1p-52, -(int)(mix64(r2) % 41)));
+        b = V;
+        const double y = sizeof(R) == 8 ? 1.0 / (double)V : fesom::rcp_exact((double)V, bad);
+        if (ma == 2 && mb == 3) a = R(mix64(r2) & 1 ? -INFINITY : INFINITY);
+        q = fesom::ratio(a, fesom::ratio_den(P, dt, V, y, eps, bad), bad);
+        ref = (R)fesom::fmin2(1.0, (double)a / den);
+        break;
+      }
+      default:
+        // the learned flux's Courant number and reciprocal variation (FP32 only)
+        if constexpr (sizeof(R) == 4) {
+          if (kind == Q_COURANT) {
+            b = fabsf(special<float>(r2, mb & 2, 10, 50, 0));
+            a = special<float>(r1, 0, -30, 30, 0);
+            q = fesom::edge_courant(a, 600.0f, b, fesom::FeatFast{bad});
+            ref = fminf(fabsf(a) * 600.0f / b, 4.0f);
+          } else {
+            b = fabsf(special<float>(r2, mb, -66, 30, 100));
+            a = 1.0f;
+            q = fesom::FeatFast{bad}.rcp(b);
+            ref = 1.0f / b;
+          }
+          plain = mb == 0;
+        } else {
+          a = b = q = ref = R(0);
+        }
         break;
     }
     if (bad && plain) atomicAdd(&out[1], 1ull);

@@ -283,7 +283,9 @@ long long tracer_device_bytes(void);
 int tracer_selftest_division(long long n, uint64_t seed, long long *mismatches, double *example4);
 /* Checks on the GPU the straight-line divisions of the five step kernels on n
  * operand pairs, in FP64 or FP32: kind 0 a / b given RN(1 / b), 1 a / b for any
- * divisor, 2 1 / b, 3 a / 3, 4 a / 6.  A quarter of the operands each is ordinary,
+ * divisor, 2 1 / b, 3 a / 3, 4 a / 6, 5 the FCT limiter's ratios (FP64 quotients
+ * in both), 6 and 7 the Courant number and reciprocal variation of the learned
+ * flux's features (FP32).  A quarter of the operands each is ordinary,
  * lies beside the edges of the ranges a kernel flags for a plain division, has
  * (nearly) all-ones or all-zero significands, and is subnormal, zero, infinite or
  * NaN.  *wrong = results not flagged whose bits differ from the IEEE quotient's

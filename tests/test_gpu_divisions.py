@@ -29,7 +29,7 @@ def test_subnormal_fields(api, oracle, scale, scheme, path):
         api.set_step_path("five")
 
 
-QUOTIENTS = ["div_fast", "div_any", "rcp", "div3", "div6"]
+QUOTIENTS = ["div_fast", "div_any", "rcp", "div3", "div6", "limiter_ratio", "courant", "variation"]
 
 
 def quotients(lib, kind, fp32, n, seed):
@@ -40,7 +40,7 @@ def quotients(lib, kind, fp32, n, seed):
 
 
 @pytest.mark.parametrize("fp32", [0, 1])
-@pytest.mark.parametrize("kind", QUOTIENTS)
+@pytest.mark.parametrize("kind", QUOTIENTS[:5])
 def test_straight_line_quotients(lib, kind, fp32):
     """Every result that is not flagged for a plain division is the IEEE quotient, on
     2^26 operand pairs; ordinary operands are flagged only for a divisor whose
@@ -49,3 +49,13 @@ def test_straight_line_quotients(lib, kind, fp32):
     wrong, flagged, ex = quotients(lib, kind, fp32, n, 77 + fp32)
     assert wrong == 0, f"a={ex[0]!r} b={ex[1]!r} got={ex[2]!r} expected={ex[3]!r}"
     assert flagged <= (4 * n / 2 ** 20 if kind in ("div_any", "rcp") else 0)
+
+
+@pytest.mark.parametrize("kind,fp32", [("limiter_ratio", 0), ("limiter_ratio", 1), ("courant", 1), ("variation", 1)])
+def test_quotients_of_the_limiter_and_the_features(lib, kind, fp32):
+    """FP64 quotients in the limiter ratios of every precision, IEEE quotients in the
+    learned flux's features: the bits of the same expressions with plain divisions."""
+    n = 1 << 26
+    wrong, flagged, ex = quotients(lib, kind, fp32, n, 5)
+    assert wrong == 0, f"a={ex[0]!r} b={ex[1]!r} got={ex[2]!r} expected={ex[3]!r}"
+    assert flagged <= 4 * n / 2 ** 20
