@@ -579,7 +579,7 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
       st_pair_il<NT, 1>(a.adf_h, t, o, out);
     }
   } else {
-    bool bad = false;
+    bool bad[2] = {false, false};  // of each level: a dry second one has no say
     // the loads of G tracers are all issued before the first is used
     constexpr int G = NT > 2 ? 2 : NT;
     [[maybe_unused]] int cell = 0;
@@ -591,7 +591,6 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
         const cix ou = (vf[q] >= R(0) ? o1 : o2) + q;
         vol[q] = m.areasvol[ou] * m.hnode_new[ou];
       }
-      if (k + 1 >= x.levels()) vol[1] = R(1);  // dry
     }
 #pragma unroll
     for (int t0 = 0; t0 < NT; t0 += G) {
@@ -625,8 +624,8 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
       const R hph = R(0.5) * (R(1) - a.ph);
       [[maybe_unused]] R cour[2];
       if constexpr (HOR == HOR_MUSCL_FEAT) {
-        cour[0] = edge_courant(vf[0], a.dt, vol[0], FeatFast{bad});
-        cour[1] = edge_courant(k + 1 < x.levels() ? vf[1] : R(0), a.dt, vol[1], FeatFast{bad});
+        cour[0] = edge_courant(vf[0], a.dt, vol[0], FeatFast{bad[0]});
+        cour[1] = edge_courant(vf[1], a.dt, vol[1], FeatFast{bad[1]});
       }
       R out[2 * G];
 #pragma unroll
@@ -655,11 +654,11 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
           const R x1 = R(2) * (b2[i][q] - b1[i][q]) + exa * gux + eyr * guy;
           R Tmean2, Tmean1;
           if (HOR != HOR_MFCT) {
-            Tmean2 = b2[i][q] - div6(x2, bad) * c2;
-            Tmean1 = b1[i][q] + div6(x1, bad) * c1;
+            Tmean2 = b2[i][q] - div6(x2, bad[q]) * c2;
+            Tmean1 = b1[i][q] + div6(x1, bad[q]) * c1;
           } else {
-            Tmean2 = b2[i][q] - div6(x2, bad);
-            Tmean1 = b1[i][q] + div6(x1, bad);
+            Tmean2 = b2[i][q] - div6(x2, bad[q]);
+            Tmean1 = b1[i][q] + div6(x1, bad[q]);
           }
           const R vp = vf[q] + fabs(vf[q]), vm = vf[q] - fabs(vf[q]);
           const R cHO = vp * Tmean1 + vm * Tmean2;
@@ -668,7 +667,7 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
           out[2 * i + q] = ho - flo;
           if constexpr (HOR == HOR_MUSCL_FEAT) {
             if (k + q < x.levels())
-              edge_features(m, a, FeatFast{bad}, t, cell + q, k + q, vf[q], cour[q], b1[i][q], b2[i][q], x1, x2, Tmean1, Tmean2, gux,
+              edge_features(m, a, FeatFast{bad[q]}, t, cell + q, k + q, vf[q], cour[q], b1[i][q], b2[i][q], x1, x2, Tmean1, Tmean2, gux,
                             guy, gdx, gdy, exa, eyr, c1, c2, sh);
           }
         }
@@ -679,7 +678,7 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
         for (int i = 0; i < G; i++) out[2 * i + 1] = R(0);
       st_pair_il<NT, G>(a.adf_h, t0, o, out);
     }
-    if (bad) edge_pair_slow<R, TS, NT, HOR, LIM>(m, a, e, k);
+    if (bad[0] || (bad[1] && k + 1 < x.levels())) edge_pair_slow<R, TS, NT, HOR, LIM>(m, a, e, k);
   }
 }
 
@@ -962,7 +961,7 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
     });
   }
 
-  bool bad = false;
+  bool bad[2] = {false, false};  // of each level: a dry second one has no say
   R hov[2 * G], lov[G][2];
 #pragma unroll
   for (int t = 0; t < G; t++)
@@ -1020,10 +1019,10 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
         const R aL = pos ? tv[q + 1] : tv[q];
         const R aR = pos ? (kk == nln - 1 ? x[t][q + 1] : tv[q + 2]) : tv[q + 1];
         R d;
-        if constexpr (UNI) d = div_fast(w * a.dt, pos ? h[q + 1] : h[q], pos ? yh[q + 1] : yh[q], bad);
+        if constexpr (UNI) d = div_fast(w * a.dt, pos ? h[q + 1] : h[q], pos ? yh[q + 1] : yh[q], bad[q]);
         else d = w * a.dt / (pos ? h[q + 1] : h[q]);
         const R cx = pos ? fmin2(d, R(1)) : fmin2(-d, R(1));
-        const R f = ppm_face(w, Tc, aL, aR, cx, [&](R z) { return div6(z, bad); });
+        const R f = ppm_face(w, Tc, aL, aR, cx, [&](R z) { return div6(z, bad[q]); });
         R v = f * A[q] * w - lov[t][q];
         if (!pos && !(w < R(0))) v = R(0) - lov[t][q];
         if (kk == 0) v = -(tv[1 + q] * w * A[q]) - lov[t][q];
@@ -1039,7 +1038,7 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
     for (int t = 0; t < G; t++) {
       R g[4];
 #pragma unroll
-      for (int q = 0; q < 2; q++) g[1 + q] = div_fast(x[t][q] - x[t][q + 1], zd[q], yz[q], bad);
+      for (int q = 0; q < 2; q++) g[1 + q] = div_fast(x[t][q] - x[t][q + 1], zd[q], yz[q], bad[q]);
       g[0] = __shfl_up_sync(kFull, g[2], 1);
       g[3] = __shfl_down_sync(kFull, g[1], 1);
 #pragma unroll
@@ -1051,8 +1050,8 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
         if (kk == 0) v = -(T1 * w * A[q]) - v;
         if (kk == 1) v = mid - v;
         if (kk == nln - 1) v = mid - v;
-        const R m1 = T1 + div3((R(2) * g[1 + q] + g[2 + q]) * za[q], bad);
-        const R m2 = T0 + div3((R(2) * g[1 + q] + g[q]) * zb[q], bad);
+        const R m1 = T1 + div3((R(2) * g[1 + q] + g[2 + q]) * za[q], bad[q]);
+        const R m2 = T0 + div3((R(2) * g[1 + q] + g[q]) * zb[q], bad[q]);
         const R tm = (w + fabs(w)) * m1 + (w - fabs(w)) * m2;
         const R f = (-(R(0.5) * (R(1) - a.pv) * tm) - a.pv * (R(0.5) * (m1 + m2)) * w) * A[q] - v;
         if (kk >= 2 && kk <= nln - 2) v = f;
@@ -1091,7 +1090,7 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
     ldv2(m.hnT + oh, hn);
     ldv2(m.yhnT + oh, yhn);
     ldv2(m.hT + oh, h);
-    bool badl = false;
+    bool badl[2] = {false, false};
 #pragma unroll
     for (int t = 0; t < G; t++) {
       const R dn = __shfl_down_sync(kFull, lov[t][0], 1);
@@ -1099,17 +1098,17 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
       for (int q = 0; q < 2; q++) {
         const R f1 = q == 0 ? lov[t][1] : (k + 2 >= nln ? R(0) : dn);
         acc[t][q] = (acc[t][q] + (lov[t][q] - f1)) * a.dt;
-        const R num = ts[t][1 + q] * h[q] + div_fast(acc[t][q], asv[q], yas[q], badl);
-        out[2 * t + q] = div_fast(num, hn[q], yhn[q], badl);
+        const R num = ts[t][1 + q] * h[q] + div_fast(acc[t][q], asv[q], yas[q], badl[q]);
+        out[2 * t + q] = div_fast(num, hn[q], yhn[q], badl[q]);
       }
     }
-    if (badl) {
+    if (badl[0] || (badl[1] && k + 1 < nln)) {
       for (int t = 0; t < G; t++)
         for (int q = 0; q < 2; q++) out[2 * t + q] = (ts[t][1 + q] * h[q] + acc[t][q] / asv[q]) / hn[q];
     }
     if (st) st_pair_il<NT, G>(a.lo, t0, o, out);
   }
-  if (bad && st) col1_vert_slow<R, TS, NT, G, VER, LIM>(m, a, t0, n, k);
+  if (st && (bad[0] || (bad[1] && k + 1 < nln))) col1_vert_slow<R, TS, NT, G, VER, LIM>(m, a, t0, n, k);
 }
 
 // The column pairs of `per` consecutive warps of the schedule, one after the
@@ -1269,12 +1268,12 @@ __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R,
   ldv2(m.rcp + o, yas);  // 1/areasvol plane (k_rcp_planes)
   if (k + 1 >= nln) asv[1] = yas[1] = R(1);  // dry
   // FP64 reciprocals of areasvol (FP64: the plane's)
-  bool badv = false;
+  bool badv[2] = {false, false};
   double yv[2];
 #pragma unroll
   for (int q = 0; q < 2; q++) {
     if constexpr (sizeof(R) == 8) yv[q] = yas[q];
-    else yv[q] = rcp_exact((double)asv[q], badv);
+    else yv[q] = rcp_exact((double)asv[q], badv[q]);
   }
   __syncwarp();
 #pragma unroll
@@ -1299,27 +1298,27 @@ __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R,
     // quotients (limiting is local) does not divide in the FP32 kernels (FP64: the
     // test costs more than it saves, 0.277 against 0.258 ms at 400x400x64).
     const double eps = (double)1e-16f;
-    bool bad = badv, need = false;
+    bool bad[2] = {badv[0], badv[1]}, need = false;  // bad of each level: a dry second one has no say
     double up[2], um[2];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const int i = 2 * t + q;
-      up[q] = ratio_den(fp[i], a.dt, asv[q], yv[q], eps, bad);
-      um[q] = ratio_den(fm[i], a.dt, asv[q], yv[q], -eps, bad);
+      up[q] = ratio_den(fp[i], a.dt, asv[q], yv[q], eps, bad[q]);
+      um[q] = ratio_den(fm[i], a.dt, asv[q], yv[q], -eps, bad[q]);
       out[2 * q] = out[2 * q + 1] = R(1);
       need |= k + q < nln && (!(up[q] > 0.0 && (double)bx[q] >= up[q]) || !(um[q] < 0.0 && (double)bn[q] <= um[q]));
     }
     if (sizeof(R) == 8 || need) {
 #pragma unroll
       for (int q = 0; q < 2; q++) {
-        out[2 * q] = ratio(bx[q], up[q], bad);
-        out[2 * q + 1] = ratio(bn[q], um[q], bad);
+        out[2 * q] = ratio(bx[q], up[q], bad[q]);
+        out[2 * q + 1] = ratio(bn[q], um[q], bad[q]);
       }
     }
     if (k + 1 >= nln) out[2] = out[3] = R(0);  // dry: read by k_col3 against a zero flux
     if (l.stores()) {
       stv4(a.rpm[t0 + t] + 2 * (size_t)o, out);
-      if (bad) {
+      if (bad[0] || (bad[1] && k + 1 < nln)) {
         for (int q = 0; q < 2; q++) {
           const int i = 2 * t + q;
           const double u = (double)fp[i] * (double)a.dt / (double)asv[q], v = (double)fm[i] * (double)a.dt / (double)asv[q];
@@ -1393,7 +1392,7 @@ __device__ __forceinline__ void col3_store(const FusedArgs<R, TS> &a, int t, cix
   }
 }
 
-// A pair's update with the divisions `div` (the fast ones, or plain ones again
+// A pair's update with the divisions `div` of each level (the fast ones, or plain ones again
 // for the lanes whose operands lie outside their range).
 template <typename R, typename TS, int NT, int G, int LIM, typename D>
 __device__ __forceinline__ void col3_update(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, int n, int k, const NodeRec &rec,
@@ -1433,14 +1432,13 @@ __device__ __forceinline__ void col3_update(const DMeshT<R> &m, const FusedArgs<
           const R p = fmin2(rs[t][2 * q], ro[t][2 * q + 1]), r = fmin2(rs[t][2 * q + 1], ro[t][2 * q]);
           g = (g >= R(0) ? p : r) * g;
         }
-        dh[t][q] = dh[t][q] + div(g * a.dt, asv[q], yas[q]);
+        dh[t][q] = dh[t][q] + div(g * a.dt, asv[q], yas[q], q);
       }
   });
 #pragma unroll
   for (int t = 0; t < G; t++) {
     R tt[2];
     ld_pair_T(a.T[t0 + t], o, a.off[t0 + t], tt);
-    if (k + 1 >= nln) tt[1] = R(0);  // dry, whatever the cell holds
     R fv[3];
     const R a2 = k + 2 < nln ? il<NT>(a.adf_v, t0 + t, o + 2) : R(0);
     if (LIM == LIM_FCT) {
@@ -1459,9 +1457,9 @@ __device__ __forceinline__ void col3_update(const DMeshT<R> &m, const FusedArgs<
     for (int q = 0; q < 2; q++) {
       R dv = R(0);
       if (LIM == LIM_FCT) dv = dv - tt[q] * h[q] + lo[2 * t + q] * hn[q];
-      dv = dv + div((fv[q] - fv[q + 1]) * a.dt, asv[q], yas[q]);
+      dv = dv + div((fv[q] - fv[q + 1]) * a.dt, asv[q], yas[q], q);
       const R del = R(0) + dh[t][q] + dv;
-      out[t][q] = tt[q] + div(del, hn[q], yhn[q]);
+      out[t][q] = tt[q] + div(del, hn[q], yhn[q], q);
     }
   }
 }
@@ -1470,7 +1468,7 @@ template <typename R, typename TS, int NT, int G, int LIM>
 __device__ __noinline__ void col3_pair_slow(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, int n, int k) {
   const NodeRec rec = node_rec(m, n);
   R out[G][2];
-  col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [](R x, R y, R) { return x / y; }, out);
+  col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [](R x, R y, R, int) { return x / y; }, out);
   for (int t = 0; t < G; t++) col3_store<R, TS, NT>(a, t0 + t, (cix)n * m.S + k, min(rec.nlev() - 1 - k, 2), out[t]);
 }
 
@@ -1480,10 +1478,10 @@ __device__ __forceinline__ void col3_pair(const DMeshT<R> &m, const FusedArgs<R,
   const int n = l.item, k = l.k();
   const NodeRec rec = node_rec(m, n);
   const int wet = min(rec.nlev() - 1 - k, 2);
-  bool bad = false;
+  bool bad[2] = {false, false};  // of each level: a dry second one has no say
   R out[G][2];
-  col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [&](R x, R y, R z) { return div_fast(x, y, z, bad); }, out);
-  if (bad) {
+  col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [&](R x, R y, R z, int q) { return div_fast(x, y, z, bad[q]); }, out);
+  if (bad[0] || (bad[1] && wet == 2)) {
     col3_pair_slow<R, TS, NT, G, LIM>(m, a, t0, n, k);
     return;
   }
