@@ -799,7 +799,10 @@ __global__ void k_level_tables(DMeshT<R> m, int n, R *t) {
     if (m.uniform_h && k >= 2 && k <= nln - 2) ppm_face_weights(HN[k - 2], HN[k - 1], HN[k], HN[k + 1], f);
     for (int i = 0; i < 3; i++) t[(LT_C1 + i) * S + k] = c[i];
     for (int i = 0; i < 5; i++) t[(LT_A + i) * S + k] = f[i];
-    t[LT_YH * S + k] = m.uniform_h && k < nln ? R(1) / H[k] : R(0);
+    // NaN: a thickness that div_fast has no quotient for (k_col1 divides again)
+    constexpr R big = sizeof(R) == 8 ? R(0x1p500) : R(0x1p60f);
+    const R h = m.uniform_h && k < nln ? H[k] : R(1);
+    t[LT_YH * S + k] = fabs(h) >= 1 / big && fabs(h) <= big ? (k < nln ? R(1) / h : R(0)) : R(NAN);
     const bool in = k >= 1 && k < m.nl - 1;
     const R zd = in ? m.Z[k - 1] - m.Z[k] : R(1);
     t[LT_ZD * S + k] = zd;
@@ -977,6 +980,8 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
       ldv2(lt + LT_D * S, fD); ldv2(lt + LT_E * S, fE);
       h[0] = m.hT[km]; ldv2(m.hT + k, h + 1);
       yh[0] = m.ltab[LT_YH * S + km]; ldv2(lt + LT_YH * S, yh + 1);
+      bad[0] = yh[0] != yh[0] || yh[1] != yh[1];
+      bad[1] = yh[1] != yh[1] || yh[2] != yh[2];
     } else {
       const R *HN = m.hnode_new + col, *H = m.hnode + col;
       const R z[5] = {HN[max(k - 2, 0)], HN[km], HN[k], HN[k + 1], HN[kp]};

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import pyoracle
-from test_gpu_pairs import run_both
+from test_gpu_pairs import array_mesh, run_both
 from test_gpu_parity import synth_case
 
 pytestmark = pytest.mark.gpu
@@ -59,3 +59,24 @@ def test_quotients_of_the_limiter_and_the_features(lib, kind, fp32):
     wrong, flagged, ex = quotients(lib, kind, fp32, n, 5)
     assert wrong == 0, f"a={ex[0]!r} b={ex[1]!r} got={ex[2]!r} expected={ex[3]!r}"
     assert flagged <= 4 * n / 2 ** 20
+
+
+@pytest.mark.parametrize("h", [0.0, 5e-324, 1e-200, 1e200])
+@pytest.mark.parametrize("scheme", [("MUSCL", "PPM", "FCT"), ("MUSCL", "PPM", "NONE"), ("MFCT", "QR4C", "FCT")])
+def test_layers_of_extreme_thickness(api, oracle, h, scheme):
+    """One old thickness (hnode, the divisor of PPM's Courant number) of zero, a
+    subnormal and far outside any ocean, the same at every node, so that the level
+    tables hold: the oracle's bits."""
+    K, uv, w, T, S, dt = synth_case(api, 13, 12, 21, True, 9)
+    names = ["elem2D_nodes", "edges", "edge_tri", "nlevels", "nlevels_nod2D", "ring_num", "ring_elem", "elem_area", "area",
+             "areasvol", "edge_dxdy", "edge_cross_dxdy", "gradient_sca", "zbar", "hnode", "hnode_new", "helem", "coord"]
+    arrays = {n: api.mesh_array(n) for n in names}
+    arrays["elem_cos"] = np.ones(api.mesh_dims()["elem2D"])
+    flat = np.array(arrays["hnode"])
+    layers = flat.reshape(-1, 20)  # 20 layers of each node one after the other
+    layers[:, 2] = h
+    layers[:, 5] = h
+    arrays["hnode"] = layers.reshape(arrays["hnode"].shape)
+    m = array_mesh(api, oracle, arrays, 1.0e5, 1.0e5)
+    with np.errstate(all="ignore"):
+        run_both(api, m, [T, S], uv, w, dt, scheme, 1)
