@@ -840,9 +840,17 @@ void capture_separate(BatchImpl &B) {
   CK(cudaStreamBeginCapture(B.stream, cudaStreamCaptureModeRelaxed));
   CK(cudaEventRecord(B.sep_events[M], B.stream));
   for (size_t m = 0; m < M; m++) CK(cudaStreamWaitEvent((cudaStream_t)B.members[m]->stream(), B.sep_events[M], 0));
-  for (auto &m : B.members) m->impl()->pdl = false;  // forked streams: plain dependencies
-  separate_steps_direct(B, 2);
-  for (auto &m : B.members) m->impl()->pdl = true;
+  {
+    struct PlainLaunches {  // forked streams: plain dependencies while they are captured
+      BatchImpl &B;
+      explicit PlainLaunches(BatchImpl &b) : B(b) { set(false); }
+      ~PlainLaunches() { set(true); }
+      void set(bool on) {
+        for (auto &m : B.members) m->impl()->pdl = on;
+      }
+    } plain(B);
+    separate_steps_direct(B, 2);
+  }
   for (size_t m = 0; m < M; m++) {
     CK(cudaEventRecord(B.sep_events[m], (cudaStream_t)B.members[m]->stream()));
     CK(cudaStreamWaitEvent(B.stream, B.sep_events[m], 0));
@@ -855,8 +863,8 @@ void capture_separate(BatchImpl &B) {
 }
 
 // Changes to the separate path, and takes one step of `nsteps` directly where
-// that must come first: it allocates the work arrays and fills the edge volume
-// fluxes, which no capture or replay may do, or swaps the buffers back to those
+// that must come first: it allocates the work arrays (the learned flux's features
+// among them) and fills the edge volume fluxes, which no capture or replay may do, or swaps the buffers back to those
 // the graph was captured with.  Returns the steps left.
 int begin_separate(BatchImpl &B, int nsteps, bool use_graph, bool always) {
   if (!B.configured) throw std::runtime_error("configure the batch first");
@@ -867,7 +875,10 @@ int begin_separate(BatchImpl &B, int nsteps, bool use_graph, bool always) {
     B.separate = true;
   }
   bool direct = always || (B.sep_exec && B.sep_key != first_buffer(B));
-  for (auto &m : B.members) direct = direct || !m->impl()->vflux_valid || m->impl()->slots < kNT;
+  for (auto &m : B.members) {
+    const EngineImpl &P = *m->impl();
+    direct = direct || !P.vflux_valid || P.slots < kNT || (B.sch.hor == HOR_MUSCL && !learned_buffers_ready(P, kNT));
+  }
   if (nsteps > 0 && (direct || !use_graph)) {
     separate_steps_direct(B, 1);
     nsteps--;

@@ -211,5 +211,7 @@ void learned_correct_f32(EngineImpl &P, int nt, const FusedArgs<float, float> &a
 void learned_release(EngineImpl &P);
 bool learned_active(const EngineImpl &P);
 void learned_slot_buffers(EngineImpl &P, int t, void **feat, void **scale);
+// whether a MUSCL batch of nt tracers runs without allocating feature buffers
+bool learned_buffers_ready(const EngineImpl &P, int nt);
 
 }  // namespace fesom

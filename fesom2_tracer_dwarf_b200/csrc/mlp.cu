@@ -914,6 +914,12 @@ void learned_slot_buffers(EngineImpl &P, int t, void **feat, void **scale) {
   *feat = L.feat[t];
   *scale = L.fscale[t];
 }
+bool learned_buffers_ready(const EngineImpl &P, int nt) {
+  if (!learned_active(P)) return true;
+  for (int t = 0; t < nt; t++)
+    if (!P.learn->feat[t]) return false;
+  return true;
+}
 bool learned_active(const EngineImpl &P) { return P.learn && P.learn->on; }
 
 void Engine::set_learned(const float *params, bool on) {
