@@ -68,9 +68,13 @@ size_t batch_smem() {
 
 // prefix: PH_COUNT rows of (ntasks + 1) running totals of each task's blocks;
 // wave_first: (nwaves + 1) first task of each wave (tasks are wave-major).
-// MINB: resident 256-thread blocks per SM the register budget is cut for
-template <int HOR, int VER, int LIM, int MINB>
-__global__ void __launch_bounds__(256, MINB)
+// One register budget, of 16 resident warps per SM (128 registers): four FP32 tracers
+// a lane do not fit fewer.  Builds for 3 to 7 blocks of 256 threads spilled 740 to
+// 6,212 bytes and were slower at every size of grid (three members of 100x100x20 to
+// 240x240x40, 8 tracers: 1.12 ms a step at 2 blocks per SM, 1.32 / 1.75 / 2.65 / 3.39 /
+// 4.21 at 3 to 7), so a tile that asks for more runs as many blocks as are resident.
+template <int HOR, int VER, int LIM>
+__global__ void __launch_bounds__(256, 2)
     k_batch_step(BatchTask *tasks, const int *prefix, int ntasks, const int *wave_first, int nwaves, GridBarrier *bar,
                  long long spin_limit, int refresh_ab) {
   extern __shared__ __align__(16) int smem[];
@@ -121,24 +125,12 @@ __global__ void __launch_bounds__(256, MINB)
 
 using BatchKernel = void (*)(BatchTask *, const int *, int, const int *, int, GridBarrier *, long long, int);
 
-template <int MINB>
-BatchKernel pick_kernel_b(const TracerScheme &s) {
-  if (s.hor == HOR_MUSCL && s.ver == VER_PPM && s.lim == LIM_FCT) return k_batch_step<HOR_MUSCL, VER_PPM, LIM_FCT, MINB>;
-  if (s.hor == HOR_MUSCL && s.ver == VER_PPM && s.lim == LIM_NONE) return k_batch_step<HOR_MUSCL, VER_PPM, LIM_NONE, MINB>;
-  if (s.hor == HOR_UPW1 && s.ver == VER_UPW1 && s.lim == LIM_FCT) return k_batch_step<HOR_UPW1, VER_UPW1, LIM_FCT, MINB>;
-  if (s.hor == HOR_UPW1 && s.ver == VER_UPW1 && s.lim == LIM_NONE) return k_batch_step<HOR_UPW1, VER_UPW1, LIM_NONE, MINB>;
+BatchKernel pick_kernel(const TracerScheme &s) {
+  if (s.hor == HOR_MUSCL && s.ver == VER_PPM && s.lim == LIM_FCT) return k_batch_step<HOR_MUSCL, VER_PPM, LIM_FCT>;
+  if (s.hor == HOR_MUSCL && s.ver == VER_PPM && s.lim == LIM_NONE) return k_batch_step<HOR_MUSCL, VER_PPM, LIM_NONE>;
+  if (s.hor == HOR_UPW1 && s.ver == VER_UPW1 && s.lim == LIM_FCT) return k_batch_step<HOR_UPW1, VER_UPW1, LIM_FCT>;
+  if (s.hor == HOR_UPW1 && s.ver == VER_UPW1 && s.lim == LIM_NONE) return k_batch_step<HOR_UPW1, VER_UPW1, LIM_NONE>;
   return nullptr;
-}
-
-// the register budget follows the resident threads per SM the tile asks for
-BatchKernel pick_kernel(const TracerScheme &s, int threads = 256, int blocks_per_sm = 2) {
-  const int minb = std::max(2, std::min(7, (threads * blocks_per_sm + 255) / 256));
-  if (minb == 7) return pick_kernel_b<7>(s);
-  if (minb == 6) return pick_kernel_b<6>(s);
-  if (minb == 5) return pick_kernel_b<5>(s);
-  if (minb == 4) return pick_kernel_b<4>(s);
-  if (minb == 3) return pick_kernel_b<3>(s);
-  return pick_kernel_b<2>(s);
 }
 
 // One persistent launch per phase: the launch walks the blocks of every task
@@ -514,7 +506,7 @@ void Batch::set_tile(const BatchTile &tile) {
     B.separate = false;
   }
   B.tile = tile;
-  B.kernel = pick_kernel(B.sch, tile.threads, tile.blocks_per_sm);
+  B.kernel = pick_kernel(B.sch);
   phase_kernels(B.sch, B.phk);
   const size_t smem = batch_smem();
   CK(cudaFuncSetAttribute(B.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
