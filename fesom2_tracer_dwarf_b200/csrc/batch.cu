@@ -497,6 +497,8 @@ void Batch::set_tile(const BatchTile &tile) {
   if (!B.configured) throw std::runtime_error("configure the batch first");
   if (tile.threads < 64 || tile.threads > 256 || tile.threads % 32) throw std::invalid_argument("threads per block in {64..256}");
   if (tile.wave < 1) throw std::invalid_argument("wave must be >= 1");
+  if (tile.cells_per_block < 32 || tile.cells_per_block > kMaxCellsPerBlock)
+    throw std::invalid_argument("cells per block must be in [32, 576]");
   for (auto &m : B.members) m->synchronize();
   CK(cudaStreamSynchronize(B.stream));
   B.release();
@@ -517,8 +519,6 @@ void Batch::set_tile(const BatchTile &tile) {
   B.grid = B.sms * B.tile.blocks_per_sm;
 
   const int M = num_members();
-  for (int m = 0; m < M; m++) B.members[m]->set_cells_per_block(tile.cells_per_block);
-
   // work arrays per (member, wave slot) and the task table, wave-major
   int max_batches = 0;
   for (int m = 0; m < M; m++) max_batches = std::max(max_batches, B.ntr[m] / kNT);
@@ -934,76 +934,75 @@ std::string Batch::autotune(int steps_per_candidate) {
   int max_batches = 0;
   for (int m = 0; m < num_members(); m++) max_batches = std::max(max_batches, B.ntr[m] / kNT);
   int best_mode = B.mode;
-  for (int cells : {256, 384, 512}) {
+  const int cells = B.tile.cells_per_block;  // no step path reads it
+  {
+    // per-member launches: no part of the tile applies
+    BatchTile t;
+    t.cells_per_block = cells;
+    t.wave = 1;
+    set_tile(t);
+    B.mode = 2;
+    const double ms = time_steps(steps_per_candidate, false) / steps_per_candidate;
+    log << "path=separate ms_per_step=" << ms << "\n";
+    if (ms < best_ms) {
+      best_ms = ms;
+      best = B.tile;
+      best_mode = 2;
+    }
+  }
+  for (int wave : {1, 2, 4}) {
+    if (B.learned) break;  // the persistent paths have no MLP phase
+    if (wave > max_batches && wave != 1) continue;
+    // one launch per phase: the tile's threads and blocks per SM do not apply
     {
-      // per-member launches: only the cells per block of the members apply
       BatchTile t;
       t.cells_per_block = cells;
-      t.wave = 1;
-      set_tile(t);
-      B.mode = 2;
-      const double ms = time_steps(steps_per_candidate, false) / steps_per_candidate;
-      log << "path=separate cells=" << cells << " ms_per_step=" << ms << "\n";
-      if (ms < best_ms) {
-        best_ms = ms;
-        best = B.tile;
-        best_mode = 2;
+      t.wave = wave;
+      bool ok = true;
+      try {
+        set_tile(t);
+      } catch (const std::exception &e) {
+        cudaGetLastError();
+        log << "path=phases wave=" << wave << " skipped: " << e.what() << "\n";
+        ok = false;
+      }
+      if (ok) {
+        B.mode = 1;
+        time_steps(1, false);  // warm-up
+        const double ms = time_steps(steps_per_candidate, false) / steps_per_candidate;
+        log << "path=phases wave=" << B.tile.wave << " ms_per_step=" << ms << "\n";
+        if (ms < best_ms) {
+          best_ms = ms;
+          best = B.tile;
+          best_mode = 1;
+        }
       }
     }
-    for (int wave : {1, 2, 4}) {
-      if (B.learned) break;  // the persistent paths have no MLP phase
-      if (wave > max_batches && wave != 1) continue;
-      // one launch per phase: the tile's threads and blocks per SM do not apply
-      {
+    for (int threads : {128, 256}) {
+      for (int bps : {2, 3, 4}) {
         BatchTile t;
         t.cells_per_block = cells;
         t.wave = wave;
-        bool ok = true;
+        t.threads = threads;
+        t.blocks_per_sm = bps;
         try {
           set_tile(t);
         } catch (const std::exception &e) {
           cudaGetLastError();
-          log << "path=phases cells=" << cells << " wave=" << wave << " skipped: " << e.what() << "\n";
-          ok = false;
+          log << "path=cooperative wave=" << wave << " threads=" << threads << " bps=" << bps << " skipped: " << e.what()
+              << "\n";
+          continue;
         }
-        if (ok) {
-          B.mode = 1;
-          time_steps(1, false);  // warm-up
-          const double ms = time_steps(steps_per_candidate, false) / steps_per_candidate;
-          log << "path=phases cells=" << cells << " wave=" << B.tile.wave << " ms_per_step=" << ms << "\n";
-          if (ms < best_ms) {
-            best_ms = ms;
-            best = B.tile;
-            best_mode = 1;
-          }
-        }
-      }
-      for (int threads : {128, 256}) {
-        for (int bps : {2, 3, 4, 5, 6, 8, 10}) {
-          BatchTile t;
-          t.cells_per_block = cells;
-          t.wave = wave;
-          t.threads = threads;
-          t.blocks_per_sm = bps;
-          try {
-            set_tile(t);
-          } catch (const std::exception &e) {
-            cudaGetLastError();
-            log << "path=cooperative cells=" << cells << " wave=" << wave << " threads=" << threads << " bps=" << bps
-                << " skipped: " << e.what() << "\n";
-            continue;
-          }
-          if (B.tile.blocks_per_sm != bps) continue;  // occupancy cap: same as a smaller candidate
-          B.mode = 0;
-          time_steps(1, false);  // warm-up
-          const double ms = time_steps(steps_per_candidate, false) / steps_per_candidate;
-          log << "path=cooperative cells=" << cells << " wave=" << B.tile.wave << " threads=" << threads
-              << " bps=" << bps << " ms_per_step=" << ms << "\n";
-          if (ms < best_ms) {
-            best_ms = ms;
-            best = B.tile;
-            best_mode = 0;
-          }
+        if (B.tile.blocks_per_sm != bps) continue;  // occupancy cap: same as a smaller candidate
+        B.mode = 0;
+        time_steps(1, false);  // warm-up
+        const double ms = time_steps(steps_per_candidate, false) / steps_per_candidate;
+        log << "path=cooperative wave=" << B.tile.wave << " threads=" << threads << " bps=" << bps << " ms_per_step=" << ms
+            << "\n";
+        if (ms < best_ms) {
+          best_ms = ms;
+          best = B.tile;
+          best_mode = 0;
         }
       }
     }
@@ -1023,7 +1022,6 @@ std::string Batch::autotune(int steps_per_candidate) {
   set_tile(best);
   B.mode = best_mode;
   log << "best: path=" << (best_mode == 2 ? "separate" : best_mode == 1 ? "phases" : "cooperative")
-      << " cells=" << best.cells_per_block
       << " wave=" << best.wave << " threads=" << best.threads << " bps=" << best.blocks_per_sm
       << " ms_per_step=" << best_ms << "\n";
   return log.str();

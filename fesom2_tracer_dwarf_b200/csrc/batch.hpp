@@ -3,7 +3,7 @@
 //
 // Every member is an FP32 Engine that owns its mesh, velocity and tracers.
 // Two step paths walk the same work list of (member, 4-tracer batch, block
-// of wet cells) items phase by phase -- ring-mean gradients, edge fluxes,
+// of level pairs) items phase by phase -- ring-mean gradients, edge fluxes,
 // vertical fluxes and low-order solution, FCT bounds and ratios, limiting and
 // update.  Path 0: ONE persistent cooperative launch per step, a grid-wide
 // barrier between phases; the kernel swaps the new and old tracer buffers in
@@ -16,9 +16,8 @@
 // independent slots share the SMs); two steps are captured as one CUDA
 // graph.  Tracer batches run in waves of a bounded number per member
 // so the work arrays stay small; every member's edge volume fluxes are
-// computed once per velocity.  An autotuner picks the path and the tile (wet
-// cells per block, i.e. nodes per block x levels), the threads per block and
-// persistent grid size of path 0, and the number of tracer batches in
+// computed once per velocity.  An autotuner picks the path, the threads per block
+// and persistent grid size of path 0, and the number of tracer batches in
 // flight.
 #pragma once
 #include <memory>
@@ -30,9 +29,9 @@
 namespace fesom {
 
 struct BatchTile {
-  int cells_per_block = 512;  // schedule tile (wet cells per block)
+  int cells_per_block = 512;  // checked and kept, but no step path has such a tile
   int threads = 256;          // threads per block
-  int blocks_per_sm = 2;      // persistent grid = SMs x this
+  int blocks_per_sm = 2;      // persistent grid = SMs x this (at most what is resident)
   int wave = 3;               // 4-tracer batches in flight per member
 };
 
