@@ -73,8 +73,8 @@ R *upload_conv(EngineImpl &P, const std::vector<double> &h) {
   return P.upload(st);
 }
 
-// Work schedules (node and edge cells, of the learned flux) for a cap on the wet
-// cells per block; the arrays of a previous tiling are released.
+// Work schedules (node and edge cells, of the learned flux alone) for a cap on the
+// wet cells per block; the arrays of a previous tiling are released.
 template <typename R>
 void build_schedules(EngineImpl &P, DMeshT<R> &d, int cells_per_block) {
   const MeshHost &M = P.mesh;
@@ -97,123 +97,250 @@ void build_schedules(EngineImpl &P, DMeshT<R> &d, int cells_per_block) {
   d.edge_sched.nblk = (int)blk.size() - 1;
 }
 
+// ---- records and pair schedules ------------------------------------------------
+// Formed on the device from the mesh arrays already there.  On the host, and copied,
+// they cost 0.75 of 5.7 s of an engine at 1000x1000x64 (FP64).
+
+int blocks_for(long long threads) { return (int)std::max<long long>(1, std::min<long long>((threads + 255) / 256, 148 * 32)); }
+
 // Levels of an edge whose up and down triangles are both there and wet.
-int edge_tri_levels(const MeshHost &M, int e) {
-  if (M.up_dn_tri[2 * e] < 0 || M.up_dn_tri[2 * e + 1] < 0) return 0;
-  return std::max(0, std::min(M.nlev_node_min[M.edge_nodes[2 * e]], M.nlev_node_min[M.edge_nodes[2 * e + 1]]) - 1);
-}
-
-DPairs upload_pairs(EngineImpl &P, const std::vector<int> &item, const std::vector<unsigned short> &lev) {
-  DPairs d;
-  d.item = P.upload(item);
-  d.lev = P.upload(lev);
-  d.nwarps = (int)(item.size() / 32);
-  return d;
-}
-
-// Pair schedule of the edges, run by run of slots: the pairs with both triangles
-// at every wet level, then the others.
-DPairs build_edge_pairs(EngineImpl &P) {
-  const MeshHost &M = P.mesh;
-  const int E = M.edge2D, run = 2048;
-  std::vector<int> item;
-  std::vector<unsigned short> lev;
-  size_t pairs = 0;
-  for (int e = 0; e < E; e++) pairs += (M.edge_levels(e) + 1) / 2;
-  item.reserve(pairs + 128 * ((size_t)E / run + 1));
-  lev.reserve(item.capacity());
-  for (int s0 = 0; s0 < E; s0 += run)
-    for (unsigned ring = 0; ring <= kPairRing; ring += kPairRing) {
-      for (int s = s0; s < std::min(E, s0 + run); s++) {
-        const int e = P.slot_edge[s], nl = M.edge_levels(e), tri = edge_tri_levels(M, e);
-        for (int k = 0; k < nl; k += 2) {
-          if ((std::min(k + 2, nl) > tri) != (ring != 0)) continue;
-          item.push_back(s);
-          lev.push_back((unsigned short)(ring | k));
-        }
-      }
-      while (item.size() % 32) {
-        item.push_back(item.back());
-        lev.push_back((unsigned short)kPairNone);
-      }
-    }
-  return upload_pairs(P, item, lev);
-}
-
-// Pair schedule of the ring-mean gradients: an edge uses its nodes' ring means from
-// level edge_tri_levels down.
-DPairs build_grad_pairs(EngineImpl &P) {
-  const MeshHost &M = P.mesh;
-  const int N = M.nod2D;
-  std::vector<int> lev0(N), item;
-  std::vector<unsigned short> lev;
-  for (int n = 0; n < N; n++) lev0[n] = std::max(0, M.nlev_node[n] - 1);
-  for (int e = 0; e < M.edge2D; e++) {
-    const int thr = edge_tri_levels(M, e);
-    for (int q = 0; q < 2; q++) {
-      int &l = lev0[M.edge_nodes[2 * (size_t)e + q]];
-      l = std::min(l, thr);
-    }
-  }
-  for (int n = 0; n < N; n++)
-    for (int k = lev0[n] / 2 * 2; lev0[n] < M.nlev_node[n] - 1 && k < M.nlev_node[n] - 1; k += 2) {
-      item.push_back(n);
-      lev.push_back((unsigned short)k);
-    }
-  while (item.size() % 32) {
-    item.push_back(item.back());
-    lev.push_back((unsigned short)kPairNone);
-  }
-  return upload_pairs(P, item, lev);
-}
-
-// Element records of the ring means (DMeshT::elem_idx, elem_geo).
 template <typename R>
-void build_elem_records(EngineImpl &P, DMeshT<R> &d) {
-  const MeshHost &M = P.mesh;
-  const int T = M.elem2D, S = P.S;
-  std::vector<int4> idx(T);
-  std::vector<R> geo(8 * (size_t)T, R(0));
-  for (int e = 0; e < T; e++) {
-    const int *en = &M.elem_nodes[3 * (size_t)e];
-    idx[e] = make_int4(en[0] * S, en[1] * S, en[2] * S, M.nlev_elem[e] - 1);
-    for (int q = 0; q < 6; q++) geo[8 * (size_t)e + q] = (R)M.grad_sca[6 * (size_t)e + q];
-    geo[8 * (size_t)e + 6] = (R)M.elem_area[e];
-  }
-  d.elem_idx = P.upload(idx);
-  d.elem_geo = P.upload(geo);
+__device__ __forceinline__ int edge_tri_levels(const DMeshT<R> &m, int s) {
+  const int2 ud = m.up_dn[s], nn = m.edge_nodes[s];
+  if (ud.x < 0 || ud.y < 0) return 0;
+  return max(0, min(m.nlev_node_min[nn.x], m.nlev_node_min[nn.y]) - 1);
 }
 
 // Per-edge records of k_edge (DMeshT::edge_idx, edge_geo).
 template <typename R>
-void build_edge_records(EngineImpl &P, DMeshT<R> &d) {
-  const MeshHost &M = P.mesh;
-  const int E = M.edge2D, S = P.S;
-  std::vector<int4> idx(3 * (size_t)E);
-  std::vector<R> geo(16 * (size_t)E, R(0));
-  for (int s = 0; s < E; s++) {
-    const int e = P.slot_edge[s], n1 = M.edge_nodes[2 * e], n2 = M.edge_nodes[2 * e + 1];
-    const int u = M.up_dn_tri[2 * e], w = M.up_dn_tri[2 * e + 1];
-    const bool pair = u >= 0 && w >= 0;
-    int un[3] = {n1, n1, n1}, dn[3] = {n2, n2, n2};
-    R *g = &geo[16 * (size_t)s];
-    if (pair)
+__global__ void k_edge_records(DMeshT<R> m, int4 *idx, R *geo) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < m.E; s += gridDim.x * blockDim.x) {
+    const int2 nn = m.edge_nodes[s], ud = m.up_dn[s];
+    const bool pair = ud.x >= 0 && ud.y >= 0;
+    int un[3] = {nn.x, nn.x, nn.x}, dn[3] = {nn.y, nn.y, nn.y};
+    R *g = geo + 16 * (size_t)s;
+    for (int q = 0; q < 16; q++) g[q] = R(0);
+    if (pair) {
       for (int q = 0; q < 3; q++) {
-        un[q] = M.elem_nodes[3 * (size_t)u + q];
-        dn[q] = M.elem_nodes[3 * (size_t)w + q];
+        un[q] = m.elem_nodes[3 * (size_t)ud.x + q];
+        dn[q] = m.elem_nodes[3 * (size_t)ud.y + q];
       }
-    for (int q = 0; pair && q < 6; q++) {
-      g[q] = (R)M.grad_sca[6 * (size_t)u + q];
-      g[6 + q] = (R)M.grad_sca[6 * (size_t)w + q];
+      for (int q = 0; q < 6; q++) {
+        g[q] = m.grad_sca[6 * (size_t)ud.x + q];
+        g[6 + q] = m.grad_sca[6 * (size_t)ud.y + q];
+      }
     }
-    g[12] = (R)M.edge_dxdy[2 * (size_t)e] * (R)M.edge_a[e];
-    g[13] = (R)M.edge_dxdy[2 * (size_t)e + 1] * (R)kREarthD;
-    idx[3 * (size_t)s] = make_int4(n1 * S, n2 * S, un[0] * S, un[1] * S);
-    idx[3 * (size_t)s + 1] = make_int4(un[2] * S, dn[0] * S, dn[1] * S, dn[2] * S);
-    idx[3 * (size_t)s + 2] = make_int4(edge_tri_levels(M, e), M.nboundary_lay[n1], M.nboundary_lay[n2], M.edge_levels(e));
+    g[12] = m.edge_dxdy[2 * (size_t)s] * m.edge_a[s];
+    g[13] = m.edge_dxdy[2 * (size_t)s + 1] * (R)kREarthD;
+    idx[3 * (size_t)s] = make_int4(nn.x * m.S, nn.y * m.S, un[0] * m.S, un[1] * m.S);
+    idx[3 * (size_t)s + 1] = make_int4(un[2] * m.S, dn[0] * m.S, dn[1] * m.S, dn[2] * m.S);
+    idx[3 * (size_t)s + 2] = make_int4(edge_tri_levels(m, s), m.nbl[nn.x], m.nbl[nn.y], m.edge_lev[s].y);
   }
-  d.edge_idx = P.upload(idx);
-  d.edge_geo = P.upload(geo);
+}
+
+// Element records of the ring means (DMeshT::elem_idx, elem_geo).
+template <typename R>
+__global__ void k_elem_records(DMeshT<R> m, int4 *idx, R *geo) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m.T; e += gridDim.x * blockDim.x) {
+    const int *en = m.elem_nodes + 3 * (size_t)e;
+    R *g = geo + 8 * (size_t)e;
+    idx[e] = make_int4(en[0] * m.S, en[1] * m.S, en[2] * m.S, m.nlev_elem[e] - 1);
+    for (int q = 0; q < 6; q++) g[q] = m.grad_sca[6 * (size_t)e + q];
+    g[6] = m.elem_area[e];
+    g[7] = R(0);
+  }
+}
+
+// Node records of the column kernels (DMeshT::nrec, ne6); holds: elements of each node
+template <typename R>
+__global__ void k_holds(DMeshT<R> m, int *holds) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 3ll * m.T; i += (long long)gridDim.x * blockDim.x)
+    atomicAdd(&holds[m.elem_nodes[i]], 1);
+}
+template <typename R>
+__global__ void k_node_records(DMeshT<R> m, const int *holds, int4 *rec, int4 *ne) {
+  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < m.N; n += gridDim.x * blockDim.x) {
+    const int p0 = m.ne_ptr[n], deg = m.ne_ptr[n + 1] - p0;
+    const bool full = m.ring_ptr[n + 1] - m.ring_ptr[n] == holds[n];
+    unsigned lev[2] = {0, 0}, r[12];
+    for (int i = 0; i < 6; i++) {
+      r[2 * i] = 0;
+      r[2 * i + 1] = (unsigned)n * (unsigned)m.S;
+      if (i >= deg) continue;
+      const int4 q = m.ne4[p0 + i];
+      r[2 * i] = (unsigned)(q.x >> 1) * (unsigned)m.S;
+      r[2 * i + 1] = (unsigned)q.w | (unsigned)(q.x & 1) << 31;
+      lev[i / 3] |= (unsigned)q.z << (10 * (i % 3));
+    }
+    rec[n] = make_int4(m.nlev_node[n] | deg << 16, (int)((unsigned)m.nlev_node_min[n] | (full ? 0x80000000u : 0u)), (int)lev[0],
+                       (int)lev[1]);
+    for (int i = 0; i < 3; i++)
+      ne[3 * (size_t)n + i] = make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]);
+  }
+}
+
+template <typename R>
+void build_records(EngineImpl &P, DMeshT<R> &d) {
+  const MeshHost &M = P.mesh;
+  for (int n = 0; n < M.nod2D; n++)
+    if (M.node_edge_ptr[n + 1] - M.node_edge_ptr[n] > 0xffff) throw std::invalid_argument("a node has more than 65535 edges");
+  int4 *eidx = P.dalloc<int4>(3 * (size_t)d.E), *tidx = P.dalloc<int4>(d.T), *nrec = P.dalloc<int4>(d.N),
+       *ne6 = P.dalloc<int4>(3 * (size_t)d.N);
+  R *egeo = P.dalloc<R>(16 * (size_t)d.E), *tgeo = P.dalloc<R>(8 * (size_t)d.T);
+  int *holds = P.dalloc<int>(d.N);
+  k_edge_records<R><<<blocks_for(d.E), 256, 0, P.stream>>>(d, eidx, egeo);
+  k_elem_records<R><<<blocks_for(d.T), 256, 0, P.stream>>>(d, tidx, tgeo);
+  k_holds<R><<<blocks_for(3ll * d.T), 256, 0, P.stream>>>(d, holds);
+  k_node_records<R><<<blocks_for(d.N), 256, 0, P.stream>>>(d, holds, nrec, ne6);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(P.stream));
+  P.dfree(holds);
+  P.bytes -= (size_t)d.N * sizeof(int);
+  d.edge_idx = eidx;
+  d.edge_geo = egeo;
+  d.elem_idx = tidx;
+  d.elem_geo = tgeo;
+  d.nrec = nrec;
+  d.ne6 = ne6;
+}
+
+// A schedule's arrays on the device: every lane without a pair, of item 0, until it
+// is filled.
+struct PairArrays {
+  int *item;
+  unsigned short *lev;
+  PairArrays(EngineImpl &P, long long entries) {
+    item = P.dalloc<int>(entries);
+    lev = P.dalloc<unsigned short>(entries);
+    if (entries) CK(cudaMemsetAsync(lev, 0xff, entries * sizeof(unsigned short), P.stream));
+  }
+  DPairs pairs(long long entries) const { return DPairs{item, lev, (int)(entries / 32)}; }
+};
+
+// Pair schedule of the edges, run by run of slots: the pairs with both triangles
+// at every wet level, then the others.  A block takes a run: with `base` null it counts
+// the pairs of both kinds, otherwise it writes them from base[2 run], base[2 run + 1].
+constexpr int kPairRun = 2048, kPairThreads = 256, kPairEach = kPairRun / kPairThreads;
+template <typename R>
+__global__ void __launch_bounds__(kPairThreads) k_edge_pairs(DMeshT<R> m, const int *base, int *count, int *item,
+                                                            unsigned short *lev) {
+  __shared__ int off[kPairRun], part[kPairThreads];
+  const int s0 = blockIdx.x * kPairRun, ns = min(m.E - s0, kPairRun), tid = threadIdx.x;
+  // pairs of edge s with both triangles at every wet level, and the others
+  auto pairs = [&](int s, int kind) {
+    const int nl = m.edge_lev[s].y, tri = edge_tri_levels(m, s), all = (nl + 1) / 2, both = tri >= nl ? all : tri / 2;
+    return kind == 0 ? both : all - both;
+  };
+  for (int kind = 0; kind < 2; kind++) {
+    int c[kPairEach], sum = 0;
+    for (int i = 0; i < kPairEach; i++) {
+      const int j = tid * kPairEach + i;
+      c[i] = j < ns ? pairs(s0 + j, kind) : 0;
+      sum += c[i];
+    }
+    part[tid] = sum;
+    __syncthreads();
+    for (int w = 1; w < kPairThreads; w *= 2) {  // inclusive sums
+      const int v = tid >= w ? part[tid - w] : 0;
+      __syncthreads();
+      part[tid] += v;
+      __syncthreads();
+    }
+    const int total = part[kPairThreads - 1];
+    if (!base) {
+      if (tid == 0) count[2 * blockIdx.x + kind] = total;
+      __syncthreads();
+      continue;
+    }
+    int o = part[tid] - sum;
+    for (int i = 0; i < kPairEach; i++) {
+      off[tid * kPairEach + i] = o;
+      o += c[i];
+    }
+    __syncthreads();
+    const size_t b = base[2 * blockIdx.x + kind];
+    for (int j = tid / 32; j < ns; j += kPairThreads / 32) {
+      const int n = (j + 1 < ns ? off[j + 1] : total) - off[j], all = (m.edge_lev[s0 + j].y + 1) / 2;
+      const int first = kind == 0 ? 0 : all - n;
+      for (int q = tid % 32; q < n; q += 32) {
+        item[b + off[j] + q] = s0 + j;
+        lev[b + off[j] + q] = (unsigned short)((kind ? kPairRing : 0u) | (unsigned)(2 * (first + q)));
+      }
+    }
+    // lanes without a pair hold the run's last edge
+    if (total > 0 && tid < (32 - total % 32) % 32) item[b + total + tid] = s0 + ns - 1;
+    __syncthreads();
+  }
+}
+template <typename R>
+DPairs build_edge_pairs(EngineImpl &P, const DMeshT<R> &d) {
+  const int runs = (d.E + kPairRun - 1) / kPairRun;
+  if (runs == 0) return DPairs{};
+  int *dev = P.dalloc<int>(2 * (size_t)runs);
+  std::vector<int> n(2 * (size_t)runs);
+  k_edge_pairs<R><<<runs, kPairThreads, 0, P.stream>>>(d, nullptr, dev, nullptr, nullptr);
+  CK(cudaGetLastError());
+  P.d2h(n.data(), dev, n.size() * sizeof(int));
+  long long total = 0;
+  for (int &x : n) {
+    const int c = (x + 31) / 32 * 32;
+    x = (int)total;
+    total += c;
+  }
+  const PairArrays a(P, total);
+  P.h2d(dev, n.data(), n.size() * sizeof(int));
+  k_edge_pairs<R><<<runs, kPairThreads, 0, P.stream>>>(d, dev, nullptr, a.item, a.lev);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(P.stream));
+  P.dfree(dev);
+  P.bytes -= n.size() * sizeof(int);
+  return a.pairs(total);
+}
+
+// Pair schedule of the ring-mean gradients: an edge uses its nodes' ring means from
+// level edge_tri_levels down.  first: each node's first such level.
+template <typename R>
+__global__ void k_grad_first(DMeshT<R> m, int *first) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < m.E; s += gridDim.x * blockDim.x) {
+    const int2 nn = m.edge_nodes[s];
+    const int tri = edge_tri_levels(m, s);
+    atomicMin(&first[nn.x], tri);
+    atomicMin(&first[nn.y], tri);
+  }
+}
+__global__ void k_grad_pairs(int N, const int *first, const int *off, int *item, unsigned short *lev) {
+  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x)
+    for (int i = off[n]; i < off[n + 1]; i++) {
+      item[i] = n;
+      lev[i] = (unsigned short)(first[n] / 2 * 2 + 2 * (i - off[n]));
+    }
+}
+template <typename R>
+DPairs build_grad_pairs(EngineImpl &P, const DMeshT<R> &d) {
+  const MeshHost &M = P.mesh;
+  const int N = M.nod2D;
+  std::vector<int> first(N), off(N + 1, 0);
+  for (int n = 0; n < N; n++) first[n] = std::max(0, M.nlev_node[n] - 1);
+  int *df = P.upload(first);
+  k_grad_first<R><<<blocks_for(d.E), 256, 0, P.stream>>>(d, df);
+  CK(cudaGetLastError());
+  P.d2h(first.data(), df, (size_t)N * sizeof(int));
+  long long total = 0;
+  for (int n = 0; n < N; n++) {
+    const int last = M.nlev_node[n] - 1;
+    if (first[n] < last) total += (last - first[n] / 2 * 2 + 1) / 2;
+    off[n + 1] = (int)total;
+  }
+  total = (total + 31) / 32 * 32;
+  const PairArrays a(P, total);
+  int *doff = P.upload(off);
+  k_grad_pairs<<<blocks_for(N), 256, 0, P.stream>>>(N, df, doff, a.item, a.lev);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(P.stream));
+  P.dfree(df);
+  P.dfree(doff);
+  P.bytes -= (2 * (size_t)N + 1) * sizeof(int);
+  return a.pairs(total);
 }
 
 // Pair schedule of the columns.  A warp takes whole columns, so that their
@@ -223,97 +350,90 @@ void build_edge_records(EngineImpl &P, DMeshT<R> &d) {
 // nodes instead of their own was slower too).  Columns
 // of more than 32 pairs are cut into pieces that overlap by one pair at each cut
 // (halo lanes: computed, not stored).
+//
+// A piece as the device fills it in: x node, y first entry, z first pair | pairs << 16,
+// w 1: its first pair is a halo, 2: its last, 4: nothing follows it in its warp.
+__global__ void k_node_pairs(int npieces, const int4 *pieces, int *item, unsigned short *lev) {
+  const int lane = threadIdx.x & 31;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < npieces; i += (gridDim.x * blockDim.x) >> 5) {
+    const int4 c = pieces[i];
+    const int first = c.z & 0xffff, n = c.z >> 16, e = c.y + lane;
+    if (lane < n) {
+      const bool halo = ((c.w & 1) && lane == 0) || ((c.w & 2) && lane == n - 1);
+      item[e] = c.x;
+      lev[e] = (unsigned short)((halo ? kPairHalo : 0u) | (unsigned)(2 * (first + lane)));
+    } else if ((c.w & 4) && e / 32 == c.y / 32) {
+      item[e] = c.x;  // lanes without a pair
+    }
+  }
+}
 DPairs build_node_pairs(EngineImpl &P) {
   const MeshHost &M = P.mesh;
-  struct Piece {
-    int node, first, n;  // pairs
-    bool lo, hi;         // its first / last pair is a halo
-  };
   const int N = M.nod2D, window = 256;
-  std::vector<int> item;
-  std::vector<unsigned short> lev;
-  std::vector<Piece> pieces;
-  std::vector<std::vector<int>> by_n(33), warps, open(33);
+  std::vector<int4> pieces;  // in the order of the entries
+  pieces.reserve(N);
+  long long warps = 0;
+  // one window: its pieces by length, the pieces of each warp, and the warps by free lanes
+  struct Piece {
+    int node, first, n, halo, next;
+  };
+  std::vector<Piece> w;
+  std::vector<int> by_n[33], open[33], head, tail;
   for (int n0 = 0; n0 < N; n0 += window) {
-    pieces.clear();
-    warps.clear();
-    for (auto &v : by_n) v.clear();
-    for (auto &v : open) v.clear();
+    w.clear();
+    head.clear();
+    tail.clear();
+    for (int i = 0; i <= 32; i++) {
+      by_n[i].clear();
+      open[i].clear();
+    }
     for (int n = n0; n < std::min(N, n0 + window); n++) {
       const int np = M.nlev_node[n] / 2;  // pairs of nlev - 1 layers
       for (int p = 0; p < np;) {
         const bool lo = p > 0;
         const int left = np - p + (lo ? 1 : 0);  // with the leading halo
-        const Piece c{n, lo ? p - 1 : 0, std::min(left, 32), lo, left > 32};
-        p = c.first + c.n - (c.hi ? 1 : 0);
-        by_n[c.n].push_back((int)pieces.size());
-        pieces.push_back(c);
+        const bool hi = left > 32;
+        const Piece c{n, lo ? p - 1 : 0, std::min(left, 32), (lo ? 1 : 0) | (hi ? 2 : 0), -1};
+        p = c.first + c.n - (hi ? 1 : 0);
+        by_n[c.n].push_back((int)w.size());
+        w.push_back(c);
       }
     }
     for (int n = 32; n >= 1; n--)
       for (int i : by_n[n]) {
         int r = n;
         while (r <= 32 && open[r].empty()) r++;
-        int w;
+        int k;
         if (r > 32) {
-          w = (int)warps.size();
-          warps.emplace_back();
+          k = (int)head.size();
+          head.push_back(i);
+          tail.push_back(i);
           r = 32;
         } else {
-          w = open[r].back();
+          k = open[r].back();
           open[r].pop_back();
+          w[tail[k]].next = i;
+          tail[k] = i;
         }
-        warps[w].push_back(i);
-        if (r - n > 0) open[r - n].push_back(w);
+        if (r - n > 0) open[r - n].push_back(k);
       }
-    for (auto &w : warps) {
-      for (int i : w) {
-        const Piece &c = pieces[i];
-        for (int q = 0; q < c.n; q++) {
-          const bool halo = (c.lo && q == 0) || (c.hi && q == c.n - 1);
-          item.push_back(c.node);
-          lev.push_back((unsigned short)((halo ? kPairHalo : 0u) | (unsigned)(2 * (c.first + q))));
-        }
-      }
-      while (item.size() % 32) {
-        item.push_back(item.back());
-        lev.push_back((unsigned short)kPairNone);
+    for (size_t k = 0; k < head.size(); k++) {
+      int e = (int)(32 * (warps + (long long)k));
+      for (int i = head[k]; i >= 0; i = w[i].next) {
+        pieces.push_back(make_int4(w[i].node, e, w[i].first | w[i].n << 16, w[i].halo | (w[i].next < 0 ? 4 : 0)));
+        e += w[i].n;
       }
     }
+    warps += (long long)head.size();
   }
-  return upload_pairs(P, item, lev);
-}
-
-// Node records of the column kernels (DMeshT::nrec, ne6).
-template <typename R>
-void build_node_records(EngineImpl &P, DMeshT<R> &d, const std::vector<int> &edge_slot) {
-  const MeshHost &M = P.mesh;
-  const int N = M.nod2D, S = P.S;
-  std::vector<int> holds(N, 0);
-  for (int e = 0; e < M.elem2D; e++)
-    for (int q = 0; q < 3; q++) holds[M.elem_nodes[3 * (size_t)e + q]]++;
-  std::vector<int4> rec(N), ne(3 * (size_t)N);
-  for (int n = 0; n < N; n++) {
-    const int p0 = M.node_edge_ptr[n], deg = M.node_edge_ptr[n + 1] - p0;
-    const bool full = (M.ring_ptr[n + 1] - M.ring_ptr[n]) == holds[n];
-    if (deg > 0xffff) throw std::invalid_argument("a node has more than 65535 edges");
-    unsigned lev[2] = {0, 0}, r[12];
-    for (int i = 0; i < 6; i++) {
-      r[2 * i] = 0;
-      r[2 * i + 1] = (unsigned)n * (unsigned)S;
-      if (i >= deg) continue;
-      const int code = M.node_edge[p0 + i], e = code >> 1, second = code & 1;
-      r[2 * i] = (unsigned)edge_slot[e] * (unsigned)S;
-      r[2 * i + 1] = (unsigned)M.edge_nodes[2 * (size_t)e + (second ? 0 : 1)] * (unsigned)S | (unsigned)second << 31;
-      lev[i / 3] |= (unsigned)M.edge_levels(e) << (10 * (i % 3));
-    }
-    rec[n] = make_int4(M.nlev_node[n] | deg << 16, (int)((unsigned)M.nlev_node_min[n] | (full ? 0x80000000u : 0u)), (int)lev[0],
-                       (int)lev[1]);
-    for (int i = 0; i < 3; i++)
-      ne[3 * (size_t)n + i] = make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]);
-  }
-  d.nrec = P.upload(rec);
-  d.ne6 = P.upload(ne);
+  const PairArrays a(P, 32 * warps);
+  int4 *dp = P.upload(pieces);
+  k_node_pairs<<<blocks_for(32ll * (long long)pieces.size()), 256, 0, P.stream>>>((int)pieces.size(), dp, a.item, a.lev);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(P.stream));
+  P.dfree(dp);
+  P.bytes -= pieces.size() * sizeof(int4);
+  return a.pairs(32 * warps);
 }
 
 template <typename R>
@@ -323,6 +443,8 @@ void build_dmesh(EngineImpl &P, DMeshT<R> &d, const std::vector<int> &slot_edge,
   d.N = N; d.T = T; d.E = E; d.nl = nl; d.S = P.S;
   std::vector<int2> en(E), et(E), el(E), ud(E);
   std::vector<double> ecross(4 * (size_t)E), edxdy(2 * (size_t)E), ea(E);
+  for (int n = 0; n < N; n++)
+    if (M.nlev_node[n] - 1 > kMaxCellsPerBlock) throw std::runtime_error("a column or edge has more levels than a block holds");
   for (int s = 0; s < E; s++) {
     const int e = slot_edge[s];
     en[s] = make_int2(M.edge_nodes[2 * e], M.edge_nodes[2 * e + 1]);
@@ -368,12 +490,9 @@ void build_dmesh(EngineImpl &P, DMeshT<R> &d, const std::vector<int> &slot_edge,
   d.hnode_new = upload_cols<R>(P, M.hnode_new.data(), L, N, L);
   d.helem = upload_cols<R>(P, M.helem.data(), L, T, L);
 
-  build_schedules(P, d, kCellsPerBlock);
-  build_edge_records(P, d);
-  d.edge_pairs = build_edge_pairs(P);
-  build_elem_records(P, d);
-  d.grad_pairs = build_grad_pairs(P);
-  build_node_records(P, d, edge_slot);
+  build_records(P, d);
+  d.edge_pairs = build_edge_pairs(P, d);
+  d.grad_pairs = build_grad_pairs(P, d);
   d.node_pairs = build_node_pairs(P);
 }
 
@@ -419,20 +538,8 @@ void build_tiles(EngineImpl &P, const std::vector<int> &edge_slot, int owned) {
 
 static_assert(Engine::kDefaultCellsPerBlock == kCellsPerBlock, "one default schedule tile");
 
-bool uniform_levels(const MeshHost &M, int *deepest) {
-  const int N = M.nod2D, L = M.nl - 1;
-  int nd = 0;
-  for (int n = 1; n < N; n++)
-    if (M.nlev_node[n] > M.nlev_node[nd]) nd = n;
-  *deepest = nd;
-  if (N <= 0) return false;
-  const size_t w = sizeof(double);
-  const double *h = &M.hnode[(size_t)nd * L], *hn = &M.hnode_new[(size_t)nd * L];
-  for (int n = 0; n < N; n++) {
-    const size_t b = w * (M.nlev_node[n] - 1);
-    if (std::memcmp(&M.hnode[(size_t)n * L], h, b) || std::memcmp(&M.hnode_new[(size_t)n * L], hn, b)) return false;
-  }
-  return true;
+void learned_schedules(EngineImpl &P) {
+  build_schedules(P, P.dm32, P.cells_per_block);
 }
 
 std::vector<int> edge_slot_order(const MeshHost &M) {
@@ -509,10 +616,8 @@ void Engine::set_cells_per_block(int cells) {
   EngineImpl &P = *p_;
   if (cells < 32 || cells > kMaxCellsPerBlock) throw std::invalid_argument("cells per block must be in [32, 576]");
   CK(cudaStreamSynchronize(P.stream));
-  if (P.prec == Precision::FP64) build_schedules(P, P.dm64, cells);
-  else build_schedules(P, P.dm32, cells);
   P.cells_per_block = cells;
-  CK(cudaStreamSynchronize(P.stream));
+  if (P.learn) learned_schedules(P);  // otherwise set_learned builds them
 }
 int Engine::cells_per_block() const { return p_->cells_per_block; }
 int Engine::level_stride() const { return p_->S; }

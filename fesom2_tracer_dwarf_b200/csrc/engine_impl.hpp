@@ -170,9 +170,9 @@ void launch_batch_f64fma(EngineImpl &P, const TracerScheme &sc, int nt, const Ba
 // Whether the fused patch kernel runs a batch of this scheme (precision,
 // storage type, vertical scheme, learned flux and plan permitting).
 bool fused_step(const EngineImpl &P, const TracerScheme &sc, bool learned);
-// Whether every node has the same hnode and hnode_new at each of its wet levels;
-// *deepest = a node with the most levels (engine.cu).
-bool uniform_levels(const MeshHost &M, int *deepest);
+// Cell schedules of the learned flux's kernels, for the engine's cells_per_block
+// (engine.cu).
+void learned_schedules(EngineImpl &P);
 // Geometry reciprocals and level tables (step_f64.cu / step_f32.cu).
 void build_rcp_f64(EngineImpl &P);
 void build_rcp_f32(EngineImpl &P);

@@ -116,6 +116,22 @@ void run_group(EngineImpl &P, const TracerScheme &sc, const FusedArgs<R, TS> &a)
   P.mark_end();
 }
 
+// Whether some wet cell's hnode or hnode_new differs, in its bits, from that of node
+// nd (a deepest one) at its level.
+template <typename R>
+__global__ void __launch_bounds__(256) k_levels_differ(DMeshT<R> m, int nd, int *flag) {
+  using U = typename std::conditional<sizeof(R) == 8, unsigned long long, unsigned>::type;
+  const U *h = reinterpret_cast<const U *>(m.hnode), *hn = reinterpret_cast<const U *>(m.hnode_new);
+  const size_t n = (size_t)m.N * m.S;
+  bool differ = false;
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
+    const int c = (int)(q / m.S), k = (int)(q - (size_t)c * m.S);
+    const size_t o = (size_t)nd * m.S + k;
+    differ |= k < m.nlev_node[c] - 1 && (h[q] != h[o] || hn[q] != hn[o]);
+  }
+  if (differ) *flag = 1;
+}
+
 // Geometry reciprocals (k_rcp_planes) and level tables, once per mesh.
 template <typename R>
 void build_rcp_planes_t(EngineImpl &P, DMeshT<R> &d) {
@@ -127,8 +143,18 @@ void build_rcp_planes_t(EngineImpl &P, DMeshT<R> &d) {
   d.rcp = rcp;
   d.rcp_plane = plane;
   // the deepest column stands for every one where the levels are uniform
-  int nd = 0;
-  const bool uni = uniform_levels(P.mesh, &nd);
+  int nd = 0, differ = 1;
+  for (int n = 1; n < d.N; n++)
+    if (P.mesh.nlev_node[n] > P.mesh.nlev_node[nd]) nd = n;
+  if (d.N > 0) {
+    int *flag = P.dalloc<int>(1);
+    k_levels_differ<R><<<std::max(grid, 1), 256, 0, P.stream>>>(d, nd, flag);
+    CK(cudaGetLastError());
+    P.d2h(&differ, flag, sizeof(int));
+    P.dfree(flag);
+    P.bytes -= sizeof(int);
+  }
+  const bool uni = !differ;
   const size_t base = uni ? (size_t)nd * d.S : 0;
   d.uniform_h = uni;
   d.hS = uni ? 0 : d.S;

@@ -927,6 +927,7 @@ void Engine::set_learned(const float *params, bool on) {
   if (P.prec != Precision::FP32) throw std::invalid_argument("the learned flux runs in the FP32 mode");
   CK(cudaStreamSynchronize(P.stream));
   if (!P.learn) {
+    learned_schedules(P);
     P.learn = new LearnedState();
     LearnedState &L = *P.learn;
     if (!mlp_alloc(L.mlp)) throw std::runtime_error("learned flux: device allocation failed");

@@ -8,9 +8,10 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("first", [0, 48])
 @pytest.mark.parametrize("fct", [0, 1])
-def test_training_step_after_the_tile_changed(api, fct):
-    """Default tile, 32 cells per block (16 times the blocks), 576 and the default
+def test_training_step_after_the_tile_changed(api, fct, first):
+    """The tile at which the learned flux is set (the default, or one given before), 32 cells per block (16 times the blocks), 576 and the default
     again: one loss and one gradient.  The loss is an FP64 sum of at most 33 x 33 x
     11 terms, reordered (12,000 x 2^-53 = 1.3e-12 relative); the gradient's order of
     FP32 additions over at most 296 blocks is never fixed (296 x 2^-24 = 1.8e-5)."""
@@ -29,7 +30,7 @@ def test_training_step_after_the_tile_changed(api, fct):
     p = init_params(3)
     p[5248:5312] = np.random.default_rng(2).standard_normal(64).astype(np.float32) * 0.3
     got = []
-    for cells in (0, 32, 576, 0):
+    for cells in (first, 32, 576, 0):
         api.set_cells_per_block(cells)
         if not got:
             assert api.lib.tracer_learn_set(p.ctypes.data, 0) == 0
