@@ -1153,24 +1153,39 @@ __global__ void __launch_bounds__(kColThreads, StepBlocks<R, NT>::col1)
 // ---------------------------------------------------------------------------
 // k_col2: bounds, in/out sums, ratios (lib/oce_adv_tra_fct.F90:105-374)
 // ---------------------------------------------------------------------------
-// Denominator of a limiter ratio, P dt / V +- eps (y = RN(1 / V)), and the ratio of
-// a bound q to it: FP64 quotients in every precision.  FP32 operands, products of two
-// of them and denominators of at least 1e-16 lie inside the exact range, or are not
-// finite: an infinite or NaN P leaves a NaN denominator, which rcp_exact flags.
+// Limiter ratios min(1, q / (P dt / V +- eps)), formed in FP64 in every precision:
+// scale() once per cell, den() per sum, ratio() per bound.
+//
+// FP64: IEEE quotients, y the plane's RN(1 / V).
+// FP32: the FP32 value nearest to the FP64 quotient's.  Reciprocals of two Newton steps
+// and four roundings leave less than 2^-50 of relative error, so the FP32 rounding is
+// the quotient's own unless the result lies within 64 ulp (2^-46) of the middle of two
+// FP32 values: one in 2^22, which sets `bad` like results below 2^-126 and, through NaN,
+// operands that are not finite.  (All quotients exact before their rounding: 3 % of a
+// step of four tracers.)
 template <typename R>
-__device__ __forceinline__ double ratio_den(R P, R dt, R V, double y, double eps, bool &bad) {
-  if constexpr (sizeof(R) == 8) return div_fast(P * dt, V, y, bad) + eps;
-  else return div_near((double)P * (double)dt, (double)V, y) + eps;
-}
-template <typename R>
-__device__ __forceinline__ R ratio(R q, double den, bool &bad) {
-  if constexpr (sizeof(R) == 8) {
-    return fmin2(1.0, div_any(q, den, bad));
-  } else {
-    bad |= !(fabsf(q) < INFINITY);
-    return (R)fmin2(1.0, div_near((double)q, den, rcp_exact(den, bad)));
+struct Ratio;
+template <>
+struct Ratio<double> {
+  static __device__ __forceinline__ double scale(double, double, double y) { return y; }
+  static __device__ __forceinline__ double den(double P, double dt, double V, double y, double eps, bool &bad) {
+    return div_fast(P * dt, V, y, bad) + eps;
   }
-}
+  static __device__ __forceinline__ double ratio(double q, double den, bool &bad) { return fmin2(1.0, div_any(q, den, bad)); }
+};
+template <>
+struct Ratio<float> {
+  static __device__ __forceinline__ double scale(float dt, float V, float) { return (double)dt * rcp_newton((double)V); }
+  static __device__ __forceinline__ double den(float P, float, float, double y, double eps, bool &) {
+    return __fma_rn((double)P, y, eps);
+  }
+  static __device__ __forceinline__ float ratio(float q, double den, bool &bad) {
+    const double r = (double)q * rcp_newton(den);
+    const unsigned u = 2u * (unsigned)__double2hiint(r), lo = (unsigned)__double2loint(r);
+    bad |= ((u - 0x70200000u > 0xffa00000u - 0x70200000u) && not_zero(r, u)) || (lo & 0x1fffffffu) - (0x10000000u - 64u) < 128u;
+    return (float)fmin2(1.0, r);
+  }
+};
 
 // FCT bounds of one cell from the ring elements, for nodes whose ring list is
 // incomplete (lib/oce_adv_tra_fct.F90:105-181).
@@ -1272,14 +1287,7 @@ __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R,
   ldv2(m.areasvol + o, asv);
   ldv2(m.rcp + o, yas);  // 1/areasvol plane (k_rcp_planes)
   if (k + 1 >= nln) asv[1] = yas[1] = R(1);  // dry
-  // FP64 reciprocals of areasvol (FP64: the plane's)
-  bool badv[2] = {false, false};
-  double yv[2];
-#pragma unroll
-  for (int q = 0; q < 2; q++) {
-    if constexpr (sizeof(R) == 8) yv[q] = yas[q];
-    else yv[q] = rcp_exact((double)asv[q], badv[q]);
-  }
+  const double yv[2] = {Ratio<R>::scale(a.dt, asv[0], yas[0]), Ratio<R>::scale(a.dt, asv[1], yas[1])};
   __syncwarp();
 #pragma unroll
   for (int t = 0; t < G; t++) {
@@ -1300,24 +1308,24 @@ __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R,
     // default-real literal.  In FP32 the denominators, where cancellation with it
     // matters, and the quotients are formed in FP64 too.  A quotient of a positive
     // denominator not above bmax is at least 1: a lane where that holds of all its
-    // quotients (limiting is local) does not divide in the FP32 kernels (FP64: the
-    // test costs more than it saves, 0.277 against 0.258 ms at 400x400x64).
+    // quotients (limiting is local) does not divide in the FP32 kernels, which round
+    // to FP32 (FP64: the test costs more than it saves, 0.277 against 0.258 ms at 400x400x64).
     const double eps = (double)1e-16f;
-    bool bad[2] = {badv[0], badv[1]}, need = false;  // bad of each level: a dry second one has no say
+    bool bad[2] = {false, false}, need = false;  // bad of each level: a dry second one has no say
     double up[2], um[2];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const int i = 2 * t + q;
-      up[q] = ratio_den(fp[i], a.dt, asv[q], yv[q], eps, bad[q]);
-      um[q] = ratio_den(fm[i], a.dt, asv[q], yv[q], -eps, bad[q]);
+      up[q] = Ratio<R>::den(fp[i], a.dt, asv[q], yv[q], eps, bad[q]);
+      um[q] = Ratio<R>::den(fm[i], a.dt, asv[q], yv[q], -eps, bad[q]);
       out[2 * q] = out[2 * q + 1] = R(1);
       need |= k + q < nln && (!(up[q] > 0.0 && (double)bx[q] >= up[q]) || !(um[q] < 0.0 && (double)bn[q] <= um[q]));
     }
     if (sizeof(R) == 8 || need) {
 #pragma unroll
       for (int q = 0; q < 2; q++) {
-        out[2 * q] = ratio(bx[q], up[q], bad[q]);
-        out[2 * q + 1] = ratio(bn[q], um[q], bad[q]);
+        out[2 * q] = Ratio<R>::ratio(bx[q], up[q], bad[q]);
+        out[2 * q + 1] = Ratio<R>::ratio(bn[q], um[q], bad[q]);
       }
     }
     if (k + 1 >= nln) out[2] = out[3] = R(0);  // dry: read by k_col3 against a zero flux

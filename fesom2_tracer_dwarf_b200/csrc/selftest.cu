@@ -155,9 +155,9 @@ __global__ void k_quotients(int kind, long long n, uint64_t seed, unsigned long 
         const double den = (double)P * (double)dt / (double)V + eps;
         a = (R)(den * ldexp(1.0 + (double)(mix64(r1) >> 12) * 0x1p-52, -(int)(mix64(r2) % 41)));
         b = V;
-        const double y = sizeof(R) == 8 ? 1.0 / (double)V : fesom::rcp_exact((double)V, bad);
+        const double y = fesom::Ratio<R>::scale(dt, V, R(1) / V);
         if (ma == 2 && mb == 3) a = R(mix64(r2) & 1 ? -INFINITY : INFINITY);
-        q = fesom::ratio(a, fesom::ratio_den(P, dt, V, y, eps, bad), bad);
+        q = fesom::Ratio<R>::ratio(a, fesom::Ratio<R>::den(P, dt, V, y, eps, bad), bad);
         ref = (R)fesom::fmin2(1.0, (double)a / den);
         break;
       }
