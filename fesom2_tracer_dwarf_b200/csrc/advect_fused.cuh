@@ -245,12 +245,15 @@ __device__ __forceinline__ double div_fast(double a, double b, double y, bool &b
   bad |= (u - 0x0f600000u > 0xf0800000u - 0x0f600000u) && not_zero(a, u);
   return div_near(a, b, y);
 }
-__device__ __forceinline__ float div_fast(float a, float b, float y, bool &bad) {
+__device__ __forceinline__ float div_near(float a, float b, float y) {
   float q = a * y;
   q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+__device__ __forceinline__ float div_fast(float a, float b, float y, bool &bad) {
   const unsigned u = 2u * __float_as_uint(a);
   bad |= (u - 0x1b000000u > 0xe3000000u - 0x1b000000u) && u != 0u;
-  return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+  return div_near(a, b, y);
 }
 
 // RN(1 / b), straight-line: the hardware's approximate reciprocal refined by
@@ -279,26 +282,40 @@ __device__ __forceinline__ float rcp_exact(float b, bool &bad) {
   bad |= u - lo > hi - lo || (__float_as_uint(b) | 0xff800000u) == 0xffffffffu;
   return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
 }
-// a / b for any divisor: the limiter ratios and the ring means.  Numerators below
-// 2^-500 (FP32: 2^-60) other than zero set `bad` too, so that no quotient underflows.
-__device__ __forceinline__ bool tiny(double a) {
+// a / b for any divisor, given y = RN(1 / b) of rcp_exact: the limiter ratios and the
+// ring means.  Numerators other than zero outside [2^-500, 2^900] (FP32: [2^-60,
+// 2^100]) set `bad`, so that no quotient underflows.
+__device__ __forceinline__ double div_any(double a, double b, double y, bool &bad) {
   const unsigned u = 2u * (unsigned)__double2hiint(a);
-  return u < 0x41600000u && not_zero(a, u);
+  bad |= (u - 0x41600000u > 0xf0800000u - 0x41600000u) && not_zero(a, u);
+  return div_near(a, b, y);
 }
-__device__ __forceinline__ bool tiny(float a) {
+__device__ __forceinline__ float div_any(float a, float b, float y, bool &bad) {
   const unsigned u = 2u * __float_as_uint(a);
-  return u < 0x43000000u && u != 0u;
-}
-// the same given y = RN(1 / b) of rcp_exact
-template <typename R>
-__device__ __forceinline__ R div_any(R a, R b, R y, bool &bad) {
-  bad |= tiny(a);
-  return div_fast(a, b, y, bad);
+  bad |= (u - 0x43000000u > 0xe3000000u - 0x43000000u) && u != 0u;
+  return div_near(a, b, y);
 }
 template <typename R>
 __device__ __forceinline__ R div_any(R a, R b, bool &bad) {
   return div_any(a, b, rcp_exact(b, bad), bad);
 }
+
+// The flag of a pair's divisions: pb[q] takes those of level q, and a dry second
+// level's has no say, whatever its cells hold.
+struct PairBad {
+  bool wet1;  // the second level is wet
+  bool any = false;
+  struct Level {
+    PairBad &p;
+    int q;
+    bool b = false;
+    __device__ __forceinline__ Level(PairBad &p, int q) : p(p), q(q) {}
+    __device__ __forceinline__ ~Level() { p.any |= b && (q == 0 || p.wet1); }
+    __device__ __forceinline__ operator bool &() { return b; }
+  };
+  __device__ __forceinline__ explicit PairBad(bool wet1) : wet1(wet1) {}
+  __device__ __forceinline__ Level operator[](int q) { return Level(*this, q); }
+};
 
 // One pair of node levels: the ring's elements one after the other (a level an
 // element does not reach adds nothing).  The pairs are the few bottom levels of
@@ -579,7 +596,7 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
       st_pair_il<NT, 1>(a.adf_h, t, o, out);
     }
   } else {
-    bool bad[2] = {false, false};  // of each level: a dry second one has no say
+    PairBad bad(k + 1 < x.levels());
     // the loads of G tracers are all issued before the first is used
     constexpr int G = NT > 2 ? 2 : NT;
     [[maybe_unused]] int cell = 0;
@@ -624,8 +641,11 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
       const R hph = R(0.5) * (R(1) - a.ph);
       [[maybe_unused]] R cour[2];
       if constexpr (HOR == HOR_MUSCL_FEAT) {
-        cour[0] = edge_courant(vf[0], a.dt, vol[0], FeatFast{bad[0]});
-        cour[1] = edge_courant(vf[1], a.dt, vol[1], FeatFast{bad[1]});
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          auto b = bad[q];
+          cour[q] = edge_courant(vf[q], a.dt, vol[q], FeatFast{b});
+        }
       }
       R out[2 * G];
 #pragma unroll
@@ -667,7 +687,7 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
           out[2 * i + q] = ho - flo;
           if constexpr (HOR == HOR_MUSCL_FEAT) {
             if (k + q < x.levels())
-              edge_features(m, a, FeatFast{bad[q]}, t, cell + q, k + q, vf[q], cour[q], b1[i][q], b2[i][q], x1, x2, Tmean1, Tmean2, gux,
+              edge_features(m, a, FeatFast{bad.any}, t, cell + q, k + q, vf[q], cour[q], b1[i][q], b2[i][q], x1, x2, Tmean1, Tmean2, gux,
                             guy, gdx, gdy, exa, eyr, c1, c2, sh);
           }
         }
@@ -678,7 +698,7 @@ __device__ __forceinline__ void edge_pair(const DMeshT<R> &m, const FusedArgs<R,
         for (int i = 0; i < G; i++) out[2 * i + 1] = R(0);
       st_pair_il<NT, G>(a.adf_h, t0, o, out);
     }
-    if (bad[0] || (bad[1] && k + 1 < x.levels())) edge_pair_slow<R, TS, NT, HOR, LIM>(m, a, e, k);
+    if (bad.any) edge_pair_slow<R, TS, NT, HOR, LIM>(m, a, e, k);
   }
 }
 
@@ -964,7 +984,7 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
     });
   }
 
-  bool bad[2] = {false, false};  // of each level: a dry second one has no say
+  PairBad bad(k + 1 < nln);
   R hov[2 * G], lov[G][2];
 #pragma unroll
   for (int t = 0; t < G; t++)
@@ -980,8 +1000,7 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
       ldv2(lt + LT_D * S, fD); ldv2(lt + LT_E * S, fE);
       h[0] = m.hT[km]; ldv2(m.hT + k, h + 1);
       yh[0] = m.ltab[LT_YH * S + km]; ldv2(lt + LT_YH * S, yh + 1);
-      bad[0] = yh[0] != yh[0] || yh[1] != yh[1];
-      bad[1] = yh[1] != yh[1] || yh[2] != yh[2];
+      bad.any = yh[0] != yh[0] || yh[1] != yh[1] || yh[2] != yh[2];
     } else {
       const R *HN = m.hnode_new + col, *H = m.hnode + col;
       const R z[5] = {HN[max(k - 2, 0)], HN[km], HN[k], HN[k + 1], HN[kp]};
@@ -1095,7 +1114,7 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
     ldv2(m.hnT + oh, hn);
     ldv2(m.yhnT + oh, yhn);
     ldv2(m.hT + oh, h);
-    bool badl[2] = {false, false};
+    PairBad badl(k + 1 < nln);
 #pragma unroll
     for (int t = 0; t < G; t++) {
       const R dn = __shfl_down_sync(kFull, lov[t][0], 1);
@@ -1107,13 +1126,13 @@ __device__ __forceinline__ void col1_pair(const DMeshT<R> &m, const FusedArgs<R,
         out[2 * t + q] = div_fast(num, hn[q], yhn[q], badl[q]);
       }
     }
-    if (badl[0] || (badl[1] && k + 1 < nln)) {
+    if (badl.any) {
       for (int t = 0; t < G; t++)
         for (int q = 0; q < 2; q++) out[2 * t + q] = (ts[t][1 + q] * h[q] + acc[t][q] / asv[q]) / hn[q];
     }
     if (st) st_pair_il<NT, G>(a.lo, t0, o, out);
   }
-  if (st && (bad[0] || (bad[1] && k + 1 < nln))) col1_vert_slow<R, TS, NT, G, VER, LIM>(m, a, t0, n, k);
+  if (st && bad.any) col1_vert_slow<R, TS, NT, G, VER, LIM>(m, a, t0, n, k);
 }
 
 // The column pairs of `per` consecutive warps of the schedule, one after the
@@ -1183,7 +1202,7 @@ struct Ratio<float> {
     const double r = (double)q * rcp_newton(den);
     const unsigned u = 2u * (unsigned)__double2hiint(r), lo = (unsigned)__double2loint(r);
     bad |= ((u - 0x70200000u > 0xffa00000u - 0x70200000u) && not_zero(r, u)) || (lo & 0x1fffffffu) - (0x10000000u - 64u) < 128u;
-    return (float)fmin2(1.0, r);
+    return fmin2(1.0f, (float)r);
   }
 };
 
@@ -1311,7 +1330,8 @@ __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R,
     // quotients (limiting is local) does not divide in the FP32 kernels, which round
     // to FP32 (FP64: the test costs more than it saves, 0.277 against 0.258 ms at 400x400x64).
     const double eps = (double)1e-16f;
-    bool bad[2] = {false, false}, need = false;  // bad of each level: a dry second one has no say
+    PairBad bad(k + 1 < nln);
+    bool need = false;
     double up[2], um[2];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -1331,7 +1351,7 @@ __device__ __forceinline__ void col2_pair(const DMeshT<R> &m, const FusedArgs<R,
     if (k + 1 >= nln) out[2] = out[3] = R(0);  // dry: read by k_col3 against a zero flux
     if (l.stores()) {
       stv4(a.rpm[t0 + t] + 2 * (size_t)o, out);
-      if (bad[0] || (bad[1] && k + 1 < nln)) {
+      if (bad.any) {
         for (int q = 0; q < 2; q++) {
           const int i = 2 * t + q;
           const double u = (double)fp[i] * (double)a.dt / (double)asv[q], v = (double)fm[i] * (double)a.dt / (double)asv[q];
@@ -1491,10 +1511,10 @@ __device__ __forceinline__ void col3_pair(const DMeshT<R> &m, const FusedArgs<R,
   const int n = l.item, k = l.k();
   const NodeRec rec = node_rec(m, n);
   const int wet = min(rec.nlev() - 1 - k, 2);
-  bool bad[2] = {false, false};  // of each level: a dry second one has no say
+  PairBad bad(wet == 2);
   R out[G][2];
   col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [&](R x, R y, R z, int q) { return div_fast(x, y, z, bad[q]); }, out);
-  if (bad[0] || (bad[1] && wet == 2)) {
+  if (bad.any) {
     col3_pair_slow<R, TS, NT, G, LIM>(m, a, t0, n, k);
     return;
   }
