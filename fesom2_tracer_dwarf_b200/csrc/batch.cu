@@ -473,8 +473,10 @@ void Batch::configure(const TracerScheme &sch, const std::vector<double> &dt, bo
   B.sch = sch;
   B.dt = dt;
   B.refresh_ab = refresh_ab;
-  for (int m = 0; m < num_members(); m++)
+  for (int m = 0; m < num_members(); m++) {
+    B.members[m]->impl()->run_warps = num_members() > 1 ? kRunShared : kRunAlone;
     for (int t = 0; t < B.ntr[m]; t++) B.members[m]->set_scheme(t, sch);
+  }
   B.configured = true;
   set_tile(B.tile);
 }

@@ -48,13 +48,21 @@ inline int pair_blocks(const DPairs &s, int threads, int per) {
   return (s.nwarps + n - 1) / n;
 }
 // Warps of a schedule that a warp takes one after the other, its loads running
-// ahead from one to the next: at most `most`, fewer where the device would not
-// fill (148 SMs x 16 warps).  Measured at 1000x1000x64: edges 1 / 2 / 4 / 8: FP64
-// 2.28 / 1.94 / 1.83 / 1.83 ms; columns (k_col1 + k_col2 + k_col3) 4.77 / 4.28 /
-// 4.62 / 4.87 ms.
-constexpr int kEdgeRun = 4, kColRun = 2;
-inline int pair_run(const DPairs &s, int most) {
-  const int n = s.nwarps / (148 * 16);
+// ahead from one to the next: at most `most`.  Measured at 1000x1000x64: edges 1 / 2 /
+// 4 / 8: FP64 2.28 / 1.94 / 1.83 / 1.83 ms; columns (k_col1 + k_col2 + k_col3) 4.77 / 4.28 /
+// 4.62 / 4.87 ms.  A run also divides the warps launched, and with them the waves that
+// the last one is a part of: fewer where less than 40 warps per SM would be left, 1.1
+// to 2.5 waves of the kernels' 16 to 36.  A step with column runs of 1 / 2: at 9,510
+// warps (150x150x64) FP64, two tracers 0.155 / 0.163 ms, FP32, one 0.057 / 0.061; at
+// 5,072 0.092 / 0.102, 0.033 / 0.044; at 13,773 (FP64, one) 0.133 / 0.128; with edge runs
+// of 1 / 2 / 4 (FP64, two): at 11,415 0.088 / 0.088 / 0.092, at 31,025 0.217 / 0.212 /
+// 0.216, at 59,943 0.407 / 0.396 / 0.398.  Engines that share the device (a batch's
+// members on their streams) fill it together, so their runs are cut at 16 warps per
+// SM: three members of 194x194x36, 213x213x29 and 188x188x26, 8 tracers: 0.904 ms a
+// step at 16, 0.920 at 40.
+constexpr int kEdgeRun = 4, kColRun = 2, kRunAlone = 40, kRunShared = 16;
+inline int pair_run(const DPairs &s, int most, int warps_per_sm) {
+  const int n = s.nwarps / (148 * warps_per_sm);
   return n < 1 ? 1 : (n > most ? most : n);
 }
 constexpr unsigned kPairNone = 0xffffu, kPairHalo = 0x8000u, kPairRing = 0x4000u, kPairLevel = 0x3fffu;

@@ -82,6 +82,7 @@ struct EngineImpl {
   cudaEvent_t ring_ev[kRing] = {};
   std::vector<Tracer> tr;
   int slots = 0;
+  int run_warps = kRunAlone;  // pair_run's warps per SM
   bool pdl = true;  // step kernels launched with programmatic serialization (not under capture)
   void *vflux = nullptr;
   bool vflux_valid = false;  // vflux holds the edge volume fluxes of the current velocity

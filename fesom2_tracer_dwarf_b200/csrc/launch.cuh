@@ -52,7 +52,7 @@ template <typename R, typename TS, int NT, int HOR, int LIM>
 void launch_edge(EngineImpl &P, const FusedArgs<R, TS> &a) {
   const DMeshT<R> &m = dmesh<R>(P);
   if (m.edge_pairs.nwarps <= 0) return;
-  const int per = pair_run(m.edge_pairs, kEdgeRun), grid = pair_blocks(m.edge_pairs, kEdgeThreads, per);
+  const int per = pair_run(m.edge_pairs, kEdgeRun, P.run_warps), grid = pair_blocks(m.edge_pairs, kEdgeThreads, per);
   P.mark_begin(KK_EDGE);
   if (a.vflux_mode == 2) launch_step(P, k_edge<R, TS, NT, HOR, LIM, true>, grid, kEdgeThreads, m, a, per);
   else launch_step(P, k_edge<R, TS, NT, HOR, LIM, false>, grid, kEdgeThreads, m, a, per);
@@ -62,7 +62,7 @@ void launch_edge(EngineImpl &P, const FusedArgs<R, TS> &a) {
 template <typename R, typename TS, int NT, int VER, int LIM>
 void launch_col1(EngineImpl &P, const FusedArgs<R, TS> &a) {
   const DMeshT<R> &m = dmesh<R>(P);
-  const int per = pair_run(m.node_pairs, kColRun);
+  const int per = pair_run(m.node_pairs, kColRun, P.run_warps);
   const int grid = pair_blocks(m.node_pairs, kColThreads, per);
   P.mark_begin(KK_COL1);
   if (VER != VER_PPM || m.uniform_h) launch_step(P, k_col1<R, TS, NT, VER, LIM, true>, grid, kColThreads, m, a, per);
@@ -105,7 +105,7 @@ void run_group(EngineImpl &P, const TracerScheme &sc, const FusedArgs<R, TS> &a)
     default: launch_col1<R, TS, NT, VER_UPW1, LIM>(P, a); break;
   }
   const DMeshT<R> &m = dmesh<R>(P);
-  const int per = pair_run(m.node_pairs, kColRun), nb = pair_blocks(m.node_pairs, kColThreads, per);
+  const int per = pair_run(m.node_pairs, kColRun, P.run_warps), nb = pair_blocks(m.node_pairs, kColThreads, per);
   if (LIM == LIM_FCT) {
     P.mark_begin(KK_COL2);
     launch_step(P, k_col2<R, TS, NT>, nb, kColThreads, m, a, per);
