@@ -22,9 +22,12 @@
 // node's incident edges in ascending edge id: every node sums its
 // contributions in the order of the reference's serial edge loop, with no
 // float atomics.  The FP64 build has no FMA contraction and keeps every
-// operation of the reference in its order; divisions by a static geometric
-// quantity use a once-per-cell reciprocal with Markstein's correction, which
-// returns the correctly rounded quotient, i.e. the same bits as a division.
+// operation of the reference in its order; divisions multiply by a reciprocal (a
+// table's for static geometry, formed on the spot otherwise) and correct the product
+// after Markstein, which gives the correctly rounded quotient, i.e. the bits of a
+// division.  They are straight-line: operands outside the range where that is exact
+// set a flag, and the lane repeats its pair with plain divisions (div_fast, div_any,
+// div_3k below; div_rcp, which branches, is left to the fused patch kernel).
 #pragma once
 #include <cstdint>
 
@@ -51,7 +54,9 @@ __device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch
 // with fewer (FP64, 400x400x64, two tracers: k_edge 0.30 ms at 4 blocks, 0.33 at 3; k_col1
 // 0.225 at 4, 0.256 / 0.30 at 3 / 5; k_col3 0.236 at 4, 0.237 / 0.32; FP32 k_edge 0.184 at 5, 0.193
 // / 0.188 at 4 / 6; k_col1 0.133 at 7, 0.141 at 5, and with BF16 storage at 500x500x48
-// 0.152, 0.172; k_col2 0.138 at 6, 0.148 at 8).  Build-time knobs.
+// 0.152, 0.172; k_col2 0.138 at 6, 0.148 at 8: as measured when each budget was chosen.
+// The present build: FP64 k_edge 0.301, k_col1 0.240, k_col2 0.256, k_col3 0.207 ms, FP32
+// 0.162, 0.132, 0.136, 0.130).  Build-time knobs.
 #ifndef FESOM_MINB_EDGE
 #define FESOM_MINB_EDGE 4
 #endif
@@ -104,9 +109,9 @@ struct StepBlocks<float, NT> {
 };
 // Tracers of a batch of NT that a lane advances together; it takes the groups one
 // after the other.  Two FP64 tracers share a column's records and geometry
-// (k_col1 0.225 ms against 2 x 0.156 for one at a time, k_col3 0.236 against 2 x 0.137),
-// except in k_col2, whose sums and bounds of two do not fit the registers (0.267
-// against 0.363).
+// (400x400x64: k_col1 0.240 ms against 2 x 0.154 for one at a time, k_col3 0.207 against
+// 2 x 0.132), except in k_col2, whose sums and bounds of two do not fit the registers
+// (one after the other 0.267, both at once 0.363, when it was chosen; 0.256 now).
 template <typename R, int NT>
 struct LaneTracers {
   static constexpr int cap(int g) { return g < NT ? g : NT; }
@@ -1537,7 +1542,7 @@ __global__ void __launch_bounds__(kColThreads, StepBlocks<R, NT>::col3)
   col3_block<R, TS, NT, LIM>(m, a, blockIdx.x, per);
 }
 
-// dynamic shared memory of the cell-map kernels (k_grad, the learned flux)
+// dynamic shared memory of the cell-map kernels (the learned flux's training)
 constexpr size_t smem_edge() { return sizeof(int) * (kMaxItemsPerBlock + 1 + kMaxCellsPerBlock + 1); }
 
 FESOM_VARIANT_END

@@ -87,6 +87,10 @@ class Batch {
   // fastest.  Returns a description of every candidate and its time.
   std::string autotune(int steps_per_candidate);
 
+  // Whether a graph of the selected persistent path is there (path 2 keeps its own until
+  // configure, set_tile, another path or another flux; it reads as false), and the bytes
+  // of the configured tile's work arrays (on path 2 they are released, and the members
+  // hold theirs).
   bool graph_captured() const;
   long long work_bytes() const;
   long long wet_cells() const;  // sum over members of wet cells x tracers

@@ -12,10 +12,10 @@
 // structure-of-arrays in int2/double2/double4 records so one vector load
 // fetches an edge's nodes, elements or cross distances.
 //
-// Work is scheduled over wet cells only: a schedule lists, for groups of
-// consecutive columns, the prefix sums of their wet-level counts, so a block
-// walks a dense range of wet cells and every lane has work even where the
-// bathymetry leaves most of a column dry.
+// Work is scheduled over wet level pairs only: a lane's entry names its column or
+// edge and the first of its two levels (DPairs), so every lane has work even where
+// the bathymetry leaves most of a column dry.  The learned flux's training kernels
+// walk single wet cells by prefix sums of the wet-level counts (DSched).
 #pragma once
 #include <cuda_runtime.h>
 

@@ -400,15 +400,16 @@ __device__ __forceinline__ void mma_over_samples(uint32_t tmem_d, uint32_t a, in
 // grad (FP32, packed like the parameters).  256 threads: warp w holds the tile rows
 // (TMEM lanes) 32 (w & 3) .. + 31 and the hidden units 32 (w >> 2) .. + 31.  What the
 // kernel spends is its SIMT epilogues (three activations of 64 units a sample on
-// the special-function and FP32 pipes), so: two CTAs per SM (46 KB, 256 TMEM
+// the special-function and FP32 pipes), so: two CTAs per SM (51 KB, 256 TMEM
 // columns), one tanh for GELU and its derivative, the first layer's derivative
 // kept in registers for the backward epilogue, bias and output-weight gradients
 // summed in registers across the tiles after a column-halving shuffle
 // reduction.  Measured on 5.8 M samples: 9.87 ms with one 128-thread CTA per SM, five
 // shuffles and a shared-memory atomic per unit and warp, and transposed operand
-// copies written two bytes at a time.
+// copies written two bytes at a time; 1.03 ms so.
 constexpr int kTrainThreads = 256;
 constexpr uint32_t kTrainTmemCols = 256;
+static_assert(2 * (TrainSmem::END + 2048) <= 227 * 1024 && 2 * kTrainTmemCols <= 512, "two CTAs per SM");
 __global__ void __launch_bounds__(kTrainThreads, 2)
     k_mlp_train(const __nv_bfloat16 *X, const float *dy, long long S, MlpDev w, float *grad, int *status) {
   extern __shared__ __align__(1024) unsigned char sm[];

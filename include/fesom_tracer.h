@@ -382,7 +382,9 @@ int tracer_batch_time_steps(int nsteps, int use_graph, double *ms);
  * between device synchronisations. */
 int tracer_batch_steps_separate(int nsteps, int use_graph);
 int tracer_batch_time_separate(int nsteps, int use_graph, double *ms);
-/* info4 = members, wet cells x tracers, work-array bytes, graph captured. */
+/* info4 = members, wet cells x tracers, work-array bytes of the configured tile (paths 0
+ * and 1; on path 2 they are released and the members hold their own), and whether a
+ * graph of path 0 or 1 is captured (0 on path 2, whose graph stays with the members). */
 int tracer_batch_info(long long *info4);
 /* Runs a grid barrier that waits for one block more than the grid holds:
  * returns 1 when the wait ran out after `limit` polls and was reported (the
