@@ -1430,7 +1430,7 @@ __device__ __forceinline__ void col3_store(const FusedArgs<R, TS> &a, int t, cix
   }
 }
 
-// A pair's update with the divisions `div` of each level (the fast ones, or plain ones again
+// A pair's update with the divisions `div` (the fast ones, or plain ones again
 // for the lanes whose operands lie outside their range).
 template <typename R, typename TS, int NT, int G, int LIM, typename D>
 __device__ __forceinline__ void col3_update(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, int n, int k, const NodeRec &rec,
@@ -1470,7 +1470,7 @@ __device__ __forceinline__ void col3_update(const DMeshT<R> &m, const FusedArgs<
           const R p = fmin2(rs[t][2 * q], ro[t][2 * q + 1]), r = fmin2(rs[t][2 * q + 1], ro[t][2 * q]);
           g = (g >= R(0) ? p : r) * g;
         }
-        dh[t][q] = dh[t][q] + div(g * a.dt, asv[q], yas[q], q);
+        dh[t][q] = dh[t][q] + div(g * a.dt, asv[q], yas[q]);
       }
   });
 #pragma unroll
@@ -1495,9 +1495,10 @@ __device__ __forceinline__ void col3_update(const DMeshT<R> &m, const FusedArgs<
     for (int q = 0; q < 2; q++) {
       R dv = R(0);
       if (LIM == LIM_FCT) dv = dv - tt[q] * h[q] + lo[2 * t + q] * hn[q];
-      dv = dv + div((fv[q] - fv[q + 1]) * a.dt, asv[q], yas[q], q);
-      const R del = R(0) + dh[t][q] + dv;
-      out[t][q] = tt[q] + div(del, hn[q], yhn[q], q);
+      dv = dv + div((fv[q] - fv[q + 1]) * a.dt, asv[q], yas[q]);
+      R del = R(0) + dh[t][q] + dv;
+      if (q == 1 && k + 1 >= nln) del = R(0);  // dry: its fluxes are zero, its cells hold anything
+      out[t][q] = tt[q] + div(del, hn[q], yhn[q]);
     }
   }
 }
@@ -1506,7 +1507,7 @@ template <typename R, typename TS, int NT, int G, int LIM>
 __device__ __noinline__ void col3_pair_slow(const DMeshT<R> &m, const FusedArgs<R, TS> &a, int t0, int n, int k) {
   const NodeRec rec = node_rec(m, n);
   R out[G][2];
-  col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [](R x, R y, R, int) { return x / y; }, out);
+  col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [](R x, R y, R) { return x / y; }, out);
   for (int t = 0; t < G; t++) col3_store<R, TS, NT>(a, t0 + t, (cix)n * m.S + k, min(rec.nlev() - 1 - k, 2), out[t]);
 }
 
@@ -1516,10 +1517,10 @@ __device__ __forceinline__ void col3_pair(const DMeshT<R> &m, const FusedArgs<R,
   const int n = l.item, k = l.k();
   const NodeRec rec = node_rec(m, n);
   const int wet = min(rec.nlev() - 1 - k, 2);
-  PairBad bad(wet == 2);
+  bool bad = false;
   R out[G][2];
-  col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [&](R x, R y, R z, int q) { return div_fast(x, y, z, bad[q]); }, out);
-  if (bad.any) {
+  col3_update<R, TS, NT, G, LIM>(m, a, t0, n, k, rec, [&](R x, R y, R z) { return div_fast(x, y, z, bad); }, out);
+  if (bad) {
     col3_pair_slow<R, TS, NT, G, LIM>(m, a, t0, n, k);
     return;
   }
