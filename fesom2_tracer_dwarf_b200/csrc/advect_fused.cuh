@@ -55,8 +55,8 @@ __device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch
 // 0.225 at 4, 0.256 / 0.30 at 3 / 5; k_col3 0.236 at 4, 0.237 / 0.32; FP32 k_edge 0.184 at 5, 0.193
 // / 0.188 at 4 / 6; k_col1 0.133 at 7, 0.141 at 5, and with BF16 storage at 500x500x48
 // 0.152, 0.172; k_col2 0.138 at 6, 0.148 at 8: as measured when each budget was chosen.
-// The present build: FP64 k_edge 0.301, k_col1 0.240, k_col2 0.256, k_col3 0.207 ms, FP32
-// 0.162, 0.132, 0.136, 0.130).  Build-time knobs.
+// The present build: FP64 k_edge 0.301, k_col1 0.240, k_col2 0.255, k_col3 0.205 ms, FP32
+// 0.162, 0.132, 0.137, 0.126).  Build-time knobs.
 #ifndef FESOM_MINB_EDGE
 #define FESOM_MINB_EDGE 4
 #endif
@@ -109,9 +109,9 @@ struct StepBlocks<float, NT> {
 };
 // Tracers of a batch of NT that a lane advances together; it takes the groups one
 // after the other.  Two FP64 tracers share a column's records and geometry
-// (400x400x64: k_col1 0.240 ms against 2 x 0.154 for one at a time, k_col3 0.207 against
-// 2 x 0.132), except in k_col2, whose sums and bounds of two do not fit the registers
-// (one after the other 0.267, both at once 0.363, when it was chosen; 0.256 now).
+// (400x400x64: k_col1 0.240 ms against 2 x 0.154 for one at a time, k_col3 0.205 against
+// 2 x 0.133), except in k_col2, whose sums and bounds of two do not fit the registers
+// (one after the other 0.267, both at once 0.363, when it was chosen; 0.255 now).
 template <typename R, int NT>
 struct LaneTracers {
   static constexpr int cap(int g) { return g < NT ? g : NT; }
